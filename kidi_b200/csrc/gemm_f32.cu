@@ -1,0 +1,384 @@
+// y[M,N] = x[M,K] * W[N,K]^T (+ bias) with 32-bit operands and 32-bit multiply-adds on the CUDA cores: the products of
+// the 32-bit engine. No reduced-precision matrix mode.
+//
+// One order of additions for every shape, so that a row's result does not depend on how many other rows share the launch,
+// on where it falls in a tile, nor on which kernel below runs: K is cut in chunks of 512; a chunk's sum is one chain of fused
+// multiply-adds over ascending k that starts from zero; the chunks' sums are added in ascending order, then the bias.
+// Elements beyond K count as zeros.
+//
+//  * rows (up to 16 rows: decoding): bound by the stream of the weights. A block has 16 features and all of K. A warp takes
+//    four chunks at a time, eight lanes each, so that a lane has up to 4 features x 8 rows although the block's tile is small.
+//    Each warp fills a ring of its own with `cp.async`; there is no barrier of the block before the end. On a B200, weights
+//    of 24,576 x 4,096: 78 us for one row (5.1 TB/s), 106 for eight (3.8 TB/s), 156 for sixteen, where the tiles take 203
+//    and 206 and the 64 x 64 tiles of scalar loads that stood here before took 1,100.
+//  * tiles (more rows): bound by the multiply-adds. Where the tiles alone leave SMs idle, the chunks of K are dealt out over
+//    several blocks, whose sums meet in a workspace ([chunks, M, N]) and are added by a kernel of their own, in the same
+//    order. 301 rows of 24,576 x 4,096: 1,475 us, 41 TFLOP/s (a register-only loop of multiply-adds reaches 58 here), before
+//    2,900. Both operands lie in shared memory by k, transposed on the way in: with rows copied as they lie the operands of a
+//    multiply-add come out of 16-byte loads into the same register bank (every second instruction lost an issue slot, 28 to
+//    36 TFLOP/s whatever the tile). Global loads are four lanes a row: a row a lane cost the load/store pipe, which the
+//    shared-memory reads need, 32 lines an instruction (31 TFLOP/s). Packed multiply-adds (two features an instruction, the
+//    row's number stored twice) were no faster (35 to 40): what they save in issue slots they take in shared-memory reads.
+#include "common.cuh"
+
+namespace {
+constexpr int CHUNK = 512;
+
+__device__ __forceinline__ void copy16(void* to, const void* from, int bytes) {       // the rest of the 16 is zero-filled
+    const unsigned address = (unsigned)__cvta_generic_to_shared(to);
+    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(address), "l"(from), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy4(void* to, const void* from, int bytes) {
+    const unsigned address = (unsigned)__cvta_generic_to_shared(to);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(address), "l"(from), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void commit_copies() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Four consecutive k of one row into shared memory (`from` is the row; k0 a multiple of 4; `alive`: the row exists).
+// ALIGNED: rows start on 16 bytes.
+template <bool ALIGNED>
+__device__ __forceinline__ void copy_piece(float* to, const float* from, int k0, int K, bool alive) {
+    if constexpr (ALIGNED) {
+        const int left = alive ? min(max(K - k0, 0), 4) : 0;
+        copy16(to, from + (left ? k0 : 0), 4 * left);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const bool there = alive && k0 + i < K;
+            copy4(to + i, from + (there ? k0 + i : 0), there ? 4 : 0);
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------------------------ rows
+constexpr int FEATURES = 16;                  // of a block
+constexpr int STEP = 16;                      // k of a stage, for each of a warp's four chunks
+constexpr int PITCH = STEP + 4;               // floats between a stage's rows: the 16-byte pieces of eight rows meet no bank twice
+constexpr int MOST_WARPS = 3;
+
+// ROWS x EACH: the rows and the features of a lane; eight lanes have a chunk's 16 features and PADDED rows (PADDED >= M).
+template <int PADDED, int EACH, int STAGES, bool ALIGNED, typename TY>
+__global__ void __launch_bounds__(32 * MOST_WARPS)
+gemm_f32_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, TY* __restrict__ y, int M, int N, int K,
+                     long long ldx, long long ldw, long long ldy, const float* __restrict__ bias) {
+    extern __shared__ __align__(16) float shared[];
+    constexpr int BY_FEATURE = FEATURES / EACH, BY_ROW = 8 / BY_FEATURE, ROWS = PADDED / BY_ROW;
+    constexpr int GROUP = (FEATURES + PADDED) * PITCH, STAGE = 4 * GROUP, PIECES = STEP / 4;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int n0 = blockIdx.x * FEATURES;
+    const int chunks = (K + CHUNK - 1) / CHUNK;
+    float* ring = shared + warp * STAGES * STAGE;
+    float* sums = shared + warps * STAGES * STAGE;                    // [chunks][PADDED][FEATURES]
+    // The warp's chunks: 4 (warp + turn * warps) + 0..3. The first of four is the longest.
+    const int turns = (chunks - 4 * warp + 4 * warps - 1) / (4 * warps);
+    const int last = 4 * (warp + (turns - 1) * warps);
+    const int steps = turns > 0 ? (turns - 1) * (CHUNK / STEP) + (min(CHUNK, K - last * CHUNK) + STEP - 1) / STEP : 0;
+
+    auto issue = [&](int step) {
+        if (step < steps) {
+            const int chunk = 4 * (warp + step / (CHUNK / STEP) * warps), k0 = chunk * CHUNK + step % (CHUNK / STEP) * STEP;
+            float* stage = ring + step % STAGES * STAGE;
+#pragma unroll
+            for (int i = 0; i < 4 * FEATURES * PIECES / 32; ++i) {
+                const int piece = lane + 32 * i, row = piece / PIECES % FEATURES, group = piece / (PIECES * FEATURES);
+                const int k = piece % PIECES * 4;
+                const bool alive = n0 + row < N;
+                copy_piece<ALIGNED>(stage + group * GROUP + row * PITCH + k, w + (alive ? n0 + row : 0) * ldw, k0 + group * CHUNK + k,
+                                    K, alive);
+            }
+#pragma unroll
+            for (int i = 0; i < (4 * PADDED * PIECES + 31) / 32; ++i) {
+                const int piece = lane + 32 * i, row = piece / PIECES % PADDED, group = piece / (PIECES * PADDED);
+                const int k = piece % PIECES * 4;
+                const bool alive = row < M;
+                if (group < 4)
+                    copy_piece<ALIGNED>(stage + group * GROUP + (FEATURES + row) * PITCH + k, x + (alive ? row : 0) * ldx,
+                                        k0 + group * CHUNK + k, K, alive);
+            }
+        }
+        commit_copies();
+    };
+
+#pragma unroll
+    for (int step = 0; step < STAGES - 1; ++step) issue(step);
+    const int group = lane >> 3, first_feature = lane % BY_FEATURE, first_row = (lane & 7) / BY_FEATURE;
+    float acc[ROWS][EACH];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int f = 0; f < EACH; ++f) acc[r][f] = 0.f;
+    for (int step = 0; step < steps; ++step) {
+        wait_copies<STAGES - 2>();
+        __syncwarp();
+        const float* weights = ring + step % STAGES * STAGE + group * GROUP + first_feature * PITCH;
+        const float* rows = ring + step % STAGES * STAGE + group * GROUP + (FEATURES + first_row) * PITCH;
+#pragma unroll
+        for (int k = 0; k < STEP; k += 4) {
+            float b[EACH][4];
+#pragma unroll
+            for (int f = 0; f < EACH; ++f)
+                *reinterpret_cast<float4*>(b[f]) = *reinterpret_cast<const float4*>(weights + f * BY_FEATURE * PITCH + k);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                float a[4];
+                *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(rows + r * BY_ROW * PITCH + k);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                    for (int f = 0; f < EACH; ++f) acc[r][f] = fmaf(a[e], b[f][e], acc[r][f]);
+            }
+        }
+        __syncwarp();
+        issue(step + STAGES - 1);
+        if (step % (CHUNK / STEP) == CHUNK / STEP - 1 || step == steps - 1) {
+            const int chunk = 4 * (warp + step / (CHUNK / STEP) * warps) + group;
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                for (int f = 0; f < EACH; ++f) {
+                    if (chunk < chunks)
+                        sums[(chunk * PADDED + first_row + r * BY_ROW) * FEATURES + first_feature + f * BY_FEATURE] = acc[r][f];
+                    acc[r][f] = 0.f;
+                }
+        }
+    }
+    __syncthreads();
+    for (int index = threadIdx.x; index < M * FEATURES; index += blockDim.x) {
+        const int row = index / FEATURES, n = n0 + index % FEATURES;
+        if (n >= N) continue;
+        float total = 0.f;
+        for (int chunk = 0; chunk < chunks; ++chunk) total += sums[(chunk * PADDED + row) * FEATURES + index % FEATURES];
+        y[row * ldy + n] = from_float<TY>(bias ? total + bias[n] : total);
+    }
+}
+
+template <int PADDED, int EACH, int STAGES, bool ALIGNED, typename TY>
+int launch_rows(const float* x, const float* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
+                const float* bias, cudaStream_t stream) {
+    const int chunks = (K + CHUNK - 1) / CHUNK, fours = (chunks + 3) / 4;
+    // As many warps as share the chunks evenly, at most MOST_WARPS (two such blocks fit an SM's shared memory).
+    const int turns = (fours + MOST_WARPS - 1) / MOST_WARPS, warps = (fours + turns - 1) / turns;
+    const size_t bytes = ((size_t)warps * STAGES * 4 * (FEATURES + PADDED) * PITCH + (size_t)chunks * PADDED * FEATURES) * sizeof(float);
+    if (bytes > 227 * 1024) return KIDI_REFUSED_SIZE;
+    auto kernel = gemm_f32_rows_kernel<PADDED, EACH, STAGES, ALIGNED, TY>;
+    if (bytes > 48 * 1024) {
+        const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (status != cudaSuccess) return (int)status;
+    }
+    return kidi_launch(kernel, dim3((N + FEATURES - 1) / FEATURES), dim3(32 * warps), bytes, stream, x, w, (TY*)y, M, N, K, ldx,
+                       ldw, ldy, bias);
+}
+
+// ----------------------------------------------------------------------------------------------------------------- tiles
+constexpr int DEPTH = 16;                     // k of a stage
+
+// TM x TN outputs a thread; a warp is 4 x 8 threads, a block WARPS_M x 2 warps.
+template <int TM, int TN, int WARPS_M, int BLOCKS>
+struct Shape {
+    static constexpr int tm = TM, tn = TN, blocks = BLOCKS, rows = 4 * TM * WARPS_M, features = 16 * TN, threads = 64 * WARPS_M;
+    static constexpr int stage = DEPTH * (rows + features);               // floats: [k][row], [k][feature]
+};
+
+// What a thread multiplies for one k: TM rows, TN features, four neighbours at a time.
+template <int TM, int TN>
+struct Operands {
+    float a[TM], b[TN];
+    __device__ __forceinline__ void load(const float* rows, const float* weights, int first_row, int first_feature, int moved) {
+#pragma unroll
+        for (int i = 0; i < TM; i += 4)
+            *reinterpret_cast<float4*>(a + i) = *reinterpret_cast<const float4*>(rows + (first_row ^ moved ^ (4 * i)));
+#pragma unroll
+        for (int j = 0; j < TN; j += 4)
+            *reinterpret_cast<float4*>(b + j) = *reinterpret_cast<const float4*>(weights + (first_feature ^ moved) + 8 * j);
+    }
+};
+
+// COUNT (2, or a multiple of 4) consecutive k of a row, zeros beyond K.
+template <int COUNT, bool ALIGNED>
+__device__ __forceinline__ void load_row(float (&to)[COUNT], const float* from, int left) {
+    if (left >= COUNT) {
+        if constexpr (ALIGNED && COUNT == 2) {
+            const float2 two = *reinterpret_cast<const float2*>(from);
+            to[0] = two.x; to[1] = two.y;
+        } else if constexpr (ALIGNED) {
+#pragma unroll
+            for (int i = 0; i < COUNT; i += 4) {
+                const float4 four = *reinterpret_cast<const float4*>(from + i);
+                to[i] = four.x; to[i + 1] = four.y; to[i + 2] = four.z; to[i + 3] = four.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < COUNT; ++i) to[i] = from[i];
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) to[i] = i < left ? from[i] : 0.f;
+    }
+}
+
+template <class S, bool ALIGNED, typename TY>
+__global__ void __launch_bounds__(S::threads, S::blocks)
+gemm_f32_tiles_kernel(const float* __restrict__ x, const float* __restrict__ w, TY* __restrict__ y, int M, int N, int K,
+                      long long ldx, long long ldw, long long ldy, const float* __restrict__ bias, int chunks_per_block,
+                      float* __restrict__ parts) {
+    extern __shared__ __align__(16) float shared[];
+    constexpr int TM = S::tm, TN = S::tn, THREADS = S::threads, ROWS = S::rows, COLUMNS = S::features;
+    constexpr int APART = THREADS / 4, X = ROWS / APART, W = COLUMNS / APART;    // rows of x and w that a thread copies a piece of
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int m0 = blockIdx.x * ROWS, n0 = blockIdx.y * COLUMNS;
+    const int chunks = (K + CHUNK - 1) / CHUNK;
+    const int first = blockIdx.z * chunks_per_block, end = min(chunks, first + chunks_per_block);
+    const int steps = (end - first - 1) * (CHUNK / DEPTH) + (min(CHUNK, K - (end - 1) * CHUNK) + DEPTH - 1) / DEPTH;
+    float* totals = shared + 2 * S::stage;                            // [TM * TN][THREADS]
+
+    // (Rows that do not exist are copies of the last one: their results are not stored.)
+    const int piece_k = threadIdx.x % 4 * 4, piece_row = threadIdx.x / 4;
+    const float *from_x[X], *from_w[W];
+#pragma unroll
+    for (int i = 0; i < X; ++i) from_x[i] = x + min(m0 + piece_row + APART * i, M - 1) * ldx + first * CHUNK + piece_k;
+#pragma unroll
+    for (int i = 0; i < W; ++i) from_w[i] = w + min(n0 + piece_row + APART * i, N - 1) * ldw + first * CHUNK + piece_k;
+    float held[X + W][4];
+    auto load = [&](int step) {
+        const int k = step * DEPTH, left = K - first * CHUNK - k - piece_k;
+#pragma unroll
+        for (int i = 0; i < X; ++i) load_row<4, ALIGNED>(held[i], from_x[i] + k, left);
+#pragma unroll
+        for (int i = 0; i < W; ++i) load_row<4, ALIGNED>(held[X + i], from_w[i] + k, left);
+    };
+    // Element (k, column) stands in column (column ^ 8 (k / 4 % 4)) of its row: a warp stores four k apart of eight rows, which
+    // meet no bank twice that way, and four neighbouring columns stay neighbours.
+    const int moved_row = piece_row ^ (piece_k * 2);
+    auto store = [&](float* stage) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+#pragma unroll
+            for (int i = 0; i < X; ++i) stage[(piece_k + e) * ROWS + moved_row + APART * i] = held[i][e];
+#pragma unroll
+            for (int i = 0; i < W; ++i) stage[DEPTH * ROWS + (piece_k + e) * COLUMNS + moved_row + APART * i] = held[X + i][e];
+        }
+    };
+
+    // A thread's rows: first_row + 16 h + 0..3; its features: first_feature + 32 g + 0..3.
+    const int first_row = (warp >> 1) * (4 * TM) + (lane >> 3) * 4, first_feature = (warp & 1) * (8 * TN) + (lane & 7) * 4;
+    float acc[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    load(0);
+    store(shared);
+    if (steps > 1) load(1);
+    __syncthreads();
+    for (int step = 0; step < steps; ++step) {
+        const float* rows = shared + (step & 1) * S::stage;
+        const float* weights = rows + DEPTH * ROWS;
+        Operands<TM, TN> operands[2];
+        operands[0].load(rows, weights, first_row, first_feature, 0);
+#pragma unroll
+        for (int k = 0; k < DEPTH; ++k) {
+            if (k + 1 < DEPTH)
+                operands[(k + 1) & 1].load(rows + (k + 1) * ROWS, weights + (k + 1) * COLUMNS, first_row, first_feature, (k + 1) / 4 * 8);
+            const Operands<TM, TN>& o = operands[k & 1];
+#pragma unroll
+            for (int j = 0; j < TN; ++j)
+#pragma unroll
+                for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(o.a[i], o.b[j], acc[i][j]);
+        }
+        if (step + 1 < steps) {
+            store(shared + (step + 1 & 1) * S::stage);
+            if (step + 2 < steps) load(step + 2);
+        }
+        __syncthreads();
+        if (step % (CHUNK / DEPTH) != CHUNK / DEPTH - 1 && step != steps - 1) continue;
+        const int chunk = first + step / (CHUNK / DEPTH);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int m = m0 + first_row + (i / 4) * 16 + i % 4;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int n = n0 + first_feature + (j / 4) * 32 + j % 4;
+                float value = acc[i][j];
+                acc[i][j] = 0.f;
+                if (parts) {
+                    if (m < M && n < N) parts[((long long)chunk * M + m) * N + n] = value;
+                    continue;
+                }
+                float* total = totals + (i * TN + j) * THREADS + threadIdx.x;
+                if (chunk) value = *total + value;
+                if (chunk < chunks - 1) *total = value;
+                else if (m < M && n < N) y[m * ldy + n] = from_float<TY>(bias ? value + bias[n] : value);
+            }
+        }
+    }
+}
+
+// The chunks' sums, added in ascending order.
+template <typename TY>
+__global__ void __launch_bounds__(256) gemm_f32_add_kernel(const float* __restrict__ parts, TY* __restrict__ y, int M, int N,
+                                                           int chunks, long long ldy, const float* __restrict__ bias) {
+    const int n = blockIdx.x * 256 + threadIdx.x, m = blockIdx.y;
+    if (n >= N) return;
+    const long long slab = (long long)M * N;
+    const float* part = parts + (long long)m * N + n;
+    float total = 0.f;
+#pragma unroll 8
+    for (int chunk = 0; chunk < chunks; ++chunk) total += part[chunk * slab];
+    y[m * ldy + n] = from_float<TY>(bias ? total + bias[n] : total);
+}
+
+template <class S, bool ALIGNED, typename TY>
+int launch_tiles(const float* x, const float* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
+                 const float* bias, int chunks_per_block, float* parts, cudaStream_t stream) {
+    const int chunks = (K + CHUNK - 1) / CHUNK, splits = (chunks + chunks_per_block - 1) / chunks_per_block;
+    const int tiles_m = (M + S::rows - 1) / S::rows, tiles_n = (N + S::features - 1) / S::features;
+    if ((splits > 1) != (parts != nullptr) || tiles_n > 65535 || splits > 65535 || (parts && M > 65535)) return KIDI_REFUSED_SIZE;
+    const size_t most = (2 * S::stage + S::tm * S::tn * S::threads) * sizeof(float);
+    const size_t bytes = chunks > 1 && !parts ? most : 2 * S::stage * sizeof(float);
+    auto kernel = gemm_f32_tiles_kernel<S, ALIGNED, TY>;
+    const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (status != cudaSuccess) return (int)status;
+    const int code = kidi_launch(kernel, dim3(tiles_m, tiles_n, splits), dim3(S::threads), bytes, stream, x, w, (TY*)y, M, N, K, ldx,
+                                 ldw, ldy, bias, chunks_per_block, parts);
+    if (code || !parts) return code;
+    return kidi_launch(gemm_f32_add_kernel<TY>, dim3((N + 255) / 256, M), dim3(256), 0, stream, (const float*)parts, (TY*)y, M, N,
+                       chunks, ldy, bias);
+}
+
+template <bool ALIGNED, typename TY>
+int launch(const float* x, const float* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
+           const float* bias, int form, int chunks_per_block, float* parts, cudaStream_t stream) {
+    if (form == 0) {
+#define KIDI_ROWS(P, F, S) launch_rows<P, F, S, ALIGNED, TY>(x, w, y, M, N, K, ldx, ldw, ldy, bias, stream)
+        if (M == 1) return KIDI_ROWS(1, 2, 4);
+        if (M == 2) return KIDI_ROWS(2, 4, 4);
+        if (M <= 4) return KIDI_ROWS(4, 4, 4);
+        if (M <= 8) return KIDI_ROWS(8, 4, 4);
+        if (M <= 16) return KIDI_ROWS(16, 4, 3);
+#undef KIDI_ROWS
+        return KIDI_REFUSED_SIZE;
+    }
+    if (chunks_per_block < 1) return KIDI_REFUSED_SIZE;
+#define KIDI_TILES(...) launch_tiles<Shape<__VA_ARGS__>, ALIGNED, TY>(x, w, y, M, N, K, ldx, ldw, ldy, bias, chunks_per_block, parts, stream)
+    if (form == 1) return KIDI_TILES(4, 8, 2, 4);
+    if (form == 2) return KIDI_TILES(8, 8, 2, 3);
+#undef KIDI_TILES
+    return KIDI_REFUSED_SIZE;
+}
+}  // namespace
+
+// `form`: 0 rows (M <= 16), 1 tiles of 32 rows, 2 tiles of 64. `chunks_per_block` (tiles): the chunks of 512 a block adds
+// up; fewer than K has: `parts` is a workspace of ceil(K / 512) * M * N floats (else null). The result is the same bit for
+// bit whatever the choice. `bias`: float32 [N] or null.
+KIDI_API int kidi_gemm_f32(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K, long long ldx, long long ldw,
+                           long long ldy, const float* bias, int form, int chunks_per_block, float* parts, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K <= 0 || (M + 63) / 64 > 65535) return KIDI_REFUSED_SIZE;
+    const bool aligned = !((uintptr_t)x & 15) && !((uintptr_t)w & 15) && !(ldx & 3) && !(ldw & 3);
+#define KIDI_CASE(A, T) launch<A, T>((const float*)x, (const float*)w, y, M, N, K, ldx, ldw, ldy, bias, form, chunks_per_block, parts, stream)
+    if (y_dtype == KIDI_F32) return aligned ? KIDI_CASE(true, float) : KIDI_CASE(false, float);
+    if (y_dtype == KIDI_BF16) return aligned ? KIDI_CASE(true, bf16) : KIDI_CASE(false, bf16);
+#undef KIDI_CASE
+    return KIDI_REFUSED_DTYPE;
+}

@@ -1,0 +1,76 @@
+"""Matrix products with 32-bit operands and 32-bit multiply-adds (csrc/gemm_f32.cu): how a shape is cut.
+
+The result is the same bit for bit whatever is chosen here (see the kernels' order of additions), so a choice may depend on
+the number of rows."""
+from __future__ import annotations
+
+import functools
+from typing import Optional, Tuple
+
+import torch
+
+from . import ops
+from .attention import sm_count
+from .ops import _check, _stream, c_int, c_longlong, c_void_p, dtype_code
+
+CHUNK = 512           # k of a chain of multiply-adds, as csrc/gemm_f32.cu has it
+ROWS, TILES_32, TILES_64 = 0, 1, 2
+ROWS_MAX = 16         # rows that the weight-streaming form takes: at 16 it is level with the tiles or ahead (114 against
+                      # 118 us at 4,096 x 12,288, 156 against 206 at 24,576 x 4,096), beyond it has no form
+ROWS_CHUNKS = 100     # chunks whose sums fit its shared memory
+TILE_N = 128
+# Microseconds that one, two, ... blocks on an SM (the last: as many as fit) take for a chunk each, measured on a B200.
+TIMES = {TILES_32: (0, 27, 38, 52, 70), TILES_64: (0, 40, 62, 80)}
+TILE_M = {TILES_32: 32, TILES_64: 64}
+PARTS_MAX = 1 << 27   # floats of the workspace (512 MB)
+
+
+@functools.lru_cache(maxsize=4096)
+def plan(rows: int, features: int, k: int, sms: int) -> Tuple[int, int]:
+    """(form, chunks a block adds up): for tiles the height and the share of K with the smallest expected time, which is
+    that of the SM with the most blocks, and what the chunks' sums cost on their way through the workspace (4 TB/s, and a
+    launch of 5 us). 301 rows of 4,096 x 12,288: a chunk a block 734 us, all 24 to a block 1,431; 512 rows of 24,576 x 4,096: 2,360 and 2,429."""
+    chunks = -(-k // CHUNK)
+    if rows <= ROWS_MAX and chunks <= ROWS_CHUNKS:
+        return ROWS, chunks
+    best, best_cost = (TILES_64, chunks), None
+    for form, times in TIMES.items():
+        tiles = -(-rows // TILE_M[form]) * -(-features // TILE_N)
+        for count in range(chunks, 0, -1):
+            splits = -(-chunks // count)
+            if splits > 1 and (chunks * rows * features > PARTS_MAX or rows > 65535):
+                break
+            rounds, rest = divmod(-(-tiles * splits // sms), len(times) - 1)
+            cost = (rounds * times[-1] + times[rest]) * count
+            if splits > 1:
+                cost += 5 + chunks * rows * features * 8 / 4e6
+            if best_cost is None or cost < best_cost:
+                best, best_cost = (form, count), cost
+    return best
+
+
+_launch = None
+
+
+def _bind():
+    global _launch
+    _launch = ops.core().kidi_gemm_f32
+    _launch.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
+                        c_void_p, c_int, c_int, c_void_p, c_void_p]
+    _launch.restype = c_int
+
+
+def gemm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
+         choice: Optional[Tuple[int, int]] = None) -> None:
+    """out = x @ weight.T (+ bias) for float32 x and weight with contiguous rows. `choice`: another plan (for tests)."""
+    if _launch is None:
+        _bind()
+    rows, k = x.shape
+    features = weight.shape[0]
+    form, count = choice or plan(rows, features, k, sm_count(x.device))
+    chunks = -(-k // CHUNK)
+    parts = torch.empty(chunks * rows * features, dtype=torch.float32, device=x.device) if form and count < chunks else None
+    _check(_launch(x.data_ptr(), weight.data_ptr(), out.data_ptr(), dtype_code(out.dtype), rows, features, k, x.stride(0),
+                   weight.stride(0), out.stride(0), bias.data_ptr() if bias is not None else 0, form, count,
+                   parts.data_ptr() if parts is not None else 0, _stream()),
+           "gemm_simt", 1 if parts is None else 2)
