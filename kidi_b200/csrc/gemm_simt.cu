@@ -1,4 +1,5 @@
-// y[M,N] = x[M,K] * W[N,K]^T with 32-bit multiply-add on the CUDA cores.
+// y[M,N] = x[M,K] * W[N,K]^T with 32-bit multiply-add on the CUDA cores, for operands of which one or both are
+// bfloat16 (gemm_f32.cu has the products of 32-bit operands).
 //
 // This is the true 32-bit matrix product (no reduced-precision matrix mode) and the
 // fallback for shapes the tensor-core kernels refuse. Every output element is one
@@ -89,8 +90,6 @@ KIDI_API int kidi_gemm_simt(const void* x, int x_dtype, const void* w, int w_dty
 #define KIDI_CASE(X, TX, W, TW, Y, TY)                                 \
     if (x_dtype == X && w_dtype == W && y_dtype == Y)                  \
         return launch<TX, TW, TY>(x, w, y, M, N, K, ldx, ldw, ldy, bias, stream);
-    KIDI_CASE(KIDI_F32, float, KIDI_F32, float, KIDI_F32, float)
-    KIDI_CASE(KIDI_F32, float, KIDI_F32, float, KIDI_BF16, bf16)
     KIDI_CASE(KIDI_F32, float, KIDI_BF16, bf16, KIDI_F32, float)
     KIDI_CASE(KIDI_F32, float, KIDI_BF16, bf16, KIDI_BF16, bf16)
     KIDI_CASE(KIDI_BF16, bf16, KIDI_F32, float, KIDI_F32, float)

@@ -773,9 +773,21 @@ def apply_row_factors(values: torch.Tensor, parts: torch.Tensor, width: int, eps
     return out
 
 
+_f32_products = None
+
+
+def _gemm_f32():
+    """The module of 32-bit products (imported at the first call: it is built on this one)."""
+    global _f32_products
+    if _f32_products is None:
+        from . import gemm_f32
+        _f32_products = gemm_f32
+    return _f32_products
+
+
 def gemm_simt(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype,
               out: Optional[torch.Tensor] = None, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """y = x @ weight.T (+ bias) with 32-bit fused multiply-adds in ascending k."""
+    """y = x @ weight.T (+ bias) with 32-bit fused multiply-adds, added in an order that depends on K and the types only."""
     _need_cuda(x, weight, bias)
     check_bias(bias, weight.shape[0])
     if x.dim() != 2 or weight.dim() != 2 or x.shape[1] != weight.shape[1]:
@@ -786,6 +798,9 @@ def gemm_simt(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype,
     N = weight.shape[0]
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
+    if x.dtype == torch.float32 and weight.dtype == torch.float32 and M > 0:
+        _gemm_f32().gemm(x, weight, out, bias)
+        return out
     _check(core().kidi_gemm_simt(_ptr(x), dtype_code(x.dtype), _ptr(weight), dtype_code(weight.dtype), _ptr(out),
                                  dtype_code(out.dtype), M, N, K, x.stride(0), weight.stride(0), out.stride(0),
                                  _ptr(bias), _stream()), "gemm_simt")

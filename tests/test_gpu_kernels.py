@@ -85,6 +85,40 @@ def test_gemm_32_bit(shape):
     assert torch.equal(alone[0], out[M // 2])
 
 
+# Edges of the 16-feature and 128-feature tiles, of 32 and 64 rows, of a stage, of the chunks of 512 k and of four of them.
+@pytest.mark.parametrize("shape", [(1, 389, 3), (2, 16, 511), (4, 17, 512), (5, 130, 513), (8, 127, 2049), (9, 40, 6145),
+                                   (16, 129, 1025), (17, 128, 15), (32, 257, 2047), (33, 64, 17), (64, 129, 1024),
+                                   (65, 300, 3001), (129, 128, 4100)])
+def test_gemm_32_bit_is_the_same_however_it_is_cut(shape):
+    from kidi_b200.kernels import gemm_f32, ops
+    M, N, K = shape
+    generator = torch.Generator().manual_seed(M + N)
+    x, w = torch.randn(M, K, generator=generator).to(DEVICE), torch.randn(N, K, generator=generator).to(DEVICE)
+    bias = torch.randn(N, generator=generator).to(DEVICE)
+    chunks = -(-K // gemm_f32.CHUNK)
+    choices = [(form, count) for form in (gemm_f32.TILES_32, gemm_f32.TILES_64) for count in sorted({1, -(-chunks // 2), chunks})]
+    if M <= gemm_f32.ROWS_MAX:
+        choices.append((gemm_f32.ROWS, chunks))
+    expected = x.double() @ w.double().T + bias.double()
+    found = ops.gemm_simt(x, w, torch.float32, bias=bias)
+    # Chains of 512 and a sum of chunks: the errors of 32-bit additions in a random walk, 2^-24 sqrt(512 + K / 512) of the
+    # result's size a deviation, six deviations and the largest of some thousand results.
+    close(found, expected, 6 * 2.0 ** -24 * math.sqrt(512 + chunks) * math.sqrt(K) / max(1.0, float(expected.abs().max())) + 1e-7,
+          "32-bit product")
+    for choice in choices:
+        out = torch.full((M, N), float("nan"), device=DEVICE)
+        gemm_f32.gemm(x, w, out, bias, choice)
+        assert torch.equal(out, found), choice
+    # Rows that start on no 16-byte boundary, results in bfloat16 and in a matrix with wider rows, and a row by itself.
+    odd = torch.empty(M, K + 1, device=DEVICE)[:, 1:].copy_(x)
+    assert torch.equal(ops.gemm_simt(odd, w, torch.float32, bias=bias), found)
+    wide = torch.zeros(M, N + 3, device=DEVICE)
+    ops.gemm_simt(x, w, torch.float32, out=wide[:, :N], bias=bias)
+    assert torch.equal(wide[:, :N], found) and not wide[:, N:].any()
+    assert torch.equal(ops.gemm_simt(x, w, torch.bfloat16, bias=bias), found.to(torch.bfloat16))
+    assert torch.equal(ops.gemm_simt(x[M // 2:M // 2 + 1], w, torch.float32, bias=bias)[0], found[M // 2])
+
+
 @pytest.mark.parametrize("rows", [1, 3, 8, 9, 16, 31, 64])
 @pytest.mark.parametrize("shape", [(389, 96), (100, 200), (4096, 1024), (40, 4104)])
 @pytest.mark.parametrize("row_tiles", [1, 2])

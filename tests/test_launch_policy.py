@@ -91,3 +91,16 @@ def test_shares_of_differential_decode_attention(monkeypatch):
     assert differential.tensor_fits(torch.bfloat16, 32, 80, 64) and differential.tensor_fits(torch.bfloat16, 128, 16, 64)
     assert not differential.tensor_fits(torch.float32, 32, 80, 64) and not differential.tensor_fits(torch.bfloat16, 40, 80, 64)
     assert not differential.tensor_fits(torch.bfloat16, 144, 80, 64) and not differential.tensor_fits(torch.bfloat16, 32, 80, 32)
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17, 32, 33, 64, 301, 4096, 70000])
+@pytest.mark.parametrize("features, k", [(1, 1), (389, 96), (4096, 12288), (151936, 4096), (128, 60000)])
+def test_a_32_bit_product_is_cut_into_whole_chunks_within_its_workspace(rows, features, k):
+    from kidi_b200.kernels import gemm_f32
+    form, count = gemm_f32.plan(rows, features, k, 148)
+    chunks = -(-k // gemm_f32.CHUNK)
+    assert 1 <= count <= chunks
+    if form == gemm_f32.ROWS:
+        assert rows <= gemm_f32.ROWS_MAX and count == chunks
+    elif count < chunks:
+        assert chunks * rows * features <= gemm_f32.PARTS_MAX and rows <= 65535
