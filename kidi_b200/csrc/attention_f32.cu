@@ -1,0 +1,579 @@
+// Causal attention in 32 bits over the cache and the step's own rows: the 32-bit engine's kernel for heads of up to 128
+// (formulas: see attention_generic.cu, which serves the other widths).
+//
+// One order of additions, so that a row's result is the same bit for bit in every batch and under every cut of the work,
+// whichever kernel below takes it. Keys are cut by their position in tiles of 64 and segments of 256. A score is one chain
+// of multiply-adds over ascending dimensions. In a segment the softmax runs on tile by tile: the running maximum m; the
+// weights' sum l <- l c + ((s0 + s1) + (s2 + s3)) with s_j a chain over 16 keys and c = exp(m_before - m); the weighted sum
+// o <- o c, then a chain of multiply-adds over ascending keys. Segments are merged in ascending order (`Merged`). A key that
+// a row does not see has no part in its sums, whatever it holds.
+//
+//  * tiles: prompts. A block takes 64 consecutive rows of a sequence for one head. Both products are register tiles of 8 x 4
+//    and 8 x 8 (8 x 4 for values of up to 64), operands by k in shared memory; keys are transposed on the way in, 16
+//    dimensions at a time, values are copied as they lie while the scores are computed. Bound by the multiply-adds and by
+//    what one warp a scheduler leaves idle (two blocks of four warps an SM: 250 registers a thread for two sets of sums):
+//    32 heads of 128 over 8, a prompt of 700 tokens 359 us (23 TFLOP/s), of 2,000 1,718 (a warp a row, head and key before:
+//    5,800 for 2,000).
+//  * rows: decoding, and steps of a few tokens a sequence. A block takes one row, up to eight heads that share a key head,
+//    and every n-th segment, and leaves its sums in a workspace, which a second kernel merges (with one block a row the block
+//    merges them itself). The grid does not depend on how long the sequences are, so a captured step serves all lengths. Bound by the stream of keys and values, 64 KB a tile and block, three blocks an SM: 8 sequences of 1,030 tokens
+//    43 us (455 before), of 4,000 110 (2.4 TB/s).
+#include <type_traits>
+
+#include "attention_args.cuh"
+
+struct AttentionF32Args {
+    AttentionArgs a;
+    const int* seq_len;     // [seqs]
+    int seqs, max_new;
+    int segments;           // the most segments a row may see (rows)
+    int shares;             // blocks that share a row's segments (rows)
+    float* parts;           // [rows, heads, segments, value_dim + 2] (rows; null for one share)
+};
+
+namespace {
+constexpr int TILE = 64, SEGMENT = 256, THREADS = 128;
+
+__device__ __forceinline__ void copy16(float* to, const float* from, const float* somewhere) {       // `from` null: zeros
+    const unsigned address = (unsigned)__cvta_generic_to_shared(to);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(address), "l"(from ? from : somewhere), "r"(from ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void commit_copies() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// The score of a key at `u` for a query at `position`, from their product.
+__device__ __forceinline__ float score_of(const AttentionArgs& a, float dot, int head, int position, int u) {
+    float score = __fmul_rn(dot, a.scale);
+    if (a.softcap > 0.f) score = __fmul_rn(a.softcap, tanhf(__fdiv_rn(score, a.softcap)));
+    if (a.slopes) score = __fmaf_rn(a.slopes[head], (float)(u - position), score);
+    if (a.distance_bias) score = __fadd_rn(score, a.distance_bias[(long long)head * a.bias_stride + min(position - u, a.bias_last)]);
+    return score;
+}
+
+// A key's weight beside the running maximum `top` (a key that is not seen has the score -infinity).
+__device__ __forceinline__ float weight_of(const AttentionArgs& a, float score, int head, float top) {
+    if (score == -INFINITY) return 0.f;
+    if (a.weight_bias) return __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-__fadd_rn(score, a.weight_bias[head]))));
+    return expf(__fsub_rn(score, top));
+}
+
+// exp(from - to) for a maximum that grew; nothing seen yet (both -infinity): 1.
+__device__ __forceinline__ float shrink(float from, float to) { return to == -INFINITY ? 1.f : expf(__fsub_rn(from, to)); }
+
+// The sums of the segments so far, as one maximum and one sum of weights; `old` and `fresh` are the factors of the weighted sum.
+struct Merged {
+    float top = -INFINITY, sum = 0.f, old = 0.f, fresh = 0.f;
+    __device__ __forceinline__ void add(float segment_top, float segment_sum) {
+        const float next = fmaxf(top, segment_top);
+        old = shrink(top, next);
+        fresh = shrink(segment_top, next);
+        sum = __fmaf_rn(segment_sum, fresh, __fmul_rn(sum, old));
+        top = next;
+    }
+};
+__device__ __forceinline__ float merge(float total, float part, float old, float fresh) {
+    return __fmaf_rn(part, fresh, __fmul_rn(total, old));
+}
+
+// What the weighted sum is multiplied and divided by at the end.
+__device__ __forceinline__ void closing(const AttentionArgs& a, int head, float top, float sum, float& factor, float& divisor) {
+    factor = divisor = 1.f;
+    if (a.weight_bias) return;
+    const float sink = a.sinks ? a.sinks[head] : -INFINITY, highest = fmaxf(top, sink);
+    factor = shrink(top, highest);
+    divisor = __fmul_rn(sum, factor);
+    if (a.sinks) divisor = __fadd_rn(divisor, expf(__fsub_rn(sink, highest)));
+}
+__device__ __forceinline__ void put(const AttentionArgs& a, int row, int head, int vd, int c, float total, float factor, float divisor) {
+    float value = __fdiv_rn(__fmul_rn(total, factor), divisor);
+    if (a.gate) value = __fmul_rn(value, __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-((const float*)a.gate)[row * a.ldg + head]))));
+    if (a.element_gate) {
+        const float gate = ((const float*)a.element_gate)[row * a.ld_element_gate + (long long)head * vd + c];
+        value = __fmul_rn(value, __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-gate))));
+    }
+    ((float*)a.out)[row * a.ldo + (long long)head * vd + c] = __fmul_rn(value, a.out_scale);
+}
+
+// Where the key and the value of position u of a sequence lie.
+__device__ __forceinline__ void key_at(const AttentionArgs& a, int u, int start, int row0, int slot, int kv_head, int d, int vd,
+                                       const float*& key, const float*& value) {
+    if (u >= start) {
+        const long long offset = (long long)(row0 + u - start) * a.ldkv;
+        key = (const float*)a.k_step + offset + (long long)kv_head * d;
+        value = (const float*)a.v_step + offset + (long long)kv_head * vd;
+    } else {
+        const long long offset = cache_row_offset(a.cache, slot, u, kv_head);
+        key = (const float*)a.k_cache + offset;
+        value = (const float*)a.v_cache + offset / d * vd;
+    }
+}
+
+// ------------------------------------------------------------------------------------------------------------------ rows
+constexpr int GROUP = 8;         // heads of a block
+constexpr int KEY_PAD = 4;       // floats between the keys of a tile: eight keys' 16-byte pieces meet no bank twice
+
+__global__ void __launch_bounds__(THREADS) attention_f32_rows_kernel(AttentionF32Args args) {
+    const AttentionArgs& a = args.a;
+    extern __shared__ __align__(16) float shared[];
+    __shared__ const float* keys_at[TILE];
+    __shared__ const float* values_at[TILE];
+    __shared__ float query[GROUP][128], scores[GROUP][TILE], top[GROUP], sum[GROUP], scale[GROUP];
+    const int d = a.head_dim, vd = a.value_dim ? a.value_dim : d, pitch = d + KEY_PAD;
+    float* keys = shared;                             // [TILE][pitch]
+    float* values = shared + TILE * pitch;            // [TILE][vd]
+    const int group = a.heads / a.kv_heads, blocks = (group + GROUP - 1) / GROUP;
+    const int row = blockIdx.x, kv_head = blockIdx.y / blocks, t = threadIdx.x;
+    const int head0 = kv_head * group + blockIdx.y % blocks * GROUP, heads = min(GROUP, kv_head * group + group - head0);
+    const int seq = a.row_seq[row];
+    if (seq < 0) {
+        if (!args.parts)
+            for (int i = t; i < heads * vd; i += THREADS) ((float*)a.out)[row * a.ldo + (long long)head0 * vd + i] = 0.f;
+        return;
+    }
+    const int position = a.row_pos[row], first = first_visible(position, a.window, a.chunk);
+    const int first_segment = first / SEGMENT, last_segment = position / SEGMENT;
+    if (first_segment + (int)blockIdx.z > last_segment) return;
+    const int slot = a.seq_slot[seq], start = a.k_step ? a.seq_start[seq] : 0x7fffffff, row0 = a.seq_row0[seq];
+    for (int i = t; i < heads * d; i += THREADS) query[i / d][i % d] = ((const float*)a.q)[row * a.ldq + (long long)head0 * d + i];
+    float acc[GROUP], total[GROUP];
+    Merged merged[GROUP];
+#pragma unroll
+    for (int h = 0; h < GROUP; ++h) total[h] = 0.f;
+
+    int low = 0, high = 0;                            // the keys of the segment that the row sees
+    auto locate = [&](int tile) {
+        if (t < TILE) {
+            const int u = tile * TILE + t;
+            const float *key = nullptr, *value = nullptr;
+            if (u >= low && u <= high) key_at(a, u, start, row0, slot, kv_head, d, vd, key, value);
+            keys_at[t] = key;
+            values_at[t] = value;
+        }
+    };
+    auto copy = [&](const float* const* from, float* to, int width, int stride) {
+        const int pieces = width / 4;
+        for (int i = t; i < TILE * pieces; i += THREADS) {
+            const int key = i / pieces, c = (i - key * pieces) * 4;
+            copy16(to + key * stride + c, from[key] ? from[key] + c : nullptr, (const float*)a.q);
+        }
+        commit_copies();
+    };
+
+    for (int segment = first_segment + blockIdx.z; segment <= last_segment; segment += args.shares) {
+        low = max(first, segment * SEGMENT);
+        high = min(position, segment * SEGMENT + SEGMENT - 1);
+        if (t < heads) {
+            top[t] = a.weight_bias ? 0.f : -INFINITY;
+            sum[t] = 0.f;
+        }
+#pragma unroll
+        for (int h = 0; h < GROUP; ++h) acc[h] = 0.f;
+        const int last = high / TILE;
+        locate(low / TILE);
+        __syncthreads();
+        copy(keys_at, keys, d, pitch);
+        for (int tile = low / TILE; tile <= last; ++tile) {
+            copy(values_at, values, vd, vd);
+            wait_copies<1>();
+            __syncthreads();                              // the keys are there (and the query)
+            {
+                const int key = t % TILE, u = tile * TILE + key;
+                float dots[GROUP / 2];
+#pragma unroll
+                for (int i = 0; i < GROUP / 2; ++i) dots[i] = 0.f;
+                for (int k = 0; k < d; k += 4) {
+                    const float4 b = *reinterpret_cast<const float4*>(keys + key * pitch + k);
+#pragma unroll
+                    for (int i = 0; i < GROUP / 2; ++i) {
+                        const int h = t / TILE + 2 * i;
+                        if (h < heads) {
+                            const float4 q = *reinterpret_cast<const float4*>(&query[h][k]);
+                            dots[i] = fmaf(q.x, b.x, dots[i]);
+                            dots[i] = fmaf(q.y, b.y, dots[i]);
+                            dots[i] = fmaf(q.z, b.z, dots[i]);
+                            dots[i] = fmaf(q.w, b.w, dots[i]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < GROUP / 2; ++i) {
+                    const int h = t / TILE + 2 * i;
+                    if (h < heads) scores[h][key] = u >= low && u <= high ? score_of(a, dots[i], head0 + h, position, u) : -INFINITY;
+                }
+            }
+            if (tile < last) {
+                __syncthreads();                          // (every value of this tile has been asked for)
+                locate(tile + 1);
+            }
+            __syncthreads();
+            if (tile < last) copy(keys_at, keys, d, pitch);
+            else commit_copies();
+            if (t < 4 * GROUP) {                          // four threads a head: the whole warp takes part in the shuffles
+                const int h = min(t >> 2, heads - 1);
+                float highest = -INFINITY;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) highest = fmaxf(highest, scores[h][(t & 3) * 16 + i]);
+                highest = fmaxf(highest, __shfl_xor_sync(0xffffffffu, highest, 1));
+                highest = fmaxf(highest, __shfl_xor_sync(0xffffffffu, highest, 2));
+                const float before = top[h], next = a.weight_bias ? 0.f : fmaxf(before, highest);
+                __syncwarp();
+                if ((t & 3) == 0 && t >> 2 < heads) {
+                    top[h] = next;
+                    scale[h] = shrink(before, next);
+                }
+            }
+            __syncthreads();
+            for (int i = t; i < heads * TILE; i += THREADS)
+                scores[i / TILE][i % TILE] = weight_of(a, scores[i / TILE][i % TILE], head0 + i / TILE, top[i / TILE]);
+            wait_copies<1>();
+            __syncthreads();                              // the weights and the values are there
+            if (t < 4 * GROUP) {
+                const int h = min(t >> 2, heads - 1);
+                float part = 0.f;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) part = __fadd_rn(part, scores[h][(t & 3) * 16 + i]);
+                part = __fadd_rn(part, __shfl_xor_sync(0xffffffffu, part, 1));
+                part = __fadd_rn(part, __shfl_xor_sync(0xffffffffu, part, 2));
+                if ((t & 3) == 0 && t >> 2 < heads) sum[h] = __fmaf_rn(sum[h], scale[h], part);
+            }
+            if (t < vd) {
+#pragma unroll
+                for (int h = 0; h < GROUP; ++h)
+                    if (h < heads) acc[h] = __fmul_rn(acc[h], scale[h]);
+                // (keys outside the row's reach have zero weights and zero values)
+                for (int key = 0; key < TILE; key += 4) {
+                    const float v[4] = {values[key * vd + t], values[(key + 1) * vd + t], values[(key + 2) * vd + t], values[(key + 3) * vd + t]};
+#pragma unroll
+                    for (int h = 0; h < GROUP; ++h)
+                        if (h < heads) {
+                            const float4 p = *reinterpret_cast<const float4*>(&scores[h][key]);
+                            acc[h] = fmaf(p.x, v[0], acc[h]);
+                            acc[h] = fmaf(p.y, v[1], acc[h]);
+                            acc[h] = fmaf(p.z, v[2], acc[h]);
+                            acc[h] = fmaf(p.w, v[3], acc[h]);
+                        }
+                }
+            }
+            __syncthreads();                              // weights, values and statistics are free again
+        }
+        if (args.parts) {
+            float* part = args.parts + (((long long)row * a.heads + head0) * args.segments + segment - first_segment) * (vd + 2);
+#pragma unroll
+            for (int h = 0; h < GROUP; ++h, part += (long long)args.segments * (vd + 2))
+                if (h < heads) {
+                    if (t < vd) part[t] = acc[h];
+                    if (t == 0) {
+                        part[vd] = top[h];
+                        part[vd + 1] = sum[h];
+                    }
+                }
+        } else {
+#pragma unroll
+            for (int h = 0; h < GROUP; ++h)
+                if (h < heads) {
+                    merged[h].add(top[h], sum[h]);
+                    total[h] = merge(total[h], acc[h], merged[h].old, merged[h].fresh);
+                }
+        }
+        __syncthreads();                                  // the statistics are free again
+    }
+    if (!args.parts && t < vd)
+#pragma unroll
+        for (int h = 0; h < GROUP; ++h)
+            if (h < heads) {
+                float factor, divisor;
+                closing(a, head0 + h, merged[h].top, merged[h].sum, factor, divisor);
+                put(a, row, head0 + h, vd, t, total[h], factor, divisor);
+            }
+}
+
+__global__ void __launch_bounds__(THREADS) attention_f32_merge_kernel(AttentionF32Args args) {
+    const AttentionArgs& a = args.a;
+    const int vd = a.value_dim ? a.value_dim : a.head_dim, row = blockIdx.x, head = blockIdx.y, c = threadIdx.x;
+    if (c >= vd) return;
+    if (a.row_seq[row] < 0) {
+        ((float*)a.out)[row * a.ldo + (long long)head * vd + c] = 0.f;
+        return;
+    }
+    const int position = a.row_pos[row], first = first_visible(position, a.window, a.chunk);
+    const int count = position / SEGMENT - first / SEGMENT + 1;
+    const float* part = args.parts + ((long long)row * a.heads + head) * args.segments * (vd + 2);
+    Merged merged;
+    float total = 0.f;
+#pragma unroll 4
+    for (int i = 0; i < count; ++i, part += vd + 2) {
+        merged.add(part[vd], part[vd + 1]);
+        total = merge(total, part[c], merged.old, merged.fresh);
+    }
+    float factor, divisor;
+    closing(a, head, merged.top, merged.sum, factor, divisor);
+    put(a, row, head, vd, c, total, factor, divisor);
+}
+
+// ----------------------------------------------------------------------------------------------------------------- tiles
+constexpr int DEPTH = 16;        // dimensions of a stage of keys
+
+// Element (k, column) of a transposed operand stands in column (column ^ 8 (k / 4 % 4)): a warp stores four k apart of eight
+// rows, which meet no bank twice that way, and four neighbouring columns stay neighbours.
+__device__ __forceinline__ int moved(int k) { return (k >> 2 & 3) * 8; }
+// Weights by key: four neighbouring rows stand in group (row / 4) ^ (key / 4 % 8).
+__device__ __forceinline__ int weight_place(int key, int row) { return key * TILE + ((row >> 2 ^ (key >> 2 & 7)) << 2 | (row & 3)); }
+
+// TN: values of a thread (the value heads are at most 16 TN wide).
+template <int TN>
+__global__ void __launch_bounds__(THREADS, 2) attention_f32_tiles_kernel(AttentionF32Args args) {
+    const AttentionArgs& a = args.a;
+    extern __shared__ __align__(16) float shared[];
+    __shared__ const float* keys_at[2][TILE];
+    __shared__ const float* values_at[2][TILE];
+    __shared__ float exchange[2][TILE], scale[TILE], old_factor[TILE], new_factor[TILE];
+    constexpr int COLUMNS = 16 * TN;
+    const int d = a.head_dim, vd = a.value_dim ? a.value_dim : d, stages = (d + DEPTH - 1) / DEPTH;
+    float* query = shared;                                    // [stages * DEPTH][TILE]
+    float* stage = query + stages * DEPTH * TILE;             // [2][DEPTH][TILE]
+    float* values = stage + 2 * DEPTH * TILE;                 // [TILE][COLUMNS]
+    float* weights = values + TILE * COLUMNS;                 // [key][row]: scores, then weights
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int seq = blockIdx.z, head = blockIdx.y, kv_head = head / (a.heads / a.kv_heads);
+    const int length = args.seq_len[seq], tile0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * TILE;      // longest walks first
+    if (tile0 >= length) return;
+    const int row0 = a.seq_row0[seq], sequence_start = a.seq_start[seq], slot = a.seq_slot[seq];
+    const int start = a.k_step ? sequence_start : 0x7fffffff;
+    const int count = min(TILE, length - tile0), position0 = sequence_start + tile0;
+    if (a.row_seq[row0] < 0) {
+        for (int i = t; i < count * vd; i += THREADS)
+            ((float*)a.out)[(row0 + tile0 + i / vd) * a.ldo + (long long)head * vd + i % vd] = 0.f;
+        return;
+    }
+    const int low = first_visible(position0, a.window, a.chunk), high = position0 + count - 1;
+
+    const int piece_k = t % 4 * 4, piece_row = t / 4;         // (of a stage: two rows, 32 apart)
+    for (int s = 0; s < stages; ++s)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = piece_row + 32 * i, k = s * DEPTH + piece_k;
+            float4 four = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r < count && k < d) four = *reinterpret_cast<const float4*>((const float*)a.q + (row0 + tile0 + r) * a.ldq + (long long)head * d + k);
+            const float e[4] = {four.x, four.y, four.z, four.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) query[(k + j) * TILE + (r ^ moved(piece_k))] = e[j];
+        }
+
+    auto locate = [&](int tile) {
+        if (t < TILE) {
+            const int u = tile * TILE + t;
+            const float *key = nullptr, *value = nullptr;
+            if (u >= low && u <= high) key_at(a, u, start, row0, slot, kv_head, d, vd, key, value);
+            keys_at[tile & 1][t] = key;
+            values_at[tile & 1][t] = value;
+        }
+    };
+    float held[2][4];
+    auto load_keys = [&](int tile, int s) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float* key = keys_at[tile & 1][piece_row + 32 * i];
+            float4 four = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (key && s * DEPTH + piece_k < d) four = *reinterpret_cast<const float4*>(key + s * DEPTH + piece_k);
+            held[i][0] = four.x; held[i][1] = four.y; held[i][2] = four.z; held[i][3] = four.w;
+        }
+    };
+
+    // The rows of a thread's outputs: first_row + 16 h + 0..3 (h: 0, 1). Its keys: first_key + 0..3; its values:
+    // first_value + 32 g + 0..3.
+    const int first_row = (warp >> 1) * 32 + (lane >> 3) * 4;
+    const int first_key = (warp & 1) * 32 + (lane & 7) * 4, first_value = (warp & 1) * (8 * TN) + (lane & 7) * 4;
+    float acc[8][TN], total[8][TN];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = total[i][j] = 0.f;
+    // The statistics of a row are kept by two threads, one for either half of a tile's keys.
+    const int own_row = t % TILE, half = t / TILE;
+    float top = a.weight_bias ? 0.f : -INFINITY, sum = 0.f;
+    Merged merged;
+
+    const int first_tile = low / TILE, last_tile = high / TILE;
+    locate(first_tile);
+    __syncthreads();
+    load_keys(first_tile, 0);
+    for (int tile = first_tile; tile <= last_tile; ++tile) {
+        // Values on their way while the scores are computed.
+        for (int i = t; i < TILE * (COLUMNS / 4); i += THREADS) {
+            const int key = i / (COLUMNS / 4), c = i % (COLUMNS / 4) * 4;
+            const float* value = values_at[tile & 1][key];
+            copy16(values + key * COLUMNS + c, value && c < vd ? value + c : nullptr, (const float*)a.q);
+        }
+        commit_copies();
+        float s[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+        for (int st = 0; st < stages; ++st) {
+            float* current = stage + (st & 1) * DEPTH * TILE;
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) current[(piece_k + e) * TILE + ((piece_row ^ moved(piece_k)) + 32 * i)] = held[i][e];
+            if (st + 1 < stages) load_keys(tile, st + 1);
+            else if (tile < last_tile) locate(tile + 1);
+            __syncthreads();
+            const float* rows = query + st * DEPTH * TILE;
+#pragma unroll
+            for (int k = 0; k < DEPTH; ++k) {
+                float q[8], b[4];
+                *reinterpret_cast<float4*>(q) = *reinterpret_cast<const float4*>(rows + k * TILE + (first_row ^ moved(k)));
+                *reinterpret_cast<float4*>(q + 4) = *reinterpret_cast<const float4*>(rows + k * TILE + (first_row ^ moved(k) ^ 16));
+                *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(current + k * TILE + (first_key ^ moved(k)));
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) s[i][j] = fmaf(q[i], b[j], s[i][j]);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int u = tile * TILE + first_key + j;
+                float four[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int r = first_row + 16 * h + i, position = position0 + r;
+                    const bool seen = r < count && u <= position && u >= first_visible(position, a.window, a.chunk);
+                    four[i] = seen ? score_of(a, s[4 * h + i][j], head, position, u) : -INFINITY;
+                }
+                *reinterpret_cast<float4*>(weights + weight_place(first_key + j, first_row + 16 * h)) = make_float4(four[0], four[1], four[2], four[3]);
+            }
+        __syncthreads();
+        float highest = -INFINITY;
+#pragma unroll 8
+        for (int key = 0; key < TILE / 2; ++key) highest = fmaxf(highest, weights[weight_place(half * 32 + key, own_row)]);
+        exchange[half][own_row] = highest;
+        if (tile < last_tile) load_keys(tile + 1, 0);         // (located before the last barrier but one)
+        __syncthreads();
+        const float next = a.weight_bias ? 0.f : fmaxf(top, fmaxf(highest, exchange[half ^ 1][own_row]));
+        const float factor = shrink(top, next);
+        top = next;
+        if (!half) scale[own_row] = factor;
+        float parts[2] = {0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll 8
+            for (int key = 0; key < 16; ++key) {
+                float* place = weights + weight_place(half * 32 + j * 16 + key, own_row);
+                const float weight = weight_of(a, *place, head, top);
+                *place = weight;
+                parts[j] = __fadd_rn(parts[j], weight);
+            }
+        const float mine = __fadd_rn(parts[0], parts[1]);
+        __syncthreads();                                      // (the maxima have been read)
+        exchange[half][own_row] = mine;
+        wait_copies<0>();
+        __syncthreads();                                      // weights, values, factors
+        const float theirs = exchange[half ^ 1][own_row];
+        sum = __fmaf_rn(sum, factor, half ? __fadd_rn(theirs, mine) : __fadd_rn(mine, theirs));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float c = scale[first_row + (i / 4) * 16 + i % 4];
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = __fmul_rn(acc[i][j], c);
+        }
+        // A tile whose keys not every row sees: a key that a row does not see is left out of its sum (its value may be anything).
+        const bool whole = tile * TILE + TILE - 1 <= position0 && tile * TILE >= first_visible(high, a.window, a.chunk) && count == TILE;
+        auto accumulate = [&](auto masked) {
+#pragma unroll 4
+            for (int key = 0; key < TILE; ++key) {
+                float p[8], v[TN];
+                *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(weights + weight_place(key, first_row));
+                *reinterpret_cast<float4*>(p + 4) = *reinterpret_cast<const float4*>(weights + weight_place(key, first_row + 16));
+#pragma unroll
+                for (int g = 0; g < TN; g += 4) *reinterpret_cast<float4*>(v + g) = *reinterpret_cast<const float4*>(values + key * COLUMNS + first_value + 8 * g);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if constexpr (decltype(masked)::value) {
+                        const int position = position0 + first_row + (i / 4) * 16 + i % 4, u = tile * TILE + key;
+                        if (u > position || u < first_visible(position, a.window, a.chunk)) continue;
+                    }
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(p[i], v[j], acc[i][j]);
+                }
+            }
+        };
+        if (whole) accumulate(std::false_type());
+        else accumulate(std::true_type());
+        if (tile == last_tile || (tile + 1) % (SEGMENT / TILE) == 0) {
+            merged.add(top, sum);
+            if (!half) {
+                old_factor[own_row] = merged.old;
+                new_factor[own_row] = merged.fresh;
+            }
+            top = a.weight_bias ? 0.f : -INFINITY;
+            sum = 0.f;
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int r = first_row + (i / 4) * 16 + i % 4;
+                const float old = old_factor[r], fresh = new_factor[r];
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    total[i][j] = merge(total[i][j], acc[i][j], old, fresh);
+                    acc[i][j] = 0.f;
+                }
+            }
+        }
+        __syncthreads();                                      // weights and values are free again
+    }
+    if (!half) closing(a, head, merged.top, merged.sum, old_factor[own_row], new_factor[own_row]);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = first_row + (i / 4) * 16 + i % 4;
+        if (r >= count) continue;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int c = first_value + (j / 4) * 32 + j % 4;
+            if (c < vd) put(a, row0 + tile0 + r, head, vd, c, total[i][j], old_factor[r], new_factor[r]);
+        }
+    }
+}
+
+template <int TN> int launch_tiles(const AttentionF32Args& args, cudaStream_t stream) {
+    const AttentionArgs& a = args.a;
+    const int stages = (a.head_dim + DEPTH - 1) / DEPTH;
+    const size_t bytes = ((size_t)(stages + 2) * DEPTH * TILE + TILE * 16 * TN + TILE * TILE) * sizeof(float);
+    auto kernel = attention_f32_tiles_kernel<TN>;
+    const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (status != cudaSuccess) return (int)status;
+    return kidi_launch(kernel, dim3((args.max_new + TILE - 1) / TILE, a.heads, args.seqs), dim3(THREADS), bytes, stream, args);
+}
+}  // namespace
+
+// `tiles`: rows 64 at a time (prompts), else one by one. The result is the same bit for bit either way.
+KIDI_API int kidi_attention_f32(const AttentionF32Args* arguments, int tiles, cudaStream_t stream) {
+    const AttentionF32Args& args = *arguments;
+    const AttentionArgs& a = args.a;
+    if (a.rows <= 0) return 0;
+    const int vd = a.value_dim ? a.value_dim : a.head_dim;
+    if (a.head_dim <= 0 || a.head_dim > 128 || a.head_dim % 4 || vd <= 0 || vd > 128 || vd % 4 || a.kv_heads <= 0 || a.heads % a.kv_heads ||
+        a.heads > 65535 || a.chunk < 0 || a.tied || (a.weight_bias && a.sinks) || (a.ldq & 3) || (a.ldkv & 3) ||
+        (((uintptr_t)a.q | (uintptr_t)a.k_step | (uintptr_t)a.v_step | (uintptr_t)a.k_cache | (uintptr_t)a.v_cache) & 15) ||
+        (a.distance_bias && (a.bias_last < 0 || a.bias_stride <= a.bias_last)) || args.seqs <= 0)
+        return KIDI_REFUSED_SIZE;
+    if (tiles) {
+        if (args.seqs > 65535 || args.max_new <= 0) return KIDI_REFUSED_SIZE;
+        return vd <= 64 ? launch_tiles<4>(args, stream) : launch_tiles<8>(args, stream);
+    }
+    const int group = a.heads / a.kv_heads, blocks = (group + GROUP - 1) / GROUP;
+    if (args.segments < 1 || args.shares < 1 || args.shares > 65535 || (args.shares > 1) != (args.parts != nullptr) ||
+        a.kv_heads * blocks > 65535)
+        return KIDI_REFUSED_SIZE;
+    const size_t bytes = (size_t)TILE * (a.head_dim + KEY_PAD + vd) * sizeof(float);
+    const cudaError_t status = cudaFuncSetAttribute(attention_f32_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (status != cudaSuccess) return (int)status;
+    const int code = kidi_launch(attention_f32_rows_kernel, dim3(a.rows, a.kv_heads * blocks, args.shares), dim3(THREADS), bytes, stream, args);
+    if (code || !args.parts) return code;
+    return kidi_launch(attention_f32_merge_kernel, dim3(a.rows, a.heads), dim3(THREADS), 0, stream, args);
+}

@@ -324,7 +324,7 @@ def run(ctx, qkv, out, *, heads, kv_heads, head_dim, scale, window, kv_view, key
                               window=window, tables=tables, kv_view=kv_view, keys_in_step=keys_in_step,
                               softcap=softcap, slopes=slopes, value_dim=value_dim, sinks=sinks, gate=gate,
                               weight_bias=weight_bias, chunk=chunk, out_scale=out_scale, tied=tied, key_eps=key_eps,
-                              distance_bias=distance_bias, element_gate=element_gate)
+                              distance_bias=distance_bias, element_gate=element_gate, ctx=ctx)
         return
     if not decode and tensor_memory_fits(qkv, out, head_dim, heads, kv_heads, scale):
         common = dict(heads=heads, kv_heads=kv_heads, head_dim=head_dim, scale=scale, window=window, sinks=sinks,
@@ -469,7 +469,7 @@ class AttentionLauncher:
 
     def launch_signature(self, dtype: torch.dtype, rows: int, longest: int, device: torch.device) -> tuple:
         """What a captured decode step freezes of this launcher's choices: the form of the
-        tensor-core decode kernel (the general kernel, which the 32-bit engine runs, has none)."""
+        tensor-core decode kernel (the kernels that the 32-bit engine runs choose nothing by length)."""
         geometry = self.geometry
         if self.reshaped or not fast_fits(dtype, geometry["heads"], geometry["kv_heads"], geometry["head_dim"], True):
             return ()

@@ -165,6 +165,7 @@ def core():
                                                c_int, c_int, c_void_p]
         lib.kidi_rope_store.argtypes = [c_void_p, c_int, c_int, c_void_p]
         lib.kidi_attention_generic.argtypes = [c_void_p, c_int, c_void_p]
+        lib.kidi_attention_f32.argtypes = [c_void_p, c_int, c_void_p]
         lib.kidi_argmax.argtypes = [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p]
         lib.kidi_sample.argtypes = [c_void_p, c_void_p, c_int, c_int, c_void_p, c_ulonglong, c_void_p, c_void_p,
                                     c_void_p, c_void_p]
@@ -225,7 +226,7 @@ def core():
             getattr(lib, name).restype = c_int
         for name in ("kidi_embedding", "kidi_add_rmsnorm", "kidi_silu_gate", "kidi_gemm_simt", "kidi_add_bias",
                      "kidi_apply_row_factors", "kidi_rope_store",
-                     "kidi_attention_generic", "kidi_argmax", "kidi_sample", "kidi_advance_decode"):
+                     "kidi_attention_generic", "kidi_attention_f32", "kidi_argmax", "kidi_sample", "kidi_advance_decode"):
             getattr(lib, name).restype = c_int
         _core = lib
     return _core
@@ -262,6 +263,11 @@ class AttentionArgs(ctypes.Structure):
                 ("gate", c_void_p), ("ldg", c_longlong), ("weight_bias", c_void_p), ("chunk", c_int),
                 ("out_scale", c_float), ("tied", c_int), ("key_eps", c_float), ("distance_bias", c_void_p),
                 ("bias_stride", c_int), ("bias_last", c_int), ("element_gate", c_void_p), ("ld_element_gate", c_longlong)]
+
+
+class AttentionF32Args(ctypes.Structure):
+    _fields_ = [("a", AttentionArgs), ("seq_len", c_void_p), ("seqs", c_int), ("max_new", c_int), ("segments", c_int),
+                ("shares", c_int), ("parts", c_void_p)]
 
 
 class WideNormArgs(ctypes.Structure):
@@ -884,7 +890,7 @@ def attention_generic(qkv: torch.Tensor, out: torch.Tensor, *, heads: int, kv_he
                       sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
                       weight_bias: Optional[torch.Tensor] = None, chunk: Optional[int] = None,
                       out_scale: float = 1.0, tied: bool = False, key_eps: float = 0.0, distance_bias=None,
-                      element_gate: Optional[torch.Tensor] = None) -> None:
+                      element_gate: Optional[torch.Tensor] = None, ctx=None, tiles: Optional[bool] = None) -> None:
     """Causal attention of every row of the step over its sequence's keys. Keys of the
     step's own rows are read from `qkv` when `keys_in_step` is set, earlier ones (or
     all of them) from the cache. `softcap` > 0 bounds a score s to softcap * tanh(s / softcap);
@@ -896,7 +902,9 @@ def attention_generic(qkv: torch.Tensor, out: torch.Tensor, *, heads: int, kv_he
     keys of the query's own run of `chunk` positions (counted from 0) are seen. `out_scale`: a factor on the result.
     `tied`: the k heads of qkv and of the cache are keys before their norm and the values too; a score takes the factor
     1 / sqrt(mean square of the key + `key_eps`). `distance_bias`: a `DistanceBias`. `element_gate` ([rows, heads *
-    value_dim], a view of the step's element type): the result is multiplied by its sigmoid."""
+    value_dim], a view of the step's element type): the result is multiplied by its sigmoid. `ctx` (the step's plan and
+    scratch memory): 32-bit rows of heads it takes go to the kernels of csrc/attention_f32.cu (`tiles`: in the form for
+    prompts or the one for single tokens, which give the same bits; None: the faster one)."""
     value_dim = head_dim if value_dim is None else int(value_dim)
     if sinks is not None and (sinks.dtype != torch.float32 or sinks.shape != (heads,) or not sinks.is_contiguous()
                               or sinks.device != qkv.device):
@@ -932,7 +940,66 @@ def attention_generic(qkv: torch.Tensor, out: torch.Tensor, *, heads: int, kv_he
         value_dim, _ptr(sinks), _ptr(gate), gate.stride(0) if gate is not None else 0, _ptr(weight_bias), int(chunk or 0),
         float(out_scale), 1 if tied else 0, float(key_eps), *(distance_bias.fields(heads) if distance_bias is not None else (0, 0, 0)),
         _ptr(element_gate), element_gate.stride(0) if element_gate is not None else 0)
+    if ctx is not None and attention_f32_fits(qkv, head_dim, value_dim, tied):
+        plan = ctx.plan
+        # A captured step serves sequences of any length: its launch follows what a sequence may hold, not what it holds now.
+        held = (window, chunk) if kv_view is not None and kv_view.ring_pages else (kv_view.table.shape[1] * kv_view.page_size,) \
+            if kv_view is not None and plan.is_decode else (plan.max_total,)
+        reach = min(bound for bound in (window, chunk, *held) if bound)
+        segments = attention_f32_segments(None if held == (window, chunk) else held[0], reach)
+        if tiles is None:
+            tiles = not plan.is_decode and attention_f32_tiles(rows, plan.n_seqs, plan.max_new, plan.max_total, reach, heads, kv_heads,
+                                                               _sms(qkv.device))
+        shares = 1 if tiles else attention_f32_shares(rows, heads, kv_heads, segments, value_dim, _sms(qkv.device))
+        parts = ctx.workspace("attention_f32", rows * heads * segments * (value_dim + 2)) if shares > 1 else None
+        more = AttentionF32Args(args, tables.seq_len.data_ptr(), plan.n_seqs, plan.max_new, segments, shares, _ptr(parts))
+        _check(core().kidi_attention_f32(ctypes.byref(more), 1 if tiles else 0, _stream()), "attention", 1 if parts is None else 2)
+        return
     _check(core().kidi_attention_generic(ctypes.byref(args), dtype_code(qkv.dtype), _stream()), "attention")
+
+
+def attention_f32_fits(qkv: torch.Tensor, head_dim: int, value_dim: int, tied: bool) -> bool:
+    """Whether the kernels of csrc/attention_f32.cu take a layer's heads: 32-bit, at most 128 wide, in 16-byte pieces. It
+    says the same of every step of a layer: the general kernel adds in another order."""
+    return (qkv.dtype == torch.float32 and not tied and head_dim <= 128 and value_dim <= 128 and head_dim % 4 == 0
+            and value_dim % 4 == 0 and qkv.stride(0) % 4 == 0 and qkv.data_ptr() % 16 == 0)
+
+
+def attention_f32_segments(longest: Optional[int], reach: int) -> int:
+    """The most segments of 256 keys that a row sees which sees at most `reach` keys, of a sequence of at most `longest` tokens
+    (None: of any length)."""
+    crossed = (reach + 254) // 256 + 1
+    return crossed if longest is None else min(-(-longest // 256), crossed)
+
+
+def attention_f32_shares(rows: int, heads: int, kv_heads: int, segments: int, value_dim: int, sms: int) -> int:
+    """How many blocks share a row's segments: enough for four rounds of three blocks an SM (a block without a segment ends at
+    once, and the blocks of the first segments come first), while the segments' sums stay below 256 MB."""
+    blocks = rows * kv_heads * -(-(heads // kv_heads) // 8)
+    if rows * heads * segments * (value_dim + 2) > 1 << 26:
+        return 1
+    return max(1, min(segments, -(-12 * sms // blocks)))
+
+
+# Microseconds, measured on a B200 at heads of 128: a step of 64 rows and 64 keys of a block (and what comes before the first),
+# and a tile of 64 keys of a block of one row.
+TILE_STEP_US, ROW_TILE_US = 20.0, 7.0
+
+
+def attention_f32_tiles(rows: int, seqs: int, max_new: int, max_total: int, reach: int, heads: int, kv_heads: int, sms: int) -> bool:
+    """Whether a step's rows go 64 at a time. Either form's time is about that of its fullest SM: two blocks of 64 rows that
+    walk the longest row's tiles of 64 keys, or three of one row and a segment. 32 heads over 8: 16 rows of one sequence behind
+    1,000 tokens 321 us in tiles and 70 by rows, 64 rows 292 and 178, 64 first rows 48 and 23, 500 rows behind 3,000 tokens
+    1,396 and 4,042."""
+    seen = min(max_total, reach + 63)
+    walk = -(-seqs * -(-max_new // 64) * heads // (2 * sms)) * (-(-seen // 64) + 1) * TILE_STEP_US
+    blocks = rows * kv_heads * -(-(heads // kv_heads) // 8) * attention_f32_segments(max_total, reach)
+    return walk < -(-blocks // (3 * sms)) * min(4, -(-max_total // 64)) * ROW_TILE_US
+
+
+def _sms(device: torch.device) -> int:
+    from .attention import sm_count
+    return sm_count(device)
 
 
 def argmax(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:

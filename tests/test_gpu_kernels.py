@@ -464,6 +464,85 @@ def test_attention_over_cache(kind, dtype, geometry):
                   f"{kind}: sequence {index} (start {start}, new {new}, in step {keys_in_step})")
 
 
+# Heads over key/value heads, widths of keys and values, what the layer adds: group sizes around the eight heads of a block,
+# widths around 16, 64 and 128, edges of tiles (64) and segments (256) in starts, lengths, windows and chunks.
+@pytest.mark.parametrize("heads, kv_heads, dim, vdim, options", [
+    (8, 2, 128, 128, ()), (2, 2, 16, 16, ("softcap",)), (9, 1, 64, 64, ("sinks", "gate")), (18, 2, 20, 36, ("slopes",)),
+    (3, 1, 128, 64, ("window",)), (4, 4, 12, 128, ("chunk", "element_gate")), (4, 2, 64, 68, ("sigmoid", "out_scale")),
+    (6, 2, 32, 32, ("bias", "sinks", "window", "softcap"))])
+def test_attention_in_32_bit_is_the_same_however_it_is_cut(heads, kv_heads, dim, vdim, options):
+    from kidi_b200.cache.sequence_cache import KVRequest, SequenceCache
+    from kidi_b200.engine.plan import StepBatch, build_plan
+    from kidi_b200.kernels import ops
+    generator = torch.Generator().manual_seed(heads * dim)
+    draw = lambda *shape: torch.randn(*shape, generator=generator).to(DEVICE)
+    starts, news = [300, 0, 511, 64, 0, 255, 0], [1, 257, 66, 193, 1, 2, 64]
+    total = sum(news)
+    width = heads * dim + kv_heads * (dim + vdim)
+    cache = SequenceCache([[KVRequest(kv_heads, dim, None, value_dim=vdim if vdim != dim else None)]], max_tokens=4096,
+                          max_positions=2048, dtype=torch.float32, device=torch.device(DEVICE))
+    slots = [cache.acquire() for _ in starts]
+    cache.reserve([(slot, start + new) for slot, start, new in zip(slots, starts, news)])
+    cache.flush_tables()
+    view = cache.views(0)[0]
+    view.keys.copy_(draw(*view.keys.shape))
+    view.values.copy_(draw(*view.values.shape))
+    qkv = draw(total, width)
+    extra = {"softcap": 2.0} if "softcap" in options else {}
+    extra.update({"slopes": draw(heads) * 0.02} if "slopes" in options else {})
+    extra.update({"sinks": draw(heads)} if "sinks" in options else {})
+    extra.update({"weight_bias": draw(heads)} if "sigmoid" in options else {})
+    extra.update({"chunk": 192} if "chunk" in options else {})
+    extra.update({"out_scale": 0.25} if "out_scale" in options else {})
+    extra.update({"distance_bias": ops.DistanceBias(draw(100, heads))} if "bias" in options else {})
+    gates = {"gate": draw(total, heads)} if "gate" in options else {}
+    gates.update({"element_gate": draw(total, heads * vdim)} if "element_gate" in options else {})
+
+    def run(rows, step_starts, step_news, step_slots, in_step, **form):
+        plan = build_plan(StepBatch(step_slots, [[0] * new for new in step_news]), step_starts, vocab_size=10)
+        tables = Tables()
+        for name in plan.FIELDS:
+            setattr(tables, name, torch.from_numpy(getattr(plan, name)).to(DEVICE))
+        if form:
+            form["ctx"] = FakeContext(plan, tables)
+        out = torch.full((len(rows), heads * vdim), float("nan"), device=DEVICE)
+        ops.attention_generic(qkv[rows], out, heads=heads, kv_heads=kv_heads, head_dim=dim, value_dim=vdim, scale=dim ** -0.5,
+                              window=130 if "window" in options else None, tables=tables, kv_view=view, keys_in_step=in_step,
+                              **extra, **{name: gate[rows] for name, gate in gates.items()}, **form)
+        return out
+
+    everything = list(range(total))
+    for in_step in (True, False):
+        if not in_step:          # the step's keys and values into the cache
+            plan = build_plan(StepBatch(slots, [[0] * new for new in news]), starts, vocab_size=10)
+            for row in range(total):
+                seq, position = int(plan.row_seq[row]), int(plan.row_pos[row])
+                page = view.group.pages[slots[seq]][position // 64]
+                at = heads * dim
+                view.keys[page, :, position % 64] = qkv[row, at:at + kv_heads * dim].view(kv_heads, dim)
+                view.values[page, :, position % 64] = qkv[row, at + kv_heads * dim:].view(kv_heads, vdim)
+        oracle = run(everything, starts, news, slots, in_step)
+        rows = run(everything, starts, news, slots, in_step, tiles=False)
+        tiles = run(everything, starts, news, slots, in_step, tiles=True)
+        # 32-bit sums of at most 577 terms in two orders, with two exponentials: 2^-24 times 577 for either, doubled.
+        close(rows, oracle, 2 * 577 * 2.0 ** -24, "against the general kernel")
+        assert torch.equal(rows, tiles)
+    # From the cache: one sequence's last rows in a step of their own, and one row alone.
+    begin = sum(news[:2])
+    for tail in (66, 3, 1):
+        picked = list(range(begin + 66 - tail, begin + 66))
+        for form in (False, True):
+            assert torch.equal(run(picked, [511 + 66 - tail], [tail], [slots[2]], False, tiles=form), rows[picked])
+    # A key that a row does not see has no part in its result, whatever it holds.
+    if "gate" not in options and "element_gate" not in options:
+        last = begin + 65
+        qkv[last, heads * dim + kv_heads * dim:] = float("nan")
+        again = run(everything, starts, news, slots, True, tiles=True)
+        others = [row for row in everything if row != last]
+        assert torch.equal(again[others], run(everything, starts, news, slots, True, tiles=False)[others])
+        assert not again[others].isnan().any() and again[last].isnan().any()
+
+
 @pytest.mark.parametrize("kind,dtype", [("generic", torch.float32), ("tensor_core", torch.bfloat16)])
 @pytest.mark.parametrize("geometry", [(8, 2, 128, None), (6, 6, 48, None), (16, 1, 32, 90), (4, 2, 64, 64),
                                       (4, 2, 256, None), (3, 1, 192, 100)])

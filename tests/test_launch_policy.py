@@ -104,3 +104,16 @@ def test_a_32_bit_product_is_cut_into_whole_chunks_within_its_workspace(rows, fe
         assert rows <= gemm_f32.ROWS_MAX and count == chunks
     elif count < chunks:
         assert chunks * rows * features <= gemm_f32.PARTS_MAX and rows <= 65535
+
+
+def test_32_bit_attention_counts_the_segments_that_a_row_can_see():
+    from kidi_b200.kernels import ops
+    for reach in (1, 2, 63, 64, 255, 256, 257, 511, 513):
+        for longest in (None, 64, 256, 257, 1000):
+            bound = ops.attention_f32_segments(longest, reach)
+            for position in range(longest or 1100):
+                first = max(0, position - reach + 1)
+                assert position // 256 - first // 256 + 1 <= bound
+    for rows, segments in ((1, 160), (8, 160), (64, 160), (512, 64), (8, 1)):
+        shares = ops.attention_f32_shares(rows, 32, 8, segments, 128, 148)
+        assert 1 <= shares <= segments and (shares == 1 or rows * 32 * segments * 130 <= 1 << 26)
