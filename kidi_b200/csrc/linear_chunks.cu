@@ -19,6 +19,14 @@
 // partial products above 2^-24 are kept), and the read-out finishes a head: divided by its root mean square, times the SiLU
 // or sigmoid of a gate, rounded to bfloat16.
 //
+// With -DKIDI_LINEAR_GATED=1 (a state-space mixer) decay and write strength come per token and head, and heads may share
+// queries and keys:
+//
+//     o_i = d(i, -1) S^T q_i + sum over j <= i of d(i, j) b_j (q_i . k_j) v_j,     S' = d(n-1, -1) S + sum of d(n-1, j) b_j k_j v_j^T
+//
+// with d(i, j) the product of a_t over j < t <= i. It is 2 to the difference of two sums of base-2 logarithms, which are kept
+// in 64 bits (a chunk's running sum reaches some thousands; what is left of a difference near zero has to be 32-bit).
+//
 // mma.sync serves these products, not tcgen05: they are 64 x 64 x dim and dim x vdim x 64 with factors that are made in
 // registers (decays, splits), which an mma.sync operand is and a tcgen05 operand is not (it would have to go through
 // shared memory three times over).
@@ -59,6 +67,10 @@ struct LinearChunksArgs {
     long long ldf;
     float eps;
     int gate_silu;          // act: 1 SiLU, 0 sigmoid
+    // the gated build only
+    const float* coef;      // [rows, heads, coef_width]: decay and write strength of a token first
+    int coef_width, k_heads, q_heads;
+    float* keeps;           // [chunks, group]: the product of a chunk's decays
 };
 
 namespace {
@@ -72,6 +84,11 @@ constexpr int DP = D + 8, EP = E + 8;               // row pitches: ldmatrix wit
 #define KIDI_LINEAR_WIDE 0
 #endif
 constexpr bool WIDE = KIDI_LINEAR_WIDE != 0;
+#ifndef KIDI_LINEAR_GATED
+#define KIDI_LINEAR_GATED 0
+#endif
+constexpr bool GATED = KIDI_LINEAR_GATED != 0;
+static_assert(!WIDE || !GATED, "retention has one decay a head");
 constexpr int SCORE_PITCH = CHUNK + 8;
 // Shared memory of the wide read-out with slices of `slice` rows of the state: two regions, one for q in three parts and
 // later the scores in three parts, one for the slices, then k in three parts, then v; the decay's powers and the rows' sums
@@ -118,6 +135,23 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// c + the products of the COUNT parts of A with one part of B. The tensor cores cut what they add off below the largest
+// summand, so in the gated build a step's products start from zero and are added rounded: over 128 state rows the read-out's
+// error falls from 2.9e-7 to 1.1e-7 of its size (the scan of scalar_recurrence.cu: 1.3e-7) at the same speed.
+template <bool ROUNDED>
+__device__ __forceinline__ void mma_parts(float (&c)[4], const unsigned (&a)[3][4], unsigned b0, unsigned b1) {
+    if constexpr (ROUNDED) {
+        float step[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int part = 2; part >= 0; --part) mma_bf16(step, a[part], b0, b1);          // the smallest part first
+#pragma unroll
+        for (int i = 0; i < 4; ++i) c[i] += step[i];
+    } else {
+#pragma unroll
+        for (int part = 2; part >= 0; --part) mma_bf16(c, a[part], b0, b1);
+    }
+}
+
 // Two 32-bit numbers as three pairs of bfloat16 numbers that add up to them.
 __device__ __forceinline__ void split_pair(float x, float y, unsigned& first, unsigned& second, unsigned& third) {
     __nv_bfloat162 pair = __floats2bfloat162_rn(x, y);
@@ -155,6 +189,35 @@ struct Chunk {
         index = first_chunk(row0, seq) + number;
     }
 };
+
+// The gated build: logs[i] = the sum of log2 a_t over the chunk's tokens t <= i (an a of zero counts as 2^-400), writes[i] = b_i
+// (zeros past the end). The first two warps; a barrier follows.
+__device__ __forceinline__ void token_logs(const LinearChunksArgs& a, const Chunk& chunk, int head, double* logs, float* writes) {
+    if (threadIdx.x >= CHUNK) return;
+    double log = 0.0;
+    float write = 0.f;
+    if ((int)threadIdx.x < chunk.tokens) {
+        const float* coef = a.coef + ((long long)(chunk.row + threadIdx.x) * a.heads + head) * a.coef_width;
+        log = coef[0] < 1e-37f ? -400.0 : log2((double)coef[0]);
+        write = coef[1];
+    }
+#pragma unroll
+    for (int step = 1; step < 32; step <<= 1) {
+        const double before = __shfl_up_sync(0xffffffffu, log, step);
+        if ((threadIdx.x & 31) >= step) log += before;
+    }
+    logs[threadIdx.x] = log;
+    writes[threadIdx.x] = write;
+}
+// Two halves of 32 tokens: the second goes on where the first ends.
+__device__ __forceinline__ double running_log(const double* logs, int i) { return i < 32 ? logs[i] : logs[31] + logs[i]; }
+
+// 2^x for a difference of logarithms: the whole part as an exponent, the rest in 32 bits. Below 2^-126: 0.
+__device__ __forceinline__ float decayed(double x) {
+    if (x < -126.0) return 0.f;
+    const double whole = rint(x);
+    return exp2f((float)(x - whole)) * __int_as_float(((int)whole + 127) << 23);
+}
 
 // The wide build: a chunk's rows of q or k (COUNT tiles at once: they turn by the same angles) as 32-bit numbers, turned by
 // position; `take(tile, row, column, x, y)` gets two neighbouring entries, or, where half the rotary width is odd,
@@ -217,11 +280,21 @@ __global__ void __launch_bounds__(THREADS) chunk_sums_kernel(LinearChunksArgs a)
     float* wide_keys = weight + CHUNK;                      // the wide build: [64][D + 4]
     const Chunk chunk(a, blockIdx.z, blockIdx.x);
     if (!chunk.live) return;
-    const int head = a.head0 + blockIdx.y;
-    load_rows<D>(k_tile, a.k + chunk.row * a.ldk + (long long)head * D, a.ldk, chunk.tokens);
+    const int head = a.head0 + blockIdx.y, k_head = GATED ? head / (a.heads / a.k_heads) : head;
+    load_rows<D>(k_tile, a.k + chunk.row * a.ldk + (long long)k_head * D, a.ldk, chunk.tokens);
     load_rows<E>(v_tile, a.v + chunk.row * a.ldv + (long long)head * E, a.ldv, chunk.tokens);
     copy_async_commit();
-    if (threadIdx.x < CHUNK)
+    if constexpr (GATED) {
+        __shared__ double logs[CHUNK];
+        __shared__ float writes[CHUNK];
+        token_logs(a, chunk, head, logs, writes);
+        __syncthreads();
+        if (threadIdx.x < CHUNK) {
+            const double all = running_log(logs, CHUNK - 1);       // (tokens past the end change nothing)
+            weight[threadIdx.x] = writes[threadIdx.x] * decayed(all - running_log(logs, threadIdx.x));
+            if (threadIdx.x == 0) a.keeps[(long long)chunk.index * a.group + blockIdx.y] = decayed(all);
+        }
+    } else if (threadIdx.x < CHUNK)
         weight[threadIdx.x] = threadIdx.x < chunk.tokens ? powf(a.decay[head], (float)(chunk.tokens - 1 - threadIdx.x)) : 0.f;
     copy_async_wait<0>();
     __syncthreads();
@@ -271,11 +344,8 @@ __global__ void __launch_bounds__(THREADS) chunk_sums_kernel(LinearChunksArgs a)
                 if (n0 + p * 16 >= E) continue;
                 unsigned values[4];
                 ldmatrix_x4_trans(values, v_tile + (kk * 16 + within + (matrix & 1) * 8) * EP + n0 + p * 16 + (matrix >> 1) * 8);
-#pragma unroll
-                for (int s = 2; s >= 0; --s) {              // the smallest part first
-                    mma_bf16(c[2 * p], parts[s], values[0], values[1]);
-                    mma_bf16(c[2 * p + 1], parts[s], values[2], values[3]);
-                }
+                mma_parts<GATED>(c[2 * p], parts, values[0], values[1]);
+                mma_parts<GATED>(c[2 * p + 1], parts, values[2], values[3]);
             }
         }
 #pragma unroll
@@ -301,7 +371,8 @@ __global__ void __launch_bounds__(WALK_THREADS) chunk_states_kernel(LinearChunks
     const float* sums = a.sums + ((long long)first_chunk(row0, seq) * a.group + blockIdx.y) * D * E + at;
     bf16* before = a.before + 3 * (((long long)first_chunk(row0, seq) * a.group + blockIdx.y) * D * E) + at;
     float* kept = a.state + ((long long)a.seq_slot[seq] * a.heads + head) * D * E + at;
-    const float decay = a.decay[head], keep = powf(decay, (float)CHUNK);
+    const float decay = GATED ? 0.f : a.decay[head], keep = GATED ? 0.f : powf(decay, (float)CHUNK);
+    const float* keeps = GATED ? a.keeps + (long long)first_chunk(row0, seq) * a.group + blockIdx.y : nullptr;
     float4 s = *reinterpret_cast<const float4*>(kept);
     float4 ahead[AHEAD];
 #pragma unroll
@@ -319,7 +390,7 @@ __global__ void __launch_bounds__(WALK_THREADS) chunk_states_kernel(LinearChunks
                 split_pair(s.z, s.w, parts[0].y, parts[1].y, parts[2].y);
 #pragma unroll
                 for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(before + 3 * c * stride + p * (D * E)) = parts[p];
-                const float factor = c + 1 < chunks ? keep : powf(decay, (float)(count - c * CHUNK));
+                const float factor = GATED ? keeps[(long long)c * a.group] : c + 1 < chunks ? keep : powf(decay, (float)(count - c * CHUNK));
                 s.x = fmaf(factor, s.x, sum.x); s.y = fmaf(factor, s.y, sum.y);
                 s.z = fmaf(factor, s.z, sum.z); s.w = fmaf(factor, s.w, sum.w);
             }
@@ -358,12 +429,16 @@ __global__ void __launch_bounds__(THREADS) chunk_read_kernel(LinearChunksArgs a)
         }
         copy_async_commit();
     };
-    load_rows<D>(q_tile, a.q + chunk.row * a.ldq + (long long)head * D, a.ldq, chunk.tokens);
+    const int q_head = GATED ? head / (a.heads / a.q_heads) : head, k_head = GATED ? head / (a.heads / a.k_heads) : head;
+    load_rows<D>(q_tile, a.q + chunk.row * a.ldq + (long long)q_head * D, a.ldq, chunk.tokens);
     load_slice(0);
-    load_rows<D>(k_tile, a.k + chunk.row * a.ldk + (long long)head * D, a.ldk, chunk.tokens);
+    load_rows<D>(k_tile, a.k + chunk.row * a.ldk + (long long)k_head * D, a.ldk, chunk.tokens);
     load_rows<E>(v_tile, a.v + chunk.row * a.ldv + (long long)head * E, a.ldv, chunk.tokens);
     if (SLICES == 1) copy_async_commit();
-    for (int i = threadIdx.x; i <= CHUNK; i += THREADS) power[i] = powf(a.decay[head], (float)i);
+    __shared__ double logs[GATED ? CHUNK : 1];
+    __shared__ float writes[GATED ? CHUNK : 1];
+    if constexpr (GATED) token_logs(a, chunk, head, logs, writes);
+    else for (int i = threadIdx.x; i <= CHUNK; i += THREADS) power[i] = powf(a.decay[head], (float)i);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int matrix = lane >> 3, within = lane & 7;
@@ -390,18 +465,26 @@ __global__ void __launch_bounds__(THREADS) chunk_read_kernel(LinearChunksArgs a)
             for (int p = 0; p < MINE; ++p) {
                 const int column = (side + 2 * p) * 16;
                 if (column >= E) continue;
+                float step[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
                 for (int part = 2; part >= 0; --part) {
                     unsigned s[4];
                     ldmatrix_x4_trans(s, current + (part * SLICE + kk * 16 + within + (matrix & 1) * 8) * EP + column + (matrix >> 1) * 8);
-                    mma_bf16(o[2 * p], q, s[0], s[1]);
-                    mma_bf16(o[2 * p + 1], q, s[2], s[3]);
+                    mma_bf16(GATED ? step[0] : o[2 * p], q, s[0], s[1]);
+                    mma_bf16(GATED ? step[1] : o[2 * p + 1], q, s[2], s[3]);
                 }
+                if constexpr (GATED)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        o[2 * p][i] += step[0][i];
+                        o[2 * p + 1][i] += step[1][i];
+                    }
             }
         }
         __syncthreads();                                    // the slice is read: its buffer takes the one after next
     }
-    const float below = power[row + g + 1], above = power[row + g + 9];
+    const double log_below = GATED ? running_log(logs, row + g) : 0.0, log_above = GATED ? running_log(logs, row + g + 8) : 0.0;
+    const float below = GATED ? decayed(log_below) : power[row + g + 1], above = GATED ? decayed(log_above) : power[row + g + 9];
 #pragma unroll
     for (int j = 0; j < 2 * MINE; ++j) {
         o[j][0] *= below; o[j][1] *= below;
@@ -415,15 +498,24 @@ __global__ void __launch_bounds__(THREADS) chunk_read_kernel(LinearChunksArgs a)
             unsigned q[4], k[4];
             ldmatrix_x4(q, q_tile + (row + within + (matrix & 1) * 8) * DP + kk * 16 + (matrix >> 1) * 8);
             ldmatrix_x4(k, k_tile + (kt * 16 + within + (matrix >> 1) * 8) * DP + kk * 16 + (matrix & 1) * 8);
-            mma_bf16(s[0], q, k[0], k[1]);
-            mma_bf16(s[1], q, k[2], k[3]);
+            float step[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+            mma_bf16(GATED ? step[0] : s[0], q, k[0], k[1]);
+            mma_bf16(GATED ? step[1] : s[1], q, k[2], k[3]);
+            if constexpr (GATED)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    s[0][i] += step[0][i];
+                    s[1][i] += step[1][i];
+                }
         }
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int back = row + g + (i >> 1) * 8 - (kt * 16 + j * 8 + 2 * t + (i & 1));
-                s[j][i] = back >= 0 ? s[j][i] * power[back] : 0.f;
+                const int key = kt * 16 + j * 8 + 2 * t + (i & 1), back = row + g + (i >> 1) * 8 - key;
+                if constexpr (GATED)
+                    s[j][i] = back >= 0 ? s[j][i] * (writes[key] * decayed((i >> 1 ? log_above : log_below) - running_log(logs, key))) : 0.f;
+                else s[j][i] = back >= 0 ? s[j][i] * power[back] : 0.f;
             }
         unsigned parts[3][4];
         split_pair(s[0][0], s[0][1], parts[0][0], parts[1][0], parts[2][0]);
@@ -436,11 +528,8 @@ __global__ void __launch_bounds__(THREADS) chunk_read_kernel(LinearChunksArgs a)
             if (column >= E) continue;
             unsigned v[4];
             ldmatrix_x4_trans(v, v_tile + (kt * 16 + within + (matrix & 1) * 8) * EP + column + (matrix >> 1) * 8);
-#pragma unroll
-            for (int part = 2; part >= 0; --part) {
-                mma_bf16(o[2 * p], parts[part], v[0], v[1]);
-                mma_bf16(o[2 * p + 1], parts[part], v[2], v[3]);
-            }
+            mma_parts<GATED>(o[2 * p], parts, v[0], v[1]);
+            mma_parts<GATED>(o[2 * p + 1], parts, v[2], v[3]);
         }
     }
     float* out = a.out + (long long)chunk.row * a.heads * E + (long long)head * E;
@@ -698,6 +787,8 @@ KIDI_API int kidi_linear_chunks(const LinearChunksArgs* args, cudaStream_t strea
     if (a.heads <= 0 || a.seqs > 65535 || a.group < 1 || a.group > 65535 || a.head0 < 0 || a.head0 + a.group > a.heads ||
         (a.ldq & 7) || (a.ldk & 7) || (a.ldv & 7) || ((uintptr_t)a.q & 15) || ((uintptr_t)a.k & 15) || ((uintptr_t)a.v & 15) ||
         ((uintptr_t)a.state & 15) || ((uintptr_t)a.out & 15) || ((uintptr_t)a.sums & 15) || ((uintptr_t)a.before & 15))
+        return KIDI_REFUSED_SIZE;
+    if (GATED && (!a.coef || a.coef_width < 2 || !a.keeps || a.k_heads < 1 || a.q_heads < 1 || a.heads % a.k_heads || a.heads % a.q_heads))
         return KIDI_REFUSED_SIZE;
 #if KIDI_LINEAR_WIDE
     if (!a.row_pos || !a.gate || !a.finished || (a.ldg & 1) || (a.ldf & 1) || ((uintptr_t)a.gate & 3) ||

@@ -35,7 +35,8 @@ class LinearChunksArgs(ctypes.Structure):
                 ("seq_len", c_void_p), ("seqs", c_int), ("heads", c_int), ("head0", c_int), ("group", c_int),
                 ("max_chunks", c_int), ("cos_table", c_void_p), ("sin_table", c_void_p), ("row_pos", c_void_p),
                 ("rotary_dim", c_int), ("key_scale", c_float), ("gate", c_void_p), ("ldg", c_longlong),
-                ("finished", c_void_p), ("ldf", c_longlong), ("eps", c_float), ("gate_silu", c_int)]
+                ("finished", c_void_p), ("ldf", c_longlong), ("eps", c_float), ("gate_silu", c_int), ("coef", c_void_p),
+                ("coef_width", c_int), ("k_heads", c_int), ("q_heads", c_int), ("keeps", c_void_p)]
 
 
 # The chunked form on the tensor cores: steps whose longest sequence brings at least this many tokens (0: never).
@@ -47,22 +48,23 @@ _library = None
 _chunk_libraries: Dict[tuple, ctypes.CDLL] = {}
 
 
-def chunk_library_request(dim: int, vdim: int, wide: bool = False):
+def chunk_library_request(dim: int, vdim: int, wide: bool = False, gated: bool = False):
     """(name, sources, definitions) of the chunked kernels for one pair of head widths (`wide`: with rotated and scaled,
-    hence 32-bit, queries and keys and a finish head by head)."""
-    defines = {"KIDI_LINEAR_DIM": dim, "KIDI_LINEAR_VDIM": vdim, **({"KIDI_LINEAR_WIDE": 1} if wide else {})}
-    return f"linear_chunks_d{dim}_v{vdim}" + ("_wide" if wide else ""), ("linear_chunks.cu",), defines
+    hence 32-bit, queries and keys and a finish head by head; `gated`: with a decay and a write strength per token)."""
+    defines = {"KIDI_LINEAR_DIM": dim, "KIDI_LINEAR_VDIM": vdim, **({"KIDI_LINEAR_WIDE": 1} if wide else {}),
+               **({"KIDI_LINEAR_GATED": 1} if gated else {})}
+    return f"linear_chunks_d{dim}_v{vdim}" + ("_wide" if wide else "_gated" if gated else ""), ("linear_chunks.cu",), defines
 
 
-def chunk_library(dim: int, vdim: int, wide: bool = False) -> ctypes.CDLL:
-    lib = _chunk_libraries.get((dim, vdim, wide))
+def chunk_library(dim: int, vdim: int, wide: bool = False, gated: bool = False) -> ctypes.CDLL:
+    lib = _chunk_libraries.get((dim, vdim, wide, gated))
     if lib is None:
-        lib = load_library(*chunk_library_request(dim, vdim, wide))
+        lib = load_library(*chunk_library_request(dim, vdim, wide, gated))
         lib.kidi_linear_chunks.argtypes = [c_void_p, c_void_p]
         lib.kidi_linear_chunks.restype = c_int
         lib.kidi_linear_chunks_scratch.argtypes = [c_int, c_int, c_int]
         lib.kidi_linear_chunks_scratch.restype = c_longlong
-        _chunk_libraries[(dim, vdim, wide)] = lib
+        _chunk_libraries[(dim, vdim, wide, gated)] = lib
     return lib
 
 
@@ -134,6 +136,33 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: t
     return out
 
 
+# The fewest tokens of a step's longest sequence from which the chunked form with gates per token is the faster one: at 32
+# heads of 128 x 64 the scan takes 15 us for 64 tokens, 26 for 128 and 229 for 1,300, the three kernels 20, 20 and 57 (16 heads
+# of 64 x 64: 11 and 17 at 64 tokens, 52 and 19 at 400).
+MIN_GATED_TOKENS = 96
+
+
+def gated_recurrence(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: torch.Tensor, state: torch.Tensor, *, heads: int,
+                     k_heads: int, q_heads: int, dim: int, vdim: int, tables, seqs: int, longest: int) -> torch.Tensor:
+    """`scalar_recurrence` (S_t = a_t S_(t-1) + b_t k_t v_t^T, o_t = S_t^T q_t) of steps whose longest sequence brings
+    `longest` tokens: in chunks on the tensor cores where the rows allow it, else as the scan."""
+    if not (0 < MIN_CHUNKED_TOKENS and MIN_GATED_TOKENS <= longest and coef.dim() == 3 and chunks_fit(q, k, v, dim, vdim, longest)):
+        return scalar_recurrence.scalar_recurrence(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim,
+                                                   vdim=vdim, tables=tables, seqs=seqs)
+    scalar_recurrence.check(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim, vdim=vdim)
+    rows = v.shape[0]
+    out = torch.empty((rows, heads * vdim), dtype=torch.float32, device=v.device)
+    for head0, here, sums, before, lib in _head_groups(rows, seqs, heads, dim, vdim, v.device, False, True):
+        keeps = torch.empty((rows // CHUNK + seqs + 1) * here, dtype=torch.float32, device=v.device)
+        args = LinearChunksArgs(
+            q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), 0, state.data_ptr(), out.data_ptr(),
+            sums, before, tables.row_seq.data_ptr(), tables.seq_slot.data_ptr(), tables.seq_row0.data_ptr(),
+            tables.seq_len.data_ptr(), seqs, heads, head0, here, -(-longest // CHUNK), coef=coef.data_ptr(),
+            coef_width=coef.shape[2], k_heads=k_heads, q_heads=q_heads, keeps=keeps.data_ptr())
+        _check(lib.kidi_linear_chunks(ctypes.byref(args), ops._stream()), "scalar_recurrence", 3)
+    return out
+
+
 FINISH_SPANS = 8                        # blocks of 32 columns that finish a head together in the one-token kernel
 
 
@@ -195,10 +224,10 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: torch.Ten
     return head_norm_gate(read, None, gate, heads, eps, 1.0, silu, out)
 
 
-def _head_groups(rows: int, seqs: int, heads: int, dim: int, vdim: int, device, wide: bool):
+def _head_groups(rows: int, seqs: int, heads: int, dim: int, vdim: int, device, wide: bool, gated: bool = False):
     """(first head, heads, address of the sums, address of the states before the chunks, library) for every launch of the
     chunked form: the heads of a step in groups that need at most SCRATCH_FLOATS of scratch memory, which they share."""
-    lib = chunk_library(dim, vdim, wide)
+    lib = chunk_library(dim, vdim, wide, gated)
     group = heads
     while group > 1 and lib.kidi_linear_chunks_scratch(rows, seqs, group) > SCRATCH_FLOATS:
         group = -(-group // 2)

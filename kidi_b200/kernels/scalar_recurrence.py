@@ -70,16 +70,9 @@ def _float_tensor(x: torch.Tensor, shape, what: str) -> None:
         raise invalid_argument(f"{what} must be a contiguous float32 tensor of shape {tuple(shape)}")
 
 
-def scalar_recurrence(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: Optional[torch.Tensor],
-                      state: torch.Tensor, *, heads: int, k_heads: int, q_heads: int, dim: int, vdim: int,
-                      extra: int = 0, q_scale: float = 1.0, tables, seqs: int,
-                      decay: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """S_t = a_t S_(t-1) + b_t k_t (v_t, 1 if `extra`)^T and o_t = S_t^T (q_scale q_t) for every sequence's rows of
-    the step, from and into `state` [slots + 1, heads, dim, vdim + extra] (float32). k [rows, k_heads * dim],
-    q [rows, q_heads * dim], v [rows, heads * vdim] are views of the step's element type (head h reads key head
-    h // (heads / k_heads), likewise q); coef float32 [rows, heads, >= 2] holds (a_t, b_t), or `decay`
-    (float32 [heads], coef None) holds a_t for every token and b_t is 1. Returns the read-out, float32
-    [rows, heads * (vdim + extra)]."""
+def check(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: Optional[torch.Tensor], state: torch.Tensor, *, heads: int,
+          k_heads: int, q_heads: int, dim: int, vdim: int, extra: int = 0, decay: Optional[torch.Tensor] = None) -> None:
+    """Raises where the operands of a recurrence do not fit one another."""
     ops._need_cuda(k, q, v, coef, state)
     rows = v.shape[0]
     for tensor, width, what in ((k, k_heads * dim, "keys"), (q, q_heads * dim, "queries"), (v, heads * vdim, "values")):
@@ -97,6 +90,20 @@ def scalar_recurrence(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: O
         raise invalid_argument("scalar recurrence: the state is float32 [slots, heads, dim, vdim (+ 1)]")
     if dim > MAX_DIM:
         raise invalid_argument(f"scalar recurrence: the kernel takes up to {MAX_DIM} state rows a head")
+
+
+def scalar_recurrence(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: Optional[torch.Tensor],
+                      state: torch.Tensor, *, heads: int, k_heads: int, q_heads: int, dim: int, vdim: int,
+                      extra: int = 0, q_scale: float = 1.0, tables, seqs: int,
+                      decay: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """S_t = a_t S_(t-1) + b_t k_t (v_t, 1 if `extra`)^T and o_t = S_t^T (q_scale q_t) for every sequence's rows of
+    the step, from and into `state` [slots + 1, heads, dim, vdim + extra] (float32). k [rows, k_heads * dim],
+    q [rows, q_heads * dim], v [rows, heads * vdim] are views of the step's element type (head h reads key head
+    h // (heads / k_heads), likewise q); coef float32 [rows, heads, >= 2] holds (a_t, b_t), or `decay`
+    (float32 [heads], coef None) holds a_t for every token and b_t is 1. Returns the read-out, float32
+    [rows, heads * (vdim + extra)]."""
+    check(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim, vdim=vdim, extra=extra, decay=decay)
+    rows = v.shape[0]
     out = torch.empty((rows, heads * (vdim + extra)), dtype=torch.float32, device=v.device)
     args = ScalarRecurrenceArgs(k.data_ptr(), k.stride(0), q.data_ptr(), q.stride(0), v.data_ptr(), v.stride(0),
                                 coef.data_ptr() if coef is not None else 0, state.data_ptr(), out.data_ptr(), tables.row_seq.data_ptr(),

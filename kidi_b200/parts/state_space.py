@@ -26,6 +26,7 @@ import torch
 from ..cache.sequence_cache import StateRequest
 from ..errors import invalid_argument, unsupported
 from ..kernels import scalar_recurrence as kernels
+from ..kernels.linear_attention import gated_recurrence
 from .base import Part, plain_rows
 from .linear import Linear
 from .registry import register_part
@@ -110,9 +111,9 @@ class StateSpaceMixer(Part):
                                    one_token=plan.is_decode)
         coef = kernels.state_space_gates(steps[:, :self.heads], self.dt_bias, self.a_log)
         values = mixed[:, :inner]
-        read = kernels.scalar_recurrence(mixed[:, inner:inner + span], mixed[:, inner + span:], values, coef, views[0],
-                                         heads=self.heads, k_heads=self.groups, q_heads=self.groups, dim=self.state,
-                                         vdim=self.vdim, tables=ctx.tables, seqs=plan.n_seqs)
+        read = gated_recurrence(mixed[:, inner:inner + span], mixed[:, inner + span:], values, coef, views[0],
+                                heads=self.heads, k_heads=self.groups, q_heads=self.groups, dim=self.state,
+                                vdim=self.vdim, tables=ctx.tables, seqs=plan.n_seqs, longest=plan.max_new)
         gated = kernels.state_space_finish(read, values, z, self.skip, self.norm, heads=self.heads, vdim=self.vdim,
                                            parts=self.norm_groups, eps=self.eps)
         return self.out.forward(gated)

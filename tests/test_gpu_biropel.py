@@ -242,6 +242,56 @@ def test_the_recurrence_kernel(dtype, heads, k_heads, dim, vdim, extra):
             assert torch.equal(found[b], results[0][b])
 
 
+@pytest.mark.parametrize("heads, k_heads, dim, vdim", [(4, 1, 128, 64), (6, 2, 64, 64), (3, 3, 16, 16), (2, 1, 128, 128)])
+def test_the_recurrence_in_chunks(heads, k_heads, dim, vdim):
+    """Chunks of 64 tokens on the tensor cores against the loop in 64 bits and beside the scan: lengths around a chunk, decays
+    of 0, 1 and everything between, a state that goes on from step to step, other slots' states left alone."""
+    from kidi_b200.kernels import linear_attention, ops, scalar_recurrence
+    generator = torch.Generator().manual_seed(dim + heads)
+    lengths, slots = (65, 1, 200, 64, 129), (2, 0, 4, 5, 1)
+    total = sum(lengths)
+    k, q = (torch.randn(total, k_heads * dim, generator=generator).to(torch.bfloat16).cuda() for _ in range(2))
+    v = torch.randn(total, heads * vdim, generator=generator).to(torch.bfloat16).cuda()
+    rate = torch.exp(4 * torch.randn(1, heads, generator=generator))
+    decay = torch.exp(-rate * torch.rand(total, heads, generator=generator) * 0.1)
+    decay[::37], decay[5::41] = 0.0, 1.0
+    coef = torch.stack([decay, torch.rand(total, heads, generator=generator)], -1).contiguous().cuda()
+    first = torch.randn(6, heads, dim, vdim, generator=generator).cuda()
+
+    def loop(state):
+        kept, out = state.double(), torch.empty(total, heads, vdim, dtype=torch.float64, device="cuda")
+        at = 0
+        for count, slot in zip(lengths, slots):
+            S = kept[slot].clone()
+            for row in range(at, at + count):
+                keys = k[row].double().view(k_heads, dim).repeat_interleave(heads // k_heads, 0)
+                queries = q[row].double().view(k_heads, dim).repeat_interleave(heads // k_heads, 0)
+                a, b = coef[row].double().unbind(-1)
+                S = a[:, None, None] * S + b[:, None, None] * keys[:, :, None] * v[row].double().view(heads, 1, vdim)
+                out[row] = torch.einsum("hde,hd->he", S, queries)
+            kept[slot] = S
+            at += count
+        return kept, out.reshape(total, -1)
+
+    common = dict(heads=heads, k_heads=k_heads, q_heads=k_heads, dim=dim, vdim=vdim, tables=step_tables(lengths, [0] * 5, slots), seqs=5)
+    state = [first.clone(), first.clone()]
+    errors = []
+    for _ in range(2):              # the second step goes on from the first one's state
+        want_state, want = loop(state[0])
+        with ops.record_launches() as names:
+            chunks = linear_attention.gated_recurrence(k, q, v, coef, state[0], longest=max(lengths), **common)
+        assert names == ["scalar_recurrence"]
+        scan = scalar_recurrence.scalar_recurrence(k, q, v, coef, state[1], **common)
+        # 32-bit sums of up to 200 tokens and 128 state rows, a rounding of at most 2^-24 a term in a random walk, and factors
+        # in three parts that leave 2^-24: some 2^-24 sqrt(200) at the worst, 1.1e-7 and 1.4e-7 measured.
+        for found in (chunks, scan):
+            errors.append(float((found.double() - want).norm() / want.norm()))
+            assert errors[-1] <= 1e-6, errors
+        for held in state[:1]:
+            assert float((held.double() - want_state).norm() / want_state.norm()) <= 1e-6
+        assert torch.equal(state[0][3], first[3])
+
+
 # ------------------------------------------------------------------ one layer of each kind
 LEFT = dict(heads=4, kv_heads=2, dim=16, vdim=24, scale=0.3)
 LAYERS = {
