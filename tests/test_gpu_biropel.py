@@ -242,6 +242,49 @@ def test_the_recurrence_kernel(dtype, heads, k_heads, dim, vdim, extra):
             assert torch.equal(found[b], results[0][b])
 
 
+@pytest.mark.parametrize("taps", [2, 3, 4])
+def test_the_short_convolution_in_pieces_of_eight_channels(taps):
+    """Rows on 16-byte boundaries give the bits of rows that start anywhere: portions around four rows, shorter than the taps,
+    sequences that meet in a thread's rows."""
+    from kidi_b200.kernels import scalar_recurrence as kernels
+    generator = torch.Generator().manual_seed(taps)
+    channels, sizes, starts, slots = 72, [1, 2, 3, 4, 5, 1, 9, 130], [0, 1, 5, 0, 0, 2, 300, 0], [3, 1, 0, 2, 7, 6, 5, 4]
+    packed = torch.randn(sum(sizes), channels + 8, generator=generator).to(torch.bfloat16).cuda()
+    weight, bias = torch.randn(channels, taps, generator=generator).cuda(), torch.randn(channels, generator=generator).cuda()
+    first = torch.randn(9, taps - 1, channels, generator=generator).to(torch.bfloat16).cuda()
+    tables = step_tables(sizes, starts, slots)
+    for silu in (True, False):
+        for add in (bias, None):
+            found, states = [], []
+            for offset in (8, 1):
+                wide = torch.zeros(packed.shape[0], channels + 8, dtype=torch.bfloat16, device="cuda")
+                wide[:, offset:offset + channels] = packed[:, :channels]
+                state = first.clone()
+                found.append(kernels.short_conv(wide[:, offset:offset + channels], weight, add, state, silu=silu, tables=tables, seqs=len(sizes)))
+                states.append(state)
+            assert torch.equal(found[0], found[1]) and torch.equal(states[0], states[1])
+
+
+@pytest.mark.parametrize("heads, vdim, parts", [(2, 8, 2), (4, 64, 1), (4, 64, 8), (9, 40, 1), (16, 64, 1), (33, 32, 1)])
+def test_the_state_space_finish_in_pieces_of_eight_entries(heads, vdim, parts):
+    """Parts of 8 to 1,056 entries (the last too wide for it), rows on 16-byte boundaries and rows that start anywhere."""
+    from kidi_b200.kernels import scalar_recurrence as kernels
+    generator = torch.Generator().manual_seed(heads)
+    rows, inner = 13, heads * vdim
+    read, weight = torch.randn(rows, inner, generator=generator).cuda(), torch.randn(inner, generator=generator).cuda()
+    skip = torch.randn(heads, generator=generator).cuda()
+    both = torch.randn(rows, 2 * inner, generator=generator).to(torch.bfloat16).cuda()
+    x, z = both[:, :inner], both[:, inner:]
+    y = (read.double() + skip.double().repeat_interleave(vdim) * x.double()) * torch.nn.functional.silu(z.double())
+    y = y.view(rows, parts, -1)
+    want = (y / (y.square().mean(-1, keepdim=True) + 1e-5).sqrt()).view(rows, inner) * weight.double()
+    odd = torch.zeros(rows, 2 * inner + 1, dtype=torch.bfloat16, device="cuda")[:, 1:].copy_(both)
+    for gate in (both, odd):
+        found = kernels.state_space_finish(read, gate[:, :inner], gate[:, inner:], skip, weight, heads=heads, vdim=vdim, parts=parts, eps=1e-5)
+        # one rounding to bfloat16 (2^-9) of a value with a 32-bit error (below 2^-18)
+        assert bool(((found.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
+
+
 @pytest.mark.parametrize("heads, k_heads, dim, vdim", [(4, 1, 128, 64), (6, 2, 64, 64), (3, 3, 16, 16), (2, 1, 128, 128)])
 def test_the_recurrence_in_chunks(heads, k_heads, dim, vdim):
     """Chunks of 64 tokens on the tensor cores against the loop in 64 bits and beside the scan: lengths around a chunk, decays
