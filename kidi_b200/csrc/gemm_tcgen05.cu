@@ -188,8 +188,29 @@ struct Params {
     const int* group_of_tile;   // [token tiles] or null: the tile's tokens take the weight rows from group * group_rows on
                                 // (a tile whose group is negative holds no tokens and is left out)
     int group_rows;
+    const int* used_of_tile;    // [token tiles] or null (all of them): the rows of a tile that are wanted, from its first one on
     GateShape gate;             // the gated form's activation (all zero: SiLU)
 };
+
+// Weights in groups: the rows' tiles are 128 tokens high. A block takes two neighbouring tiles of one group at once (the
+// weights are loaded once for both, and at 128 tokens a tile the operands' way from the L2 is what bounds it: 32 KB for 256
+// cycles of matrix instructions against 48 KB for 512), and of those the tokens that are wanted, in steps of 16. Which tiles
+// begin such a piece of work every block finds out for itself, in shared memory.
+constexpr int GROUP_TILE = 128, MOST_GROUP_TILES = 1024;
+constexpr int GROUP_BOX = 64;        // tokens of a copy
+struct GroupPieces {
+    int count;                       // pieces of work
+    short tile[MOST_GROUP_TILES];    // a piece's first tile
+    short group[MOST_GROUP_TILES];   // of a tile (-1: none), then of a piece
+    unsigned char wanted[MOST_GROUP_TILES];   // of a tile in rows, then of a piece in steps of 16 tokens
+};
+
+// Shared memory of a block: the stages, the gated epilogue's exchange buffer and two buffers of results on their way out;
+// behind them (`pieces`) what a block knows of weights in groups.
+template <int BN, int STAGES> __host__ __device__ constexpr size_t shared_floor() {
+    constexpr int columns = epilogue_columns<BN>();
+    return (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 64 * (columns + 1) * sizeof(float) + 2 * columns * BM * sizeof(bf16);
+}
 
 // Tiles are numbered so that the blocks at work at one time share few weight tiles and few token
 // tiles (see `locate`). With a tile for every block, block b takes whole tiles b,
@@ -222,6 +243,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     __shared__ unsigned long long full_bar[STAGES], empty_bar[STAGES], ready_bar[2], drained_bar[2];
     __shared__ unsigned tmem_base_slot;
     __shared__ int gave_up, is_last;
+    constexpr bool PIECES = BN == 256 && sizeof(TY) == 2;      // the build that serves weights in groups
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Where block c's piece of the line begins, and which block holds k-block g of the line.
@@ -235,21 +257,72 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     // feature tile (the blocks at work at one time share few weight tiles and eight token tiles,
     // however long the prompt), column after column.
     const int feature_tiles = (int)(p.tiles / p.token_tiles);
+    const bool grouped = PIECES && p.group_of_tile;
+    GroupPieces* pieces = reinterpret_cast<GroupPieces*>(tiles + shared_floor<BN, STAGES>());      // (grouped launches only)
+    if constexpr (PIECES) {
+        if (grouped) {
+            for (int i = threadIdx.x; i < p.token_tiles; i += THREADS) {
+                pieces->group[i] = (short)p.group_of_tile[i];
+                pieces->wanted[i] = p.used_of_tile ? (unsigned char)min(max(p.used_of_tile[i], 0), GROUP_TILE) : GROUP_TILE;
+            }
+            __syncthreads();
+            if (warp == 0) {
+                int count = 0;
+                for (int base = 0; base < p.token_tiles; base += 32) {
+                    const int i = base + lane;
+                    const int group = i < p.token_tiles ? pieces->group[i] : -1;
+                    int first = i;                         // of the run of the tile's group
+                    while (group >= 0 && first > 0 && pieces->group[first - 1] == group) --first;
+                    const bool begins = group >= 0 && !((i - first) & 1) && pieces->wanted[i] > 0;
+                    const unsigned all = __ballot_sync(0xffffffffu, begins);
+                    if (begins) pieces->tile[count + __popc(all & ((1u << lane) - 1))] = (short)i;
+                    count += __popc(all);
+                }
+                if (lane == 0) pieces->count = count;
+            }
+            __syncthreads();
+            // (a piece's number is at most its tile's: what is overwritten here has been read by then only if everybody reads first)
+            constexpr int MINE = (MOST_GROUP_TILES + THREADS - 1) / THREADS;
+            short group[MINE];
+            unsigned char wanted[MINE];
+#pragma unroll
+            for (int k = 0; k < MINE; ++k) {
+                const int i = threadIdx.x + k * THREADS;
+                group[k] = -1;
+                wanted[k] = 0;
+                if (i < pieces->count) {
+                    const int tile = pieces->tile[i];
+                    const bool two = tile + 1 < p.token_tiles && pieces->group[tile + 1] == pieces->group[tile] && pieces->wanted[tile + 1] > 0;
+                    group[k] = pieces->group[tile];
+                    wanted[k] = (unsigned char)((two ? GROUP_TILE + pieces->wanted[tile + 1] + 15 : pieces->wanted[tile] + 15) / 16);
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < MINE; ++k) {
+                const int i = threadIdx.x + k * THREADS;
+                if (i < pieces->count) {
+                    pieces->group[i] = group[k];
+                    pieces->wanted[i] = wanted[k];
+                }
+            }
+            __syncthreads();
+        }
+    }
+    const int token_tiles = grouped ? pieces->count : p.token_tiles;
+    const long long whole_tiles = grouped ? (long long)token_tiles * feature_tiles : p.tail_first;
+    const int rounds = grouped ? (int)((whole_tiles + gridDim.x - 1) / gridDim.x) : p.rounds;
     auto locate = [&](long long tile, int& token_tile, int& feature_tile) {
         const long long column = tile / (8LL * feature_tiles), within = tile - column * 8 * feature_tiles;
-        const int wide = min(8, p.token_tiles - (int)column * 8);
+        const int wide = min(8, token_tiles - (int)column * 8);
         token_tile = (int)column * 8 + (int)(within % wide);
         feature_tile = (int)(within / wide);
     };
-
-    // Weights in groups (the experts of a routed feed-forward): the first weight row of a tile's group, -1: no such tile.
-    auto group_begin = [&](long long tile) -> int {
-        if (!p.group_of_tile) return 0;
-        int token_tile, feature_tile;
-        locate(tile, token_tile, feature_tile);
-        const int group = p.group_of_tile[token_tile];
-        return group < 0 ? -1 : group * p.group_rows;
-    };
+    // A tile's first token, its tokens (in steps of 16) and, with weights in groups (the experts of a routed feed-forward), its
+    // group's first weight row.
+    auto first_token = [&](int token_tile) { return grouped ? pieces->tile[token_tile] * GROUP_TILE : token_tile * BN; };
+    auto columns_of = [&](int token_tile) { return grouped ? pieces->wanted[token_tile] * 16 : BN; };
+    auto group_begin = [&](int token_tile) { return grouped ? pieces->group[token_tile] * p.group_rows : 0; };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -281,9 +354,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         auto load = [&](long long tile, int kb_first, int kb_count) {
             int token_tile, feature_tile;
             locate(tile, token_tile, feature_tile);
-            const int begin = group_begin(tile);
-            if (begin < 0) return;
-            const int f0 = begin + feature_tile * SPAN, t0 = token_tile * BN;
+            const int f0 = group_begin(token_tile) + feature_tile * SPAN, t0 = first_token(token_tile);
+            const int boxes = grouped ? (columns_of(token_tile) + GROUP_BOX - 1) / GROUP_BOX : 0;
             for (int i = 0; i < kb_count; ++i, ++issued) {
                 const int s = issued % STAGES;
                 if (issued >= STAGES && !mbarrier_wait(&empty_bar[s], ((issued / STAGES) - 1) & 1, abort_flag)) {
@@ -291,7 +363,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     return;
                 }
                 unsigned char* stage = tiles + (size_t)s * STAGE_BYTES;
-                mbarrier_expect_tx(&full_bar[s], STAGE_BYTES);
+                mbarrier_expect_tx(&full_bar[s], boxes ? A_BYTES + boxes * GROUP_BOX * BK * 2 : STAGE_BYTES);
                 const int k = (kb_first + i) * BK;
                 if (GATED) {
                     tma_load_2d(stage, &map_w, &full_bar[s], k, f0);                            // 64 gate rows
@@ -299,11 +371,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 } else {
                     tma_load_2d(stage, &map_w, &full_bar[s], k, f0);
                 }
-                tma_load_2d(stage + A_BYTES, &map_x, &full_bar[s], k, t0);
+                if (boxes)
+                    for (int box = 0; box < boxes; ++box)
+                        tma_load_2d(stage + A_BYTES + box * GROUP_BOX * BK * 2, &map_x, &full_bar[s], k, t0 + box * GROUP_BOX);
+                else
+                    tma_load_2d(stage + A_BYTES, &map_x, &full_bar[s], k, t0);
             }
         };
-        for (int round = 0; round < p.rounds && !*abort_flag; ++round)
-            if (blockIdx.x + (long long)round * gridDim.x < p.tail_first)
+        for (int round = 0; round < rounds && !*abort_flag; ++round)
+            if (blockIdx.x + (long long)round * gridDim.x < whole_tiles)
                 load(blockIdx.x + (long long)round * gridDim.x, 0, p.k_blocks);
         for (long long g = piece_begin; g < piece_end && !*abort_flag;) {
             const long long tile = g / p.k_blocks;
@@ -319,9 +395,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         }
     } else if (warp == 1 && lane == 0) {
         // -------------------------------------------------------------- issuer
-        constexpr unsigned idesc = make_instr_desc(BN);
         int consumed = 0, done = 0;                        // stages read, accumulators finished
-        auto multiply = [&](int kb_count) {
+        auto multiply = [&](int kb_count, int columns) {
+            const unsigned idesc = make_instr_desc(columns);
             const int buffer = done & 1;
             // The accumulator's last reader (two pieces of work ago) must have read it out.
             if (done >= 2 && !mbarrier_wait(&drained_bar[buffer], ((done >> 1) - 1) & 1, abort_flag)) {
@@ -347,14 +423,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             umma_commit(&ready_bar[buffer]);  // arrives when the accumulator is complete
             ++done;
         };
-        for (int round = 0; round < p.rounds && !*abort_flag; ++round)
-            if (blockIdx.x + (long long)round * gridDim.x < p.tail_first &&
-                group_begin(blockIdx.x + (long long)round * gridDim.x) >= 0)
-                multiply(p.k_blocks);
+        for (int round = 0; round < rounds && !*abort_flag; ++round) {
+            const long long tile = blockIdx.x + (long long)round * gridDim.x;
+            if (tile >= whole_tiles) break;
+            int token_tile, feature_tile;
+            locate(tile, token_tile, feature_tile);
+            multiply(p.k_blocks, columns_of(token_tile));
+        }
         for (long long g = piece_begin; g < piece_end && !*abort_flag;) {
             const int kb_first = (int)(g % p.k_blocks);
             const int kb_count = (int)min((long long)(p.k_blocks - kb_first), piece_end - g);
-            multiply(kb_count);
+            multiply(kb_count, BN);
             g += kb_count;
         }
     } else if (warp >= 2) {
@@ -370,7 +449,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         auto finish = [&](long long tile, long long tail_tile, int kb_first, int kb_count) {
             int token_tile, feature_tile;
             locate(tile, token_tile, feature_tile);
-            const int f0 = feature_tile * SPAN, t0 = token_tile * BN;
+            const int f0 = feature_tile * SPAN, t0 = first_token(token_tile), columns = columns_of(token_tile);
             const int buffer = done & 1;
             const unsigned accumulator = tmem_base + buffer * BUFFER_COLUMNS + ((unsigned)(quarter * 32) << 16);
             bool ok = !*abort_flag && mbarrier_wait(&ready_bar[buffer], (done >> 1) & 1, abort_flag);
@@ -412,7 +491,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             {
                 TY* y = (TY*)p.y;
 #pragma unroll 1
-                for (int c = 0; c < BN; c += CW) {
+                for (int c = 0; c < columns; c += CW) {
                     float v[CW];
                     if (ok) tmem_load<CW>(accumulator + c, v);
                     else
@@ -453,7 +532,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                         asm volatile("bar.sync 1, 128;" ::: "memory");
                         if (threadIdx.x == 64) {
                             tma_store_2d(&map_y, out, f0, t0 + c);
-                            if (CW > 16) tma_store_2d(&map_y, out + 16 * SPAN, f0, t0 + c + 16);
+                            if (CW > 16 && c + 16 < columns) tma_store_2d(&map_y, out + 16 * SPAN, f0, t0 + c + 16);
                             tma_store_commit();
                         }
                         ++staged_chunks;
@@ -546,9 +625,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 p.counters[gridDim.x + first_block] = 0;
             }
         };
-        for (int round = 0; round < p.rounds; ++round)
-            if (blockIdx.x + (long long)round * gridDim.x < p.tail_first &&
-                group_begin(blockIdx.x + (long long)round * gridDim.x) >= 0)
+        for (int round = 0; round < rounds; ++round)
+            if (blockIdx.x + (long long)round * gridDim.x < whole_tiles)
                 finish(blockIdx.x + (long long)round * gridDim.x, -1, 0, p.k_blocks);
         for (long long g = piece_begin; g < piece_end;) {
             const long long tail_tile = g / p.k_blocks;
@@ -624,13 +702,10 @@ int make_store_map(CUtensorMap* map, void* base, long long tokens, long long fea
     return status == CUDA_SUCCESS ? 0 : 1000 + (int)status;
 }
 
-// Shared memory of a block: the stages, a kilobyte to align them, the gated epilogue's exchange
-// buffer and two buffers of results on their way out.
-template <int BN, int STAGES>
+// The same with a kilobyte to align the stages.
+template <int BN, int STAGES, typename TY>
 constexpr size_t shared_bytes() {
-    constexpr int columns = epilogue_columns<BN>();
-    return (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 1024 + 64 * (columns + 1) * sizeof(float) +
-           2 * columns * BM * sizeof(bf16);
+    return shared_floor<BN, STAGES>() + 1024 + (BN == 256 && sizeof(TY) == 2 ? sizeof(GroupPieces) : 0);
 }
 
 // Sets the kernel up (once) and returns how many of its blocks the device promises to hold on an SM
@@ -640,7 +715,7 @@ constexpr size_t shared_bytes() {
 // wait for each other make use of.
 template <int BN, int STAGES, bool GATED, typename TY>
 int blocks_per_sm() {
-    constexpr size_t shared = shared_bytes<BN, STAGES>();
+    constexpr size_t shared = shared_bytes<BN, STAGES, TY>();
     static_assert(shared <= (BN <= 64 ? 113 : 227) * 1024, "the stages fit an SM's shared memory (twice for small tiles)");
     static std::atomic<int> known_by_device[64];         // 0: not asked yet; else the answer + 1
     int device = 0;
@@ -666,7 +741,7 @@ int blocks_per_sm() {
 template <int BN, int STAGES, bool GATED, typename TY>
 int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const CUtensorMap& map_y, const Params& p, int blocks,
            cudaStream_t stream) {
-    constexpr size_t shared = shared_bytes<BN, STAGES>();
+    constexpr size_t shared = shared_bytes<BN, STAGES, TY>();
     auto kernel = gemm_tcgen05_kernel<BN, STAGES, GATED, TY>;
     const int per_sm = blocks_per_sm<BN, STAGES, GATED, TY>();
     if (per_sm <= 0) return KIDI_REFUSED_SIZE;
@@ -791,7 +866,7 @@ KIDI_API int kidi_gemm_tcgen05(const void* x, const void* w, void* y, int y_dtyp
     p.features = features;
     p.k_blocks = (K + BK - 1) / BK;
     p.token_tiles = (tokens + bn - 1) / bn;
-    p.group_of_tile = nullptr;
+    p.group_of_tile = p.used_of_tile = nullptr;
     p.group_rows = 0;
     p.gate = GateShape{};
     const long long tiles = (long long)((features + span - 1) / span) * p.token_tiles;
@@ -832,42 +907,51 @@ KIDI_API int kidi_gemm_tcgen05(const void* x, const void* w, void* y, int y_dtyp
 
 // The same for weights in groups (the experts of a routed feed-forward) and rows that are sorted by group: x [tokens, K] in
 // tiles of 128 rows, tile i's rows taking group group_of_tile[i] of w [groups, features (2 * features when gated), K]
-// (negative: the tile holds nothing; its rows of y are not written). Whole tiles only; no bias. `gate`: the gated form's
-// activation (null: SiLU).
+// (negative: the tile holds nothing; its rows of y are not written). `used` (or null): only the first used[i] rows of tile i
+// are wanted; a group's tiles follow one another, and all but its last are full. Whole tiles only; no bias. `gate`: the gated
+// form's activation (null: SiLU).
 KIDI_API int kidi_gemm_tcgen05_grouped(const void* x, const void* w, void* y, int tokens, int features, int K, long long ldx,
-                                       long long ldy, int gated, int groups, const int* group_of_tile, int* error,
+                                       long long ldy, int gated, int groups, const int* group_of_tile, const int* used, int* error,
                                        const GateShape* gate, cudaStream_t stream) {
-    constexpr int BN = 128;
+    constexpr int BN = 256;
     if (tokens <= 0 || features <= 0) return 0;
     const long long rows = (long long)groups * features * (gated ? 2 : 1);
     if (K <= 0 || (K & 7) || (ldx & 7) || (ldy & 7) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)y & 15) ||
-        groups <= 0 || rows > 0x7fffffffLL || tokens % BN || !group_of_tile || !error)
+        groups <= 0 || groups > 32767 || rows > 0x7fffffffLL || tokens % GROUP_TILE || !group_of_tile || !error)
         return KIDI_REFUSED_SIZE;
     const int span = gated ? 64 : BM;
-    Params p;
-    memset(&p, 0, sizeof(p));
-    p.y = y;
-    p.error = error;
-    p.ldy = ldy;
-    p.tokens = tokens;
-    p.features = features;
-    p.k_blocks = (K + BK - 1) / BK;
-    p.token_tiles = tokens / BN;
-    p.tiles = (long long)((features + span - 1) / span) * p.token_tiles;
-    p.group_of_tile = group_of_tile;
-    p.group_rows = features * (gated ? 2 : 1);
-    p.staged = 1;
-    if (gate) p.gate = *gate;
-    const long long sms = sm_count_of_current_device();
-    const int blocks = (int)(p.tiles < sms ? p.tiles : sms);
-    if (p.tiles / blocks > 0x7fffffffLL) return KIDI_REFUSED_SIZE;
-    p.rounds = (int)((p.tiles + blocks - 1) / blocks);
-    p.tail_first = p.tiles;
-    CUtensorMap map_w, map_x, map_y;
-    int status = make_map(&map_w, w, rows, K, K, gated ? 64 : BM);
-    if (!status) status = make_map(&map_x, x, tokens, K, ldx, BN);
-    if (!status) status = make_store_map(&map_y, y, tokens, features, ldy, span);
-    if (status) return status;
-    if (gated) return by_tokens<true, bf16>(BN, map_w, map_x, map_y, p, blocks, stream);
-    return by_tokens<false, bf16>(BN, map_w, map_x, map_y, p, blocks, stream);
+    const int feature_tiles = (features + span - 1) / span;
+    // A launch knows 1,024 tiles; more go in several (tiles of one group that fall into two launches are not paired).
+    for (int first = 0; first < tokens / GROUP_TILE; first += MOST_GROUP_TILES) {
+        const int count = tokens / GROUP_TILE - first < MOST_GROUP_TILES ? tokens / GROUP_TILE - first : MOST_GROUP_TILES;
+        const bf16* from = (const bf16*)x + (long long)first * GROUP_TILE * ldx;
+        bf16* to = (bf16*)y + (long long)first * GROUP_TILE * ldy;
+        Params p;
+        memset(&p, 0, sizeof(p));
+        p.y = to;
+        p.error = error;
+        p.ldy = ldy;
+        p.tokens = count * GROUP_TILE;
+        p.features = features;
+        p.k_blocks = (K + BK - 1) / BK;
+        p.token_tiles = count;
+        p.tiles = (long long)feature_tiles * count;
+        p.group_of_tile = group_of_tile + first;
+        p.used_of_tile = used ? used + first : nullptr;
+        p.group_rows = features * (gated ? 2 : 1);
+        p.staged = 1;
+        if (gate) p.gate = *gate;
+        const long long sms = sm_count_of_current_device();
+        const int blocks = (int)(p.tiles < sms ? p.tiles : sms);
+        p.rounds = 1;                    // (the kernel counts its rounds itself: it knows how many pieces of work there are)
+        p.tail_first = p.tiles;
+        CUtensorMap map_w, map_x, map_y;
+        int status = make_map(&map_w, w, rows, K, K, gated ? 64 : BM);
+        if (!status) status = make_map(&map_x, from, p.tokens, K, ldx, GROUP_BOX);
+        if (!status) status = make_store_map(&map_y, to, p.tokens, features, ldy, span);
+        if (!status) status = gated ? by_tokens<true, bf16>(BN, map_w, map_x, map_y, p, blocks, stream)
+                                    : by_tokens<false, bf16>(BN, map_w, map_x, map_y, p, blocks, stream);
+        if (status) return status;
+    }
+    return 0;
 }

@@ -350,7 +350,7 @@ KIDI_API int kidi_expert_slots(const void* x, int dtype, const void* gate_up, co
 constexpr int GROUP_TILE = 128, GROUP_THREADS = 1024;
 __global__ void __launch_bounds__(GROUP_THREADS) group_slots_kernel(const int* __restrict__ chosen, int* __restrict__ source,
                                                                     int* __restrict__ place, int* __restrict__ expert_of_tile,
-                                                                    int slots, int experts, int rows) {
+                                                                    int* __restrict__ used_of_tile, int slots, int experts, int rows) {
     __shared__ int count[1024], begin[1025], warp_total[32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     count[threadIdx.x] = 0;
@@ -375,7 +375,11 @@ __global__ void __launch_bounds__(GROUP_THREADS) group_slots_kernel(const int* _
     for (int row = threadIdx.x; row < rows; row += GROUP_THREADS) source[row] = -1;
     for (int tile = threadIdx.x + begin[GROUP_THREADS]; tile < rows / GROUP_TILE; tile += GROUP_THREADS) expert_of_tile[tile] = -1;
     for (int e = warp; e < experts; e += 32)
-        for (int tile = begin[e] + lane; tile < begin[e + 1]; tile += 32) expert_of_tile[tile] = e;
+        for (int tile = begin[e] + lane; tile < begin[e + 1]; tile += 32) {
+            expert_of_tile[tile] = e;
+            if (used_of_tile) used_of_tile[tile] = min(GROUP_TILE, count[e] - (tile - begin[e]) * GROUP_TILE);
+        }
+    __syncthreads();
     count[threadIdx.x] = begin[threadIdx.x] * GROUP_TILE;          // the next free row of an expert
     __syncthreads();
     for (int i = threadIdx.x; i < slots; i += GROUP_THREADS) {
@@ -391,13 +395,14 @@ KIDI_API int kidi_group_slots_rows(int slots, int experts) {
     return rows > 0x7fffffffLL ? -1 : (int)rows;
 }
 
-KIDI_API int kidi_group_slots(const int* chosen, int* source, int* place, int* expert_of_tile, int slots, int experts,
-                              cudaStream_t stream) {
+// `used_of_tile` (or null): the rows of a used tile that hold slots.
+KIDI_API int kidi_group_slots(const int* chosen, int* source, int* place, int* expert_of_tile, int* used_of_tile, int slots,
+                              int experts, cudaStream_t stream) {
     const int rows = kidi_group_slots_rows(slots, experts);
     if (slots <= 0) return 0;
     if (experts <= 0 || experts > 1024 || rows < 0) return KIDI_REFUSED_SIZE;
-    return kidi_launch(group_slots_kernel, 1, GROUP_THREADS, 0, stream, chosen, source, place, expert_of_tile, slots, experts,
-                       rows);
+    return kidi_launch(group_slots_kernel, 1, GROUP_THREADS, 0, stream, chosen, source, place, expert_of_tile, used_of_tile, slots,
+                       experts, rows);
 }
 
 // ------------------------------------------------------ gather / combine

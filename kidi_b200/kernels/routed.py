@@ -29,7 +29,7 @@ def library():
                                           c_void_p]
         lib.kidi_combine_slots.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                            c_void_p, c_void_p, c_void_p]
-        lib.kidi_group_slots.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]
+        lib.kidi_group_slots.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]
         lib.kidi_group_slots_rows.argtypes = [c_int, c_int]
         for name in ("kidi_group_slots", "kidi_group_slots_rows", "kidi_route", "kidi_expert_slots", "kidi_gather_slots", "kidi_combine_slots"):
             getattr(lib, name).restype = c_int
@@ -130,6 +130,11 @@ def group_slots(chosen: torch.Tensor, experts: int):
     """Groups the (row, choice) pairs of `chosen` (int32, slot = row * top + choice) by expert on the device: (source,
     place, expert_of_tile), int32: the slot of every grouped row (-1: padding), the row of every slot, the expert of every
     tile of 128 rows (-1: not used). The order within an expert is not fixed."""
+    return group_slots_used(chosen, experts)[:3]
+
+
+def group_slots_used(chosen: torch.Tensor, experts: int):
+    """The same with a fourth table, int32: how many rows of every used tile hold slots (its first ones)."""
     ops._need_cuda(chosen)
     if chosen.dtype != torch.int32 or not chosen.is_contiguous():
         raise invalid_argument("group_slots takes the router's choices")
@@ -139,10 +144,10 @@ def group_slots(chosen: torch.Tensor, experts: int):
         raise invalid_argument("group_slots: too many slots")
     source = torch.empty(rows, dtype=torch.int32, device=chosen.device)
     place = torch.empty(slots, dtype=torch.int32, device=chosen.device)
-    tiles = torch.empty(rows // 128, dtype=torch.int32, device=chosen.device)
-    _check(library().kidi_group_slots(chosen.data_ptr(), source.data_ptr(), place.data_ptr(), tiles.data_ptr(), slots,
-                                      int(experts), ops._stream()), "group_slots")
-    return source, place, tiles
+    tiles, used = (torch.empty(rows // 128, dtype=torch.int32, device=chosen.device) for _ in range(2))
+    _check(library().kidi_group_slots(chosen.data_ptr(), source.data_ptr(), place.data_ptr(), tiles.data_ptr(), used.data_ptr(),
+                                      slots, int(experts), ops._stream()), "group_slots")
+    return source, place, tiles, used
 
 
 def gather_slots(x: torch.Tensor, order: torch.Tensor, weight: torch.Tensor, top: int, weight_on_input: bool) -> torch.Tensor:

@@ -55,7 +55,7 @@ def _library():
                                           c_void_p, c_void_p]
         lib.kidi_gemm_tcgen05.restype = c_int
         lib.kidi_gemm_tcgen05_grouped.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
-                                                  c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]
+                                                  c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
         lib.kidi_gemm_tcgen05_grouped.restype = c_int
         lib.kidi_gemm_tcgen05_token_tile.argtypes = [c_int]
         lib.kidi_gemm_tcgen05_token_tile.restype = c_int
@@ -149,23 +149,26 @@ GROUP_TILE = 128                        # rows of a tile of a grouped product
 
 
 def gemm_grouped(x: torch.Tensor, weight: torch.Tensor, group_of_tile: torch.Tensor, gated: bool,
-                 shape: Optional[ops.GateShape] = None) -> torch.Tensor:
+                 shape: Optional[ops.GateShape] = None, used: Optional[torch.Tensor] = None) -> torch.Tensor:
     """A product with weights in groups: rows 128 i .. 128 i + 127 of x [rows, K] take weight[group_of_tile[i]] of
     weight [groups, features, K] (`gated`: [groups, 2 * features, K], gate rows first, and the result is silu(gate) * up);
-    bfloat16. Rows of tiles whose group (int32) is negative are not written. `shape`: another activation than SiLU."""
-    _need_cuda(x, weight, group_of_tile)
+    bfloat16. Rows of tiles whose group (int32) is negative are not written. `shape`: another activation than SiLU. `used`
+    (int32, a number a tile): only a tile's first rows are wanted; a group's tiles follow one another, the last one alone may
+    lack rows, and what the others hold is not defined."""
+    _need_cuda(x, weight, group_of_tile, used)
     groups, height, K = weight.shape
     rows = x.shape[0]
     if (x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or x.dim() != 2 or x.shape[1] != K or x.stride(1) != 1
             or not weight.is_contiguous() or rows % GROUP_TILE or (gated and height % 2)
-            or group_of_tile.dtype != torch.int32 or group_of_tile.shape != (rows // GROUP_TILE,)):
+            or group_of_tile.dtype != torch.int32 or group_of_tile.shape != (rows // GROUP_TILE,)
+            or (used is not None and (used.dtype != torch.int32 or used.shape != group_of_tile.shape or not used.is_contiguous()))):
         raise invalid_argument("gemm_grouped: the operands do not fit this kernel")
     features = height // 2 if gated else height
     out = torch.empty((rows, features), dtype=torch.bfloat16, device=x.device)
     _, _, error = _device_state(x.device)
     _check(_library().kidi_gemm_tcgen05_grouped(
         _ptr(x), _ptr(weight), _ptr(out), rows, features, K, x.stride(0), out.stride(0), 1 if gated else 0, groups,
-        _ptr(group_of_tile), _ptr(error), ctypes.byref(shape) if shape is not None else None, _stream()),
+        _ptr(group_of_tile), _ptr(used), _ptr(error), ctypes.byref(shape) if shape is not None else None, _stream()),
         "gemm_bounded_gate[tcgen05, groups]" if gated and shape is not None and shape.bounded
         else "gemm_silu_gate[tcgen05, groups]" if gated else "gemm_tcgen05[groups]")
     return out

@@ -210,12 +210,12 @@ class RoutedExperts(Part):
                                        shape=self.shape, share=share)
         if GROUPED and self.hidden % 8 == 0 and self.inter % 8 == 0 \
                 and 0 < routed.group_rows(slots, self.experts) <= 4 * slots:
-            source, place, tiles = routed.group_slots(chosen, self.experts)
+            source, place, tiles, used = routed.group_slots_used(chosen, self.experts)
             gathered = routed.gather_slots(x, source, weight, self.top, self.weight_on_input)
-            mid = tcgen05.gemm_grouped(gathered, self.gate_up, tiles, self.gated, shape=self.shape)
+            mid = tcgen05.gemm_grouped(gathered, self.gate_up, tiles, self.gated, shape=self.shape, used=used)
             if not self.gated:
                 mid = self._activate(mid)
-            result = tcgen05.gemm_grouped(mid, self.down, tiles, False)
+            result = tcgen05.gemm_grouped(mid, self.down, tiles, False, used=used)
             return routed.combine_slots(result, place, weight, rows, self.top, self.weight_on_input, shared(), share)
         # Many rows: (row, choice) pairs in the order of their experts (a stable sort, so a row's place among
         # its expert's rows follows its place in the step), one host round trip for the counts.

@@ -828,6 +828,32 @@ def test_products_over_groups_of_experts(rows, experts, top, hidden, inter, gate
         assert torch.allclose(got[128 * tile:128 * tile + 128], want, atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("counts,hidden,inter", [((1, 16, 17, 127, 128, 129, 0, 255, 256, 257, 400, 513), 136, 72), ((300, 0, 40), 64, 136),
+                                                 ((131000, 129, 1), 64, 64)])
+def test_products_over_groups_take_two_tiles_of_a_group_at_once(counts, hidden, inter, gated):
+    """Runs of one tile, of pairs and of pairs with one tile more, last tiles of any height, more tiles than a launch knows:
+    every wanted row against the product with its group's weights."""
+    from kidi_b200.kernels import routed, tcgen05
+    generator = torch.Generator().manual_seed(hidden)
+    chosen = torch.cat([torch.full((count,), expert) for expert, count in enumerate(counts)])
+    chosen = chosen[torch.randperm(chosen.numel(), generator=generator)].int()
+    source, place, tiles, used = routed.group_slots_used(chosen.view(-1, 1).cuda(), len(counts))
+    live = tiles >= 0
+    assert torch.equal(used[live].cpu(), torch.cat([torch.tensor([128] * (n // 128) + [n % 128] * (n % 128 > 0)) for n in counts]).int())
+    x = torch.randn(source.numel(), hidden, generator=generator).bfloat16().cuda()
+    weight = (torch.randn(len(counts), (2 if gated else 1) * inter, hidden, generator=generator) / hidden ** 0.5).bfloat16().cuda()
+    for wanted in (used, None):
+        got = tcgen05.gemm_grouped(x, weight, tiles, gated, used=wanted)
+        for expert in range(len(counts)):
+            rows = place[(chosen == expert).cuda()].long() if wanted is not None else \
+                (torch.where(tiles == expert)[0][:, None] * 128 + torch.arange(128, device="cuda")).reshape(-1)
+            y = x[rows].double() @ weight[expert].double().t()
+            want = plain_dibesun.silu(y[:, :inter]) * y[:, inter:] if gated else y
+            assert torch.allclose(got[rows].double(), want, atol=2e-2, rtol=2e-2)
+    assert tcgen05.error_code(torch.device("cuda:0")) == 0
+
+
 def test_routed_prompts_grouped_on_the_device_and_sorted_on_the_host(monkeypatch, record_property):
     """The same prompt through both forms of the routed feed-forward: each names its kernels, the logits agree within
     bfloat16 rounding, and a request in a batch is what it is alone."""
