@@ -27,72 +27,97 @@
 #include "common.cuh"
 
 // ---------------------------------------------------------------- choose
-// One row of weights against ROWS rows of x (the first `here` of them; `hidden` apart), a warp's share; the caller sums over
-// the warp. A row's sum runs in the same order whatever ROWS is.
-template <int ROWS, typename T, typename TW>
-__device__ __forceinline__ void dots(const TW* __restrict__ w, const T* __restrict__ x, int K, int lane, int here, float (&a)[ROWS]) {
+// COLS rows of weights (those at `w`, `apart` elements apart, the first `wide` of them) against ROWS rows of x (the first
+// `here` of them; `hidden` apart), a warp's share; the caller sums over the warp. A pair's sum runs in the same order
+// whatever ROWS and COLS are.
+template <int ROWS, int COLS, typename T, typename TW>
+__device__ __forceinline__ void dots(const TW* __restrict__ w, long long apart, int wide, const T* __restrict__ x, int K,
+                                     int lane, int here, float (&a)[COLS][ROWS]) {
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) a[r] = 0.f;
+    for (int c = 0; c < COLS; ++c)
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) a[c][r] = 0.f;
     if constexpr (sizeof(T) == 2 && sizeof(TW) == 2) {
         if (!(K & 7) && !((uintptr_t)w & 15) && !((uintptr_t)x & 15)) {
+#pragma unroll (ROWS > 1 ? 2 : 4)
             for (int k = lane * 8; k < K; k += 256) {
-                const uint4 rw = *reinterpret_cast<const uint4*>(w + k);
-                const __nv_bfloat162* pw = reinterpret_cast<const __nv_bfloat162*>(&rw);
-                float2 fw[4];
+                uint4 rw[COLS], rx[ROWS];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) fw[i] = __bfloat1622float2(pw[i]);
+                for (int c = 0; c < COLS; ++c) rw[c] = *reinterpret_cast<const uint4*>(w + min(c, wide - 1) * apart + k);
 #pragma unroll
-                for (int r = 0; r < ROWS; ++r) {
-                    const uint4 rx = *reinterpret_cast<const uint4*>(x + (long long)min(r, here - 1) * K + k);
-                    const __nv_bfloat162* px = reinterpret_cast<const __nv_bfloat162*>(&rx);
+                for (int r = 0; r < ROWS; ++r)
+                    rx[r] = *reinterpret_cast<const uint4*>(x + (long long)min(r, here - 1) * K + k);
+                float2 fw[COLS][4];
+#pragma unroll
+                for (int c = 0; c < COLS; ++c)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) fw[c][i] = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&rw[c])[i]);
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r)
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        const float2 fx = __bfloat1622float2(px[i]);
-                        a[r] = fmaf(fw[i].x, fx.x, a[r]);
-                        a[r] = fmaf(fw[i].y, fx.y, a[r]);
+                        const float2 fx = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&rx[r])[i]);
+#pragma unroll
+                        for (int c = 0; c < COLS; ++c) {
+                            a[c][r] = fmaf(fw[c][i].x, fx.x, a[c][r]);
+                            a[c][r] = fmaf(fw[c][i].y, fx.y, a[c][r]);
+                        }
                     }
-                }
             }
             return;
         }
     }
     for (int k = lane; k < K; k += 32) {
-        const float value = to_float(w[k]);
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) a[r] = fmaf(value, to_float(x[(long long)min(r, here - 1) * K + k]), a[r]);
+        for (int c = 0; c < COLS; ++c) {
+            const float value = to_float(w[min(c, wide - 1) * apart + k]);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) a[c][r] = fmaf(value, to_float(x[(long long)min(r, here - 1) * K + k]), a[c][r]);
+        }
     }
 }
 
-// A block ROWS rows: its sixteen warps share the experts (a warp a router row at a time, 32-bit sums in an order
+// A block ROWS rows: its 16 / COLS warps share the experts (a warp COLS router rows at a time, 32-bit sums in an order
 // that depends on the width only), then a warp a row takes the `top` largest scores, one after the other.
-template <int ROWS, typename T, typename TW>
-__global__ void __launch_bounds__(544) route_kernel(const T* __restrict__ x, const TW* __restrict__ router,
-                                                    int* __restrict__ chosen, float* __restrict__ weight, int hidden,
-                                                    int experts, int top, int renormalise, int softmax, int groups,
-                                                    int keep, float renormalise_eps, const float* __restrict__ bias,
-                                                    const float* __restrict__ correction, int two_largest, float weight_scale,
-                                                    const TW* __restrict__ share_row, float* __restrict__ share, int rows) {
+// Bound by its instructions and by the wait for each step's reads. On prompts (ROWS = 4) half of the instructions turn x
+// into 32 bits, so a warp takes two experts for them, and two steps' reads are in flight; eight warps a block let all
+// blocks of a prompt's 1,500 rows run at once. 1,500 rows of 2,048 and 16 experts (an empty launch: 6 us): 17 us, 23.5 with
+// an expert a warp and one step in flight; 64 experts: 37, 60.
+template <int ROWS, int COLS, typename T, typename TW>
+__global__ void __launch_bounds__((16 / COLS + 1) * 32, COLS > 1 ? 3 : 2) route_kernel(
+    const T* __restrict__ x, const TW* __restrict__ router, int* __restrict__ chosen, float* __restrict__ weight, int hidden,
+    int experts, int top, int renormalise, int softmax, int groups, int keep, float renormalise_eps,
+    const float* __restrict__ bias, const float* __restrict__ correction, int two_largest, float weight_scale,
+    const TW* __restrict__ share_row, float* __restrict__ share, int rows) {
+    constexpr int WARPS = 16 / COLS;
+    static_assert(ROWS <= WARPS, "a warp a row chooses");
     extern __shared__ float scores[];      // for each row: [experts] scores, then [experts] what may still be chosen
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row0 = blockIdx.x * ROWS, here = min(ROWS, rows - row0);
     const T* block_rows = x + (long long)row0 * hidden;
-    float dot[ROWS];
-    if (warp == 16) {                      // (launched where it is asked for) the gate of the expert that every row passes
-        dots<ROWS, T, TW>(share_row, block_rows, hidden, lane, here, dot);
+    if (warp == WARPS) {                   // (launched where it is asked for) the gate of the expert that every row passes
+        float dot[1][ROWS];
+        dots<ROWS, 1, T, TW>(share_row, 0, 1, block_rows, hidden, lane, here, dot);
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
-            const float z = warp_sum(dot[r]);
+            const float z = warp_sum(dot[0][r]);
             if (lane == 0 && r < here) share[row0 + r] = 1.0f / (1.0f + expf(-z));
         }
     }
-    for (int e = warp; warp < 16 && e < experts; e += 16) {
-        dots<ROWS, T, TW>(router + (long long)e * hidden, block_rows, hidden, lane, here, dot);
+    for (int e = warp * COLS; warp < WARPS && e < experts; e += 16) {
+        float dot[COLS][ROWS];
+        const int wide = min(COLS, experts - e);
+        dots<ROWS, COLS, T, TW>(router + (long long)e * hidden, hidden, wide, block_rows, hidden, lane, here, dot);
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            float z = warp_sum(dot[r]);
-            if (bias) z += bias[e];
-            if (lane == 0) scores[2 * experts * r + e] = softmax ? z : 1.0f / (1.0f + expf(-z));
-        }
+        for (int c = 0; c < COLS; ++c)
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                float z = warp_sum(dot[c][r]);
+                if (c < wide && lane == 0) {
+                    if (bias) z += bias[e + c];
+                    scores[2 * experts * r + e + c] = softmax ? z : 1.0f / (1.0f + expf(-z));
+                }
+            }
     }
     __syncthreads();
     if (warp >= here) return;
@@ -193,12 +218,15 @@ KIDI_API int kidi_route(const void* x, int dtype, const void* router, int weight
         (long long)keep * (experts / groups) < top)
         return KIDI_REFUSED_SIZE;
     const size_t shared = (size_t)experts * 2 * sizeof(float);
-    constexpr int ROWS = 4;                  // rows of a block where there are enough of them (experts <= 1,024: 32 KB)
-    const bool many = rows >= 512;
+    constexpr int ROWS = 4, COLS = 2;        // rows of a block where there are enough of them (experts <= 1,024: 32 KB)
+    // Up to 296 rows the blocks of a row each all run at once (two an SM): 10 us at 256 rows of 2,048 and 16 experts against
+    // 12 for four rows a block; at 384 rows 15 against 12.
+    const bool many = rows > 296;
 #define KIDI_CASE(D, T, W, TW)                                                                                        \
     if (dtype == D && weight_dtype == W)                                                                              \
-        return kidi_launch(many ? route_kernel<ROWS, T, TW> : route_kernel<1, T, TW>,                                 \
-                           (unsigned)(many ? (rows + ROWS - 1) / ROWS : rows), share ? 544 : 512,                     \
+        return kidi_launch(many ? route_kernel<ROWS, COLS, T, TW> : route_kernel<1, 1, T, TW>,                        \
+                           (unsigned)(many ? (rows + ROWS - 1) / ROWS : rows),                                        \
+                           (many ? 512 / COLS : 512) + (share ? 32 : 0),                                              \
                            many ? ROWS * shared : shared, stream, (const T*)x, (const TW*)router, chosen, weight,     \
                            hidden, experts, top, renormalise, softmax, groups, keep, renormalise_eps, bias,           \
                            correction, two_largest, weight_scale, (const TW*)share_row, share, rows);

@@ -375,6 +375,35 @@ def test_the_router_with_a_bias(dtype):
             assert torch.allclose(weight.double().cpu(), torch.softmax(best.values, -1), atol=1e-5)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("experts,hidden,rows,shared", [(16, 2048, 513, False), (17, 264, 515, True), (1, 1000, 297, True),
+                                                        (33, 77, 514, False)])
+def test_the_router_on_a_prompt_is_that_of_single_rows(dtype, experts, hidden, rows, shared):
+    """Several rows and two experts a warp choose and weigh, bit by bit, as a row at a time does. A logit is off by at most
+    (hidden / 32 + 5) roundings of the sum of its products' sizes, 0.64 sqrt(hidden) here, and a weight by twice that:
+    below hidden * 8 * 2^-24."""
+    from kidi_b200.kernels import routed
+    generator = torch.Generator().manual_seed(experts + hidden)
+    x = torch.randn(rows, hidden, generator=generator).to(dtype)
+    router = (torch.randn(experts, hidden, generator=generator) * hidden ** -0.5).to(dtype)
+    row = torch.randn(1, hidden, generator=generator).to(dtype).cuda()
+    top = min(experts, 3)
+
+    def make(part):
+        share = torch.zeros(len(part), device="cuda")
+        extra = {"share_row": row, "share": share} if shared else {}
+        return *routed.route(part.cuda(), router.cuda(), top, False, "softmax", **extra), share
+
+    whole = make(x)
+    for first in range(0, rows, 100):
+        for all_rows, some in zip(whole, make(x[first:first + 100])):
+            assert torch.equal(all_rows[first:first + 100], some)
+    scores = torch.softmax(x.double() @ router.double().t(), -1)
+    want = scores.gather(1, whole[0].cpu().long())
+    assert torch.allclose(whole[1].cpu().double(), want, rtol=hidden * 2.0 ** -24 * 8, atol=0)
+    assert torch.allclose(want, scores.topk(top).values, rtol=1e-4)
+
+
 # ------------------------------------------------------------------ one layer
 ONE = configs.layer(configs.attention(4, 2, 16, 24, 0.4, chunk=70, softcap=3.0), configs.linear(3, 12, 20, (0.6, 0.95, 0.999)),
                     configs.routed(6, 2, 24, shared=16), left_scale=1.1, right_scale=0.6)
