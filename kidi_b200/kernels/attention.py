@@ -1,7 +1,8 @@
 """Chooses and launches the attention kernel for a step.
 
 The generic kernel takes every element type, head width up to 256 and any number of
-heads, for prompts and for single tokens; it is the only one the 32-bit engine uses.
+heads, for prompts and for single tokens. The 32-bit engine uses kernels of its own for
+heads of up to 128 in 16-byte pieces (csrc/attention_f32.cu) and the generic one otherwise.
 The bfloat16 engine uses the tensor-core kernels, which are compiled for the head
 width of the loaded model at the first call: a prefill kernel for steps that bring
 several tokens per sequence and a split-key decode kernel for steps of one token per

@@ -6,8 +6,8 @@ registered part. The bias is kept in 32-bit and added in the epilogue of this pa
 product kernels (after the vendor library's product, by a kernel of its own). Which
 kernel runs follows the element types:
 
-* a 32-bit input or a 32-bit weight: the 32-bit CUDA-core product (ascending-k fused
-  multiply-adds; no reduced-precision matrix mode);
+* a 32-bit input or a 32-bit weight: the 32-bit CUDA-core products (fused multiply-adds in
+  an order that depends on the width only; no reduced-precision matrix mode);
 * bfloat16 by bfloat16 with up to 8 rows (decode): the weight-streaming `mma.sync`
   kernel of this package (`kernels/skinny.py`);
 * bfloat16 by bfloat16 with 9 to 16 rows and a large weight (16384 output features or
