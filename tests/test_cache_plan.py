@@ -46,6 +46,23 @@ def test_groups_have_storage_of_their_own():
     assert cache.bytes() == 2 * full.keys.numel() * 4 + 2 * ring.keys.numel() * 4
 
 
+@pytest.mark.parametrize("grown", [[0], [0, 1, 2, 3], [1, 2, 4], [0, 2, 4, 5], [5]])
+def test_changed_rows_of_the_tables_reach_the_device(grown):
+    """Every changed row is copied, whichever rows lie beside each other, and no other row."""
+    cache = make_cache(max_tokens=2048)
+    slots = sorted(cache.acquire() for _ in range(6))
+    cache.reserve([(slots[index], 70 + index) for index in grown])
+    before = [group.table_host.copy() for group in cache.kv_groups]
+    for group in cache.kv_groups:
+        group.table.fill_(-1)
+    cache.flush_tables()
+    for group, host in zip(cache.kv_groups, before):
+        assert not group._dirty and (group.table_host == host).all()
+        for row in range(group.table.shape[0]):
+            want = host[row].tolist() if row in {slots[index] for index in grown} else [-1] * host.shape[1]
+            assert group.table[row].tolist() == want
+
+
 def test_pages_follow_lengths_and_come_back():
     cache = make_cache(max_tokens=640)
     a, b = cache.acquire(), cache.acquire()
