@@ -46,11 +46,14 @@ class StepContext:
         self.plan, self.tables, self.cache, self.dtype, self.device = plan, tables, cache, dtype, device
         self._workspaces = workspaces if workspaces is not None else {}
         self._side_stream = None
+        self._branch = ""              # what scratch memory is called by in front of its name (see `beside`)
 
     def workspace(self, name: str, count: int, zero: bool = False) -> torch.Tensor:
         """Scratch memory of at least `count` 32-bit elements that kernels of one step may
         use one after another (it is kept between steps and grows on demand). With `zero`
-        it is filled with zeros when it is made; its users leave it zero."""
+        it is filled with zeros when it is made; its users leave it zero. Work that is queued
+        `beside` others has memory of its own under every name."""
+        name = self._branch + name
         held = self._workspaces.get(name)
         if held is None or held.numel() < count:
             make = torch.zeros if zero else torch.empty
@@ -61,11 +64,18 @@ class StepContext:
     def beside(self, work):
         """Queues `work()` beside whatever the caller queues before it calls the returned function, which waits for the
         work (on the device) and returns its result. In a captured step the two become branches of the graph that may run
-        at the same time; elsewhere `work()` is queued at once, in the caller's order. The work must not use scratch
-        memory (`workspace`) that the caller's own launches use meanwhile, and what it writes for the caller is allocated
-        before the call or returned."""
+        at the same time; elsewhere `work()` is queued at once, in the caller's order. Its scratch memory (`workspace`) is
+        not the caller's, in either case (so that the step that runs before a capture makes what the capture takes);
+        what it writes for the caller is allocated before the call or returned."""
+        def queue():
+            branch, self._branch = self._branch, "beside:"
+            try:
+                return work()
+            finally:
+                self._branch = branch
+
         if self.device.type != "cuda" or not torch.cuda.is_current_stream_capturing():
-            result = work()
+            result = queue()
             return lambda: result
         main = torch.cuda.current_stream(self.device)
         if self._side_stream is None:
@@ -73,7 +83,7 @@ class StepContext:
         side = self._side_stream
         side.wait_stream(main)
         with torch.cuda.stream(side):
-            result = work()
+            result = queue()
 
         def join():
             main.wait_stream(side)

@@ -163,6 +163,44 @@ def test_attention_part_prompt_then_tokens(dtype, window):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_two_attention_mixers_side_by_side_in_a_captured_step(dtype):
+    """Both mixers of a captured single-token step keep their segments' sums in scratch memory at the same time: every replay
+    gives the bits of the step that is not captured, in which one mixer runs behind the other."""
+    from kidi_b200.cache.sequence_cache import SequenceCache
+    from kidi_b200.parts.base import all_parameters, bind_all
+    from kidi_b200.parts.registry import build_part
+    from kidi_b200.parts.spec import PartSpec
+    child = {"hidden_size": 256, "num_heads": 4, "num_kv_heads": 1, "head_dim": 64}
+    part = build_part("mixer", PartSpec("parallel_mixers", {
+        "hidden_size": 256, "combine": "plain", "left": PartSpec("attention", child, "left."),
+        "right": PartSpec("attention", child, "right.")}), make_env(dtype, max_positions=4096))
+    generator = torch.Generator().manual_seed(5)
+    bind_all(part, {prefix + spec.name: (torch.randn(spec.shape, generator=generator) * 0.1).to(dtype).to(DEVICE)
+                    for prefix, spec in all_parameters(part)})
+    cache = SequenceCache([part.cache_requests()], max_tokens=8192, max_positions=4096, dtype=dtype, device=DEVICE)
+    slots = [cache.acquire() for _ in range(2)]
+    held = list(zip(slots, (3900, 1500)))
+    cache.reserve(held)
+    cache.commit(held)
+    views = cache.views(0)
+    for view in views:
+        view.keys.copy_(torch.randn(view.keys.shape, generator=generator).to(dtype))
+        view.values.copy_(torch.randn(view.values.shape, generator=generator).to(dtype))
+    ctx, _ = run_step(cache, slots, [[0], [0]], dtype)
+    x = torch.randn(2, 256, generator=generator).to(dtype).to(DEVICE)
+    expected = part.forward(x, ctx, views, True).clone()
+    assert any("beside" in name for name in ctx._workspaces) and any("beside" not in name for name in ctx._workspaces)
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream(device=DEVICE)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        captured = part.forward(x, ctx, views, True)
+    for _ in range(200):
+        graph.replay()
+        assert torch.equal(captured, expected)
+    assert bool(expected.isfinite().all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_part_with_biases(dtype):
     """The same mixer with a bias on the fused q/k/v projection (bound from q, k and v biases by
     the loader's concatenation rule) and on the output projection: prompts of 5 and 150 rows

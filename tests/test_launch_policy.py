@@ -117,3 +117,21 @@ def test_32_bit_attention_counts_the_segments_that_a_row_can_see():
     for rows, segments in ((1, 160), (8, 160), (64, 160), (512, 64), (8, 1)):
         shares = ops.attention_f32_shares(rows, 32, 8, segments, 128, 148)
         assert 1 <= shares <= segments and (shares == 1 or rows * 32 * segments * 130 <= 1 << 26)
+
+
+def test_work_beside_others_has_scratch_memory_of_its_own():
+    from kidi_b200.engine.engine import StepContext
+    ctx = StepContext(None, None, None, torch.float32, torch.device("cpu"))
+
+    def work():
+        inner = ctx.workspace("sums", 8)
+        nested = ctx.beside(lambda: ctx.workspace("counters", 4, zero=True))()
+        return inner, nested, ctx.workspace("sums", 8)
+
+    mine = ctx.workspace("sums", 8), ctx.workspace("counters", 4, zero=True)
+    inner, nested, again = ctx.beside(work)()
+    assert inner is again and inner is not mine[0] and nested is not mine[1]
+    assert ctx.workspace("sums", 8) is mine[0] and ctx.workspace("counters", 4, zero=True) is mine[1]
+    with pytest.raises(ZeroDivisionError):
+        ctx.beside(lambda: 1 / 0)
+    assert ctx.workspace("sums", 8) is mine[0]
