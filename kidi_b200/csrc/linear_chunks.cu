@@ -219,6 +219,43 @@ __device__ __forceinline__ float decayed(double x) {
     return exp2f((float)(x - whole)) * __int_as_float(((int)whole + 127) << 23);
 }
 
+// The key tile on the diagonal holds tokens that come after some of its rows. Their scores are zeros, and zero times an infinity
+// or a NaN is a NaN: where the tile's values hold one, it is taken out of the product and added, one by one, to the rows that
+// see it. `v`: 16 keys x 16 columns as ldmatrix left them, `tile`: the first of them in shared memory, `parts`: the scores of the
+// warp's 16 rows against the keys, `left` and `right`: what the products of 8 columns each are added to.
+__device__ __forceinline__ void leave_out_later_tokens(unsigned (&v)[4], const bf16* tile, const unsigned (&parts)[3][4],
+                                                       float (&left)[4], float (&right)[4]) {
+    unsigned found = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) found |= (v[i] & 0x7f80u) == 0x7f80u || (v[i] & 0x7f800000u) == 0x7f800000u;
+    if (!__any_sync(0xffffffffu, found)) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if ((v[i] & 0x7f80u) == 0x7f80u) v[i] &= 0xffff0000u;
+        if ((v[i] & 0x7f800000u) == 0x7f800000u) v[i] &= 0xffffu;
+    }
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll 1
+    for (int key = 0; key < 16; ++key) {
+        float score[2] = {0.f, 0.f};              // of rows g and g + 8: the three parts of it, the smallest first
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+            for (int part = 2; part >= 0; --part) {
+                const unsigned pair = __shfl_sync(0xffffffffu, key < 8 ? parts[part][half] : parts[part][2 + half], (lane & ~3) | (key & 7) >> 1);
+                score[half] += __uint_as_float(key & 1 ? pair & 0xffff0000u : pair << 16);
+            }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float value = __bfloat162float(tile[key * EP + (e >> 1) * 8 + 2 * t + (e & 1)]);
+            if (isfinite(value)) continue;
+            float(&c)[4] = e >> 1 ? right : left;
+            if (key <= g) c[e & 1] = fmaf(score[0], value, c[e & 1]);
+            if (key <= g + 8) c[2 + (e & 1)] = fmaf(score[1], value, c[2 + (e & 1)]);
+        }
+    }
+}
+
 // The wide build: a chunk's rows of q or k (COUNT tiles at once: they turn by the same angles) as 32-bit numbers, turned by
 // position; `take(tile, row, column, x, y)` gets two neighbouring entries, or, where half the rotary width is odd,
 // `take_one(tile, row, column, x)` every entry. A warp takes a row; a lane that takes entries of rotated pairs has read their
@@ -528,6 +565,7 @@ __global__ void __launch_bounds__(THREADS) chunk_read_kernel(LinearChunksArgs a)
             if (column >= E) continue;
             unsigned v[4];
             ldmatrix_x4_trans(v, v_tile + (kt * 16 + within + (matrix & 1) * 8) * EP + column + (matrix >> 1) * 8);
+            if (kt == (warp & 3)) leave_out_later_tokens(v, v_tile + kt * 16 * EP + column, parts, o[2 * p], o[2 * p + 1]);
             mma_parts<GATED>(o[2 * p], parts, v[0], v[1]);
             mma_parts<GATED>(o[2 * p + 1], parts, v[2], v[3]);
         }
@@ -721,6 +759,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 2) chunk_read_wide_kernel(Linear
             if (column >= E) continue;
             unsigned v[4];
             ldmatrix_x4_trans(v, v_tile + (kt * 16 + within + (matrix & 1) * 8) * EP + column + (matrix >> 1) * 8);
+            if (kt == (warp & 3)) leave_out_later_tokens(v, v_tile + kt * 16 * EP + column, parts, o[2 * p], o[2 * p + 1]);
 #pragma unroll
             for (int part = 2; part >= 0; --part) {
                 mma_bf16(o[2 * p], parts[part], v[0], v[1]);

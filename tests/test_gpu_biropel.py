@@ -335,6 +335,46 @@ def test_the_recurrence_in_chunks(heads, k_heads, dim, vdim):
         assert torch.equal(state[0][3], first[3])
 
 
+@pytest.mark.parametrize("form", ["gates per token", "one decay", "retention"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_a_token_does_not_reach_earlier_ones_of_its_chunk(form, value):
+    """A value that is no finite number, first, last and in the middle of a tile of 16 keys: the rows before it, the other
+    columns and the other sequence keep their bits, the rows from it on show it, in chunks as in the scan."""
+    from kidi_b200.kernels import linear_attention, scalar_recurrence
+    generator = torch.Generator().manual_seed(8)
+    heads, dim, vdim, lengths, slots = 2, 64, 64, (130, 100), (1, 0)
+    total, column = sum(lengths), 19
+    q, k, v, gate = (torch.randn(total, heads * 64, generator=generator).to(torch.bfloat16).cuda() for _ in range(4))
+    coef = (torch.rand(total, heads, 2, generator=generator) * 0.5 + 0.5).cuda()
+    decay = torch.tensor([0.9, 0.99]).cuda()
+    common = dict(heads=heads, dim=dim, vdim=vdim, tables=step_tables(lengths, [0, 0], slots), seqs=2)
+    more = dict(one_token=False, longest=max(lengths))
+
+    def run(values, chunks=True):
+        state = torch.zeros(3, heads, dim, vdim, device="cuda")
+        if form == "retention":
+            out = torch.empty(total, heads * vdim, dtype=torch.bfloat16, device="cuda")
+            return linear_attention.retention(q, k, values, gate, decay, state, out, cos=None, sin=None, rotary_dim=0, key_scale=0.1,
+                                              eps=1e-6, silu=True, **common, **more)
+        if form == "one decay":
+            return linear_attention.linear_attention(q, k, values, decay, state, **common, **more) if chunks else \
+                scalar_recurrence.scalar_recurrence(k, q, values, None, state, k_heads=heads, q_heads=heads, decay=decay, **common)
+        groups = dict(k_heads=heads, q_heads=heads)
+        return linear_attention.gated_recurrence(k, q, values, coef, state, longest=max(lengths), **groups, **common) if chunks else \
+            scalar_recurrence.scalar_recurrence(k, q, values, coef, state, **groups, **common)
+
+    whole = run(v)
+    for row in (0, 9, 16, 31, 63, 64, 79, 129):
+        bad = v.clone()
+        bad[row, column] = value
+        found = run(bad)
+        hurt = torch.zeros(total, heads * vdim, dtype=torch.bool, device="cuda")
+        hurt[row:lengths[0], slice(0, vdim) if form == "retention" else column] = True      # (retention's norm spans a head)
+        assert torch.equal(found[~hurt], whole[~hurt]) and not found[row:lengths[0], column].isfinite().any()
+        if form != "retention":
+            assert torch.equal(run(bad, chunks=False).isfinite(), ~hurt)
+
+
 # ------------------------------------------------------------------ one layer of each kind
 LEFT = dict(heads=4, kv_heads=2, dim=16, vdim=24, scale=0.3)
 LAYERS = {
