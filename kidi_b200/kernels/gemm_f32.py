@@ -53,11 +53,13 @@ _launch = None
 
 
 def _bind():
+    """(Another thread takes `_launch` as soon as it is there: without its types, addresses would be passed in 32 bits.)"""
     global _launch
-    _launch = ops.core().kidi_gemm_f32
-    _launch.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
-                        c_void_p, c_int, c_int, c_void_p, c_void_p]
-    _launch.restype = c_int
+    launch = ops.core().kidi_gemm_f32
+    launch.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
+                       c_void_p, c_int, c_int, c_void_p, c_void_p]
+    launch.restype = c_int
+    _launch = launch
 
 
 def gemm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,

@@ -106,6 +106,25 @@ def test_a_32_bit_product_is_cut_into_whole_chunks_within_its_workspace(rows, fe
         assert chunks * rows * features <= gemm_f32.PARTS_MAX and rows <= 65535
 
 
+def test_the_32_bit_product_is_handed_out_with_its_types(monkeypatch):
+    """Other threads call the library's function as soon as the module names it."""
+    from kidi_b200.kernels import gemm_f32
+
+    class Function:
+        def __setattr__(self, name, value):
+            assert gemm_f32._launch is None
+            object.__setattr__(self, name, value)
+
+    class Library:
+        kidi_gemm_f32 = Function()
+
+    monkeypatch.setattr(gemm_f32, "_launch", None)
+    monkeypatch.setattr(gemm_f32.ops, "core", Library)
+    gemm_f32._bind()
+    assert gemm_f32._launch is Library.kidi_gemm_f32 and gemm_f32._launch.restype is gemm_f32.c_int
+    assert len(gemm_f32._launch.argtypes) == 15
+
+
 def test_32_bit_attention_counts_the_segments_that_a_row_can_see():
     from kidi_b200.kernels import ops
     for reach in (1, 2, 63, 64, 255, 256, 257, 511, 513):
