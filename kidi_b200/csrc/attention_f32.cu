@@ -32,7 +32,7 @@ struct AttentionF32Args {
 };
 
 namespace {
-constexpr int TILE = 64, SEGMENT = 256, THREADS = 128;
+constexpr int TILE = 64, SEGMENT = 256, THREADS = 128, MOST_WIDE = 128;
 
 __device__ __forceinline__ void copy16(float* to, const float* from, const float* somewhere) {       // `from` null: zeros
     const unsigned address = (unsigned)__cvta_generic_to_shared(to);
@@ -543,9 +543,11 @@ __global__ void __launch_bounds__(THREADS, 2) attention_f32_tiles_kernel(Attenti
 template <int TN> int launch_tiles(const AttentionF32Args& args, cudaStream_t stream) {
     const AttentionArgs& a = args.a;
     const int stages = (a.head_dim + DEPTH - 1) / DEPTH;
-    const size_t bytes = ((size_t)(stages + 2) * DEPTH * TILE + TILE * 16 * TN + TILE * TILE) * sizeof(float);
+    auto needed = [](int stages) { return ((size_t)(stages + 2) * DEPTH * TILE + TILE * 16 * TN + TILE * TILE) * sizeof(float); };
+    const size_t bytes = needed(stages);
     auto kernel = attention_f32_tiles_kernel<TN>;
-    const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    // (One bound for heads of every width: another thread may be between setting its own and its launch.)
+    const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)needed(MOST_WIDE / DEPTH));
     if (status != cudaSuccess) return (int)status;
     return kidi_launch(kernel, dim3((args.max_new + TILE - 1) / TILE, a.heads, args.seqs), dim3(THREADS), bytes, stream, args);
 }
@@ -571,7 +573,8 @@ KIDI_API int kidi_attention_f32(const AttentionF32Args* arguments, int tiles, cu
         a.kv_heads * blocks > 65535)
         return KIDI_REFUSED_SIZE;
     const size_t bytes = (size_t)TILE * (a.head_dim + KEY_PAD + vd) * sizeof(float);
-    const cudaError_t status = cudaFuncSetAttribute(attention_f32_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    constexpr size_t most = (size_t)TILE * (2 * MOST_WIDE + KEY_PAD) * sizeof(float);         // (as in launch_tiles)
+    const cudaError_t status = cudaFuncSetAttribute(attention_f32_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (status != cudaSuccess) return (int)status;
     const int code = kidi_launch(attention_f32_rows_kernel, dim3(a.rows, a.kv_heads * blocks, args.shares), dim3(THREADS), bytes, stream, args);
     if (code || !args.parts) return code;

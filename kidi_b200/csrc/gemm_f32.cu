@@ -56,6 +56,7 @@ constexpr int FEATURES = 16;                  // of a block
 constexpr int STEP = 16;                      // k of a stage, for each of a warp's four chunks
 constexpr int PITCH = STEP + 4;               // floats between a stage's rows: the 16-byte pieces of eight rows meet no bank twice
 constexpr int MOST_WARPS = 3;
+constexpr size_t MOST_SHARED = 227 * 1024;
 
 // ROWS x EACH: the rows and the features of a lane; eight lanes have a chunk's 16 features and PADDED rows (PADDED >= M).
 template <int PADDED, int EACH, int STAGES, bool ALIGNED, typename TY>
@@ -160,12 +161,11 @@ int launch_rows(const float* x, const float* w, void* y, int M, int N, int K, lo
     // As many warps as share the chunks evenly, at most MOST_WARPS (two such blocks fit an SM's shared memory).
     const int turns = (fours + MOST_WARPS - 1) / MOST_WARPS, warps = (fours + turns - 1) / turns;
     const size_t bytes = ((size_t)warps * STAGES * 4 * (FEATURES + PADDED) * PITCH + (size_t)chunks * PADDED * FEATURES) * sizeof(float);
-    if (bytes > 227 * 1024) return KIDI_REFUSED_SIZE;
+    if (bytes > MOST_SHARED) return KIDI_REFUSED_SIZE;
     auto kernel = gemm_f32_rows_kernel<PADDED, EACH, STAGES, ALIGNED, TY>;
-    if (bytes > 48 * 1024) {
-        const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (status != cudaSuccess) return (int)status;
-    }
+    // (One bound for every launch: another thread may be between setting its own and its launch.)
+    const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST_SHARED);
+    if (status != cudaSuccess) return (int)status;
     return kidi_launch(kernel, dim3((N + FEATURES - 1) / FEATURES), dim3(32 * warps), bytes, stream, x, w, (TY*)y, M, N, K, ldx,
                        ldw, ldy, bias);
 }

@@ -464,6 +464,57 @@ def test_attention_over_cache(kind, dtype, geometry):
                   f"{kind}: sequence {index} (start {start}, new {new}, in step {keys_in_step})")
 
 
+def test_32_bit_kernels_of_several_sizes_on_several_threads():
+    """A launch that needs more shared memory beside another thread's that needs less, each on a stream of its own: no launch
+    fails and every result keeps its bits."""
+    import threading
+    from kidi_b200.engine.plan import StepBatch, build_plan
+    from kidi_b200.kernels import gemm_f32, ops
+    generator = torch.Generator().manual_seed(3)
+    draw = lambda *shape: torch.randn(*shape, generator=generator).to(DEVICE)
+
+    def product(k):
+        x, w = draw(8, k), draw(48, k)
+        return lambda: ops.gemm_simt(x, w, torch.float32)
+
+    def attention(width, tiles):
+        plan = build_plan(StepBatch([0], [[0] * 70]), [0], vocab_size=2)
+        tables = Tables()
+        for name in plan.FIELDS:
+            setattr(tables, name, torch.from_numpy(getattr(plan, name)).to(DEVICE))
+        qkv = draw(70, 3 * width)
+
+        def call():
+            out = torch.empty(70, width, device=DEVICE)
+            ops.attention_generic(qkv, out, heads=1, kv_heads=1, head_dim=width, scale=0.1, window=None, tables=tables, kv_view=None,
+                                  keys_in_step=True, ctx=FakeContext(plan, tables), tiles=tiles)
+            return out
+        return call
+
+    assert gemm_f32.plan(8, 48, 12288, 148)[0] == gemm_f32.ROWS
+    pairs = [(product(2048), product(12288)), (attention(16, False), attention(128, False)), (attention(16, True), attention(64, True))]
+    for calls in pairs:
+        wants = [call() for call in calls]
+        torch.cuda.synchronize()
+        wrong = []
+
+        def repeat(call, want):
+            with torch.cuda.stream(torch.cuda.Stream(device=DEVICE)):
+                try:
+                    for _ in range(300):
+                        if not torch.equal(call(), want):
+                            wrong.append("other bits")
+                except Exception as error:
+                    wrong.append(str(error))
+
+        threads = [threading.Thread(target=repeat, args=pair) for pair in list(zip(calls, wants)) * 2]
+        for thread in threads:
+            thread.start()
+        for thread in threads:
+            thread.join()
+        assert not wrong, wrong[:3]
+
+
 # Heads over key/value heads, widths of keys and values, what the layer adds: group sizes around the eight heads of a block,
 # widths around 16, 64 and 128, edges of tiles (64) and segments (256) in starts, lengths, windows and chunks.
 @pytest.mark.parametrize("heads, kv_heads, dim, vdim, options", [
