@@ -331,17 +331,25 @@ __global__ void __launch_bounds__(256) gemm_f32_add_kernel(const float* __restri
 template <class S, bool ALIGNED, typename TY>
 int launch_tiles(const float* x, const float* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
                  const float* bias, int chunks_per_block, float* parts, cudaStream_t stream) {
+    constexpr int MOST = 65535;                                // blocks along the second and third axis of a grid
     const int chunks = (K + CHUNK - 1) / CHUNK, splits = (chunks + chunks_per_block - 1) / chunks_per_block;
-    const int tiles_m = (M + S::rows - 1) / S::rows, tiles_n = (N + S::features - 1) / S::features;
-    if ((splits > 1) != (parts != nullptr) || tiles_n > 65535 || splits > 65535 || (parts && M > 65535)) return KIDI_REFUSED_SIZE;
+    const int tiles_m = (M + S::rows - 1) / S::rows;
+    if ((splits > 1) != (parts != nullptr) || splits > MOST || (parts && (M > MOST || (N - 1) / S::features >= MOST)))
+        return KIDI_REFUSED_SIZE;
     const size_t most = (2 * S::stage + S::tm * S::tn * S::threads) * sizeof(float);
     const size_t bytes = chunks > 1 && !parts ? most : 2 * S::stage * sizeof(float);
     auto kernel = gemm_f32_tiles_kernel<S, ALIGNED, TY>;
     const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (status != cudaSuccess) return (int)status;
-    const int code = kidi_launch(kernel, dim3(tiles_m, tiles_n, splits), dim3(S::threads), bytes, stream, x, w, (TY*)y, M, N, K, ldx,
-                                 ldw, ldy, bias, chunks_per_block, parts);
-    if (code || !parts) return code;
+    for (int n0 = 0; n0 < N; n0 += MOST * S::features) {       // (8.4 million features a launch)
+        const int here = N - n0 < MOST * S::features ? N - n0 : MOST * S::features;
+        const int code = kidi_launch(kernel, dim3(tiles_m, (here + S::features - 1) / S::features, splits), dim3(S::threads), bytes,
+                                     stream, x, w + n0 * ldw, (TY*)y + n0, M, here, K, ldx, ldw, ldy, bias ? bias + n0 : nullptr,
+                                     chunks_per_block, parts);
+        if (code) return code;
+        if (N - here == n0) break;                             // (n0 must not pass the largest int)
+    }
+    if (!parts) return 0;
     return kidi_launch(gemm_f32_add_kernel<TY>, dim3((N + 255) / 256, M), dim3(256), 0, stream, (const float*)parts, (TY*)y, M, N,
                        chunks, ldy, bias);
 }

@@ -464,6 +464,17 @@ def test_attention_over_cache(kind, dtype, geometry):
                   f"{kind}: sequence {index} (start {start}, new {new}, in step {keys_in_step})")
 
 
+def test_gemm_32_bit_with_more_features_than_a_grid_has_tiles():
+    from kidi_b200.kernels import ops
+    generator = torch.Generator(device=DEVICE).manual_seed(1)
+    features, edge = 65535 * 128 + 130, 65535 * 128
+    x, w = torch.randn(17, 4, generator=generator, device=DEVICE), torch.randn(features, 4, generator=generator, device=DEVICE)
+    bias = torch.randn(features, generator=generator, device=DEVICE)
+    found = ops.gemm_simt(x, w, torch.float32, bias=bias)
+    for begin, end in ((0, 300), (edge - 200, edge + 130), (edge, features)):
+        assert torch.equal(found[:, begin:end], ops.gemm_simt(x, w[begin:end], torch.float32, bias=bias[begin:end]))
+
+
 def test_32_bit_kernels_of_several_sizes_on_several_threads():
     """A launch that needs more shared memory beside another thread's that needs less, each on a stream of its own: no launch
     fails and every result keeps its bits."""
