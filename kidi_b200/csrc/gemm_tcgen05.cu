@@ -185,7 +185,7 @@ struct Params {
     long long tail_first;  // the first tile of the tail
     int share, extra;      // of the tail's k-blocks a block takes `share`, the first `extra` blocks one more
     int staged;            // results leave through shared memory and TMA stores (bfloat16 y, 16-byte aligned rows)
-    const int* group_of_tile;   // [token tiles] or null: the tile's tokens take the weight rows from group * group_rows on
+    const int* group_of_tile;   // [token tiles] (GROUPED): the tile's tokens take the weight rows from group * group_rows on
                                 // (a tile whose group is negative holds no tokens and is left out)
     int group_rows;
     const int* used_of_tile;    // [token tiles] or null (all of them): the rows of a tile that are wanted, from its first one on
@@ -206,7 +206,7 @@ struct GroupPieces {
 };
 
 // Shared memory of a block: the stages, the gated epilogue's exchange buffer and two buffers of results on their way out;
-// behind them (`pieces`) what a block knows of weights in groups.
+// behind them (`pieces`, in the build for weights in groups) what a block knows of those.
 template <int BN, int STAGES> __host__ __device__ constexpr size_t shared_floor() {
     constexpr int columns = epilogue_columns<BN>();
     return (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 64 * (columns + 1) * sizeof(float) + 2 * columns * BM * sizeof(bf16);
@@ -223,7 +223,9 @@ template <int BN, int STAGES> __host__ __device__ constexpr size_t shared_floor(
 // A block keeps its ring of operand stages full across the borders of tiles, and the accumulator
 // is double-buffered in tensor memory (2 x BN columns): while the four epilogue warps read one
 // piece of work out, the tensor core is at the next.
-template <int BN, int STAGES, bool GATED, typename TY>
+// GROUPED: weights in groups, a build of its own, so that the others carry neither its tables nor its widths of a tile that are
+// known at run time only (as run-time branches they cost 1,801 rows through gate, up and down of 4,096 x 12,288 0.9%).
+template <int BN, int STAGES, bool GATED, typename TY, bool GROUPED = false>
 __global__ void __launch_bounds__(THREADS, BN <= 64 ? 2 : 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     const __grid_constant__ CUtensorMap map_y, Params p) {
@@ -243,7 +245,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     __shared__ unsigned long long full_bar[STAGES], empty_bar[STAGES], ready_bar[2], drained_bar[2];
     __shared__ unsigned tmem_base_slot;
     __shared__ int gave_up, is_last;
-    constexpr bool PIECES = BN == 256 && sizeof(TY) == 2;      // the build that serves weights in groups
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Where block c's piece of the line begins, and which block holds k-block g of the line.
@@ -257,61 +258,58 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     // feature tile (the blocks at work at one time share few weight tiles and eight token tiles,
     // however long the prompt), column after column.
     const int feature_tiles = (int)(p.tiles / p.token_tiles);
-    const bool grouped = PIECES && p.group_of_tile;
-    GroupPieces* pieces = reinterpret_cast<GroupPieces*>(tiles + shared_floor<BN, STAGES>());      // (grouped launches only)
-    if constexpr (PIECES) {
-        if (grouped) {
-            for (int i = threadIdx.x; i < p.token_tiles; i += THREADS) {
-                pieces->group[i] = (short)p.group_of_tile[i];
-                pieces->wanted[i] = p.used_of_tile ? (unsigned char)min(max(p.used_of_tile[i], 0), GROUP_TILE) : GROUP_TILE;
-            }
-            __syncthreads();
-            if (warp == 0) {
-                int count = 0;
-                for (int base = 0; base < p.token_tiles; base += 32) {
-                    const int i = base + lane;
-                    const int group = i < p.token_tiles ? pieces->group[i] : -1;
-                    int first = i;                         // of the run of the tile's group
-                    while (group >= 0 && first > 0 && pieces->group[first - 1] == group) --first;
-                    const bool begins = group >= 0 && !((i - first) & 1) && pieces->wanted[i] > 0;
-                    const unsigned all = __ballot_sync(0xffffffffu, begins);
-                    if (begins) pieces->tile[count + __popc(all & ((1u << lane) - 1))] = (short)i;
-                    count += __popc(all);
-                }
-                if (lane == 0) pieces->count = count;
-            }
-            __syncthreads();
-            // (a piece's number is at most its tile's: what is overwritten here has been read by then only if everybody reads first)
-            constexpr int MINE = (MOST_GROUP_TILES + THREADS - 1) / THREADS;
-            short group[MINE];
-            unsigned char wanted[MINE];
-#pragma unroll
-            for (int k = 0; k < MINE; ++k) {
-                const int i = threadIdx.x + k * THREADS;
-                group[k] = -1;
-                wanted[k] = 0;
-                if (i < pieces->count) {
-                    const int tile = pieces->tile[i];
-                    const bool two = tile + 1 < p.token_tiles && pieces->group[tile + 1] == pieces->group[tile] && pieces->wanted[tile + 1] > 0;
-                    group[k] = pieces->group[tile];
-                    wanted[k] = (unsigned char)((two ? GROUP_TILE + pieces->wanted[tile + 1] + 15 : pieces->wanted[tile] + 15) / 16);
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int k = 0; k < MINE; ++k) {
-                const int i = threadIdx.x + k * THREADS;
-                if (i < pieces->count) {
-                    pieces->group[i] = group[k];
-                    pieces->wanted[i] = wanted[k];
-                }
-            }
-            __syncthreads();
+    [[maybe_unused]] GroupPieces* pieces = reinterpret_cast<GroupPieces*>(tiles + shared_floor<BN, STAGES>());
+    if constexpr (GROUPED) {
+        for (int i = threadIdx.x; i < p.token_tiles; i += THREADS) {
+            pieces->group[i] = (short)p.group_of_tile[i];
+            pieces->wanted[i] = p.used_of_tile ? (unsigned char)min(max(p.used_of_tile[i], 0), GROUP_TILE) : GROUP_TILE;
         }
+        __syncthreads();
+        if (warp == 0) {
+            int count = 0;
+            for (int base = 0; base < p.token_tiles; base += 32) {
+                const int i = base + lane;
+                const int group = i < p.token_tiles ? pieces->group[i] : -1;
+                int first = i;                         // of the run of the tile's group
+                while (group >= 0 && first > 0 && pieces->group[first - 1] == group) --first;
+                const bool begins = group >= 0 && !((i - first) & 1) && pieces->wanted[i] > 0;
+                const unsigned all = __ballot_sync(0xffffffffu, begins);
+                if (begins) pieces->tile[count + __popc(all & ((1u << lane) - 1))] = (short)i;
+                count += __popc(all);
+            }
+            if (lane == 0) pieces->count = count;
+        }
+        __syncthreads();
+        // (a piece's number is at most its tile's: what is overwritten here has been read by then only if everybody reads first)
+        constexpr int MINE = (MOST_GROUP_TILES + THREADS - 1) / THREADS;
+        short group[MINE];
+        unsigned char wanted[MINE];
+#pragma unroll
+        for (int k = 0; k < MINE; ++k) {
+            const int i = threadIdx.x + k * THREADS;
+            group[k] = -1;
+            wanted[k] = 0;
+            if (i < pieces->count) {
+                const int tile = pieces->tile[i];
+                const bool two = tile + 1 < p.token_tiles && pieces->group[tile + 1] == pieces->group[tile] && pieces->wanted[tile + 1] > 0;
+                group[k] = pieces->group[tile];
+                wanted[k] = (unsigned char)((two ? GROUP_TILE + pieces->wanted[tile + 1] + 15 : pieces->wanted[tile] + 15) / 16);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < MINE; ++k) {
+            const int i = threadIdx.x + k * THREADS;
+            if (i < pieces->count) {
+                pieces->group[i] = group[k];
+                pieces->wanted[i] = wanted[k];
+            }
+        }
+        __syncthreads();
     }
-    const int token_tiles = grouped ? pieces->count : p.token_tiles;
-    const long long whole_tiles = grouped ? (long long)token_tiles * feature_tiles : p.tail_first;
-    const int rounds = grouped ? (int)((whole_tiles + gridDim.x - 1) / gridDim.x) : p.rounds;
+    const int token_tiles = GROUPED ? pieces->count : p.token_tiles;
+    const long long whole_tiles = GROUPED ? (long long)token_tiles * feature_tiles : p.tail_first;
+    const int rounds = GROUPED ? (int)((whole_tiles + gridDim.x - 1) / gridDim.x) : p.rounds;
     auto locate = [&](long long tile, int& token_tile, int& feature_tile) {
         const long long column = tile / (8LL * feature_tiles), within = tile - column * 8 * feature_tiles;
         const int wide = min(8, token_tiles - (int)column * 8);
@@ -320,9 +318,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     };
     // A tile's first token, its tokens (in steps of 16) and, with weights in groups (the experts of a routed feed-forward), its
     // group's first weight row.
-    auto first_token = [&](int token_tile) { return grouped ? pieces->tile[token_tile] * GROUP_TILE : token_tile * BN; };
-    auto columns_of = [&](int token_tile) { return grouped ? pieces->wanted[token_tile] * 16 : BN; };
-    auto group_begin = [&](int token_tile) { return grouped ? pieces->group[token_tile] * p.group_rows : 0; };
+    auto first_token = [&](int token_tile) { return GROUPED ? pieces->tile[token_tile] * GROUP_TILE : token_tile * BN; };
+    auto columns_of = [&](int token_tile) { return GROUPED ? pieces->wanted[token_tile] * 16 : BN; };
+    auto group_begin = [&](int token_tile) { return GROUPED ? pieces->group[token_tile] * p.group_rows : 0; };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -355,7 +353,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             int token_tile, feature_tile;
             locate(tile, token_tile, feature_tile);
             const int f0 = group_begin(token_tile) + feature_tile * SPAN, t0 = first_token(token_tile);
-            const int boxes = grouped ? (columns_of(token_tile) + GROUP_BOX - 1) / GROUP_BOX : 0;
+            const int boxes = (columns_of(token_tile) + GROUP_BOX - 1) / GROUP_BOX;
             for (int i = 0; i < kb_count; ++i, ++issued) {
                 const int s = issued % STAGES;
                 if (issued >= STAGES && !mbarrier_wait(&empty_bar[s], ((issued / STAGES) - 1) & 1, abort_flag)) {
@@ -363,7 +361,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     return;
                 }
                 unsigned char* stage = tiles + (size_t)s * STAGE_BYTES;
-                mbarrier_expect_tx(&full_bar[s], boxes ? A_BYTES + boxes * GROUP_BOX * BK * 2 : STAGE_BYTES);
+                mbarrier_expect_tx(&full_bar[s], GROUPED ? A_BYTES + boxes * GROUP_BOX * BK * 2 : STAGE_BYTES);
                 const int k = (kb_first + i) * BK;
                 if (GATED) {
                     tma_load_2d(stage, &map_w, &full_bar[s], k, f0);                            // 64 gate rows
@@ -371,7 +369,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 } else {
                     tma_load_2d(stage, &map_w, &full_bar[s], k, f0);
                 }
-                if (boxes)
+                if (GROUPED)
                     for (int box = 0; box < boxes; ++box)
                         tma_load_2d(stage + A_BYTES + box * GROUP_BOX * BK * 2, &map_x, &full_bar[s], k, t0 + box * GROUP_BOX);
                 else
@@ -426,8 +424,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         for (int round = 0; round < rounds && !*abort_flag; ++round) {
             const long long tile = blockIdx.x + (long long)round * gridDim.x;
             if (tile >= whole_tiles) break;
-            int token_tile, feature_tile;
-            locate(tile, token_tile, feature_tile);
+            int token_tile = 0, feature_tile;
+            if (GROUPED) locate(tile, token_tile, feature_tile);
             multiply(p.k_blocks, columns_of(token_tile));
         }
         for (long long g = piece_begin; g < piece_end && !*abort_flag;) {
@@ -532,7 +530,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                         asm volatile("bar.sync 1, 128;" ::: "memory");
                         if (threadIdx.x == 64) {
                             tma_store_2d(&map_y, out, f0, t0 + c);
-                            if (CW > 16 && c + 16 < columns) tma_store_2d(&map_y, out + 16 * SPAN, f0, t0 + c + 16);
+                            if (CW > 16 && (!GROUPED || c + 16 < columns)) tma_store_2d(&map_y, out + 16 * SPAN, f0, t0 + c + 16);
                             tma_store_commit();
                         }
                         ++staged_chunks;
@@ -703,9 +701,9 @@ int make_store_map(CUtensorMap* map, void* base, long long tokens, long long fea
 }
 
 // The same with a kilobyte to align the stages.
-template <int BN, int STAGES, typename TY>
+template <int BN, int STAGES, bool GROUPED>
 constexpr size_t shared_bytes() {
-    return shared_floor<BN, STAGES>() + 1024 + (BN == 256 && sizeof(TY) == 2 ? sizeof(GroupPieces) : 0);
+    return shared_floor<BN, STAGES>() + 1024 + (GROUPED ? sizeof(GroupPieces) : 0);
 }
 
 // Sets the kernel up (once) and returns how many of its blocks the device promises to hold on an SM
@@ -713,9 +711,9 @@ constexpr size_t shared_bytes() {
 // tensor memory the device reports one, whatever its other needs; two such blocks do run on an SM
 // together where shared memory and tensor memory allow (measured), which launches whose blocks do not
 // wait for each other make use of.
-template <int BN, int STAGES, bool GATED, typename TY>
+template <int BN, int STAGES, bool GATED, typename TY, bool GROUPED = false>
 int blocks_per_sm() {
-    constexpr size_t shared = shared_bytes<BN, STAGES, TY>();
+    constexpr size_t shared = shared_bytes<BN, STAGES, GROUPED>();
     static_assert(shared <= (BN <= 64 ? 113 : 227) * 1024, "the stages fit an SM's shared memory (twice for small tiles)");
     static std::atomic<int> known_by_device[64];         // 0: not asked yet; else the answer + 1
     int device = 0;
@@ -723,7 +721,7 @@ int blocks_per_sm() {
     std::atomic<int>& known = known_by_device[device];
     int value = known.load(std::memory_order_acquire) - 1;
     if (value < 0) {
-        auto kernel = gemm_tcgen05_kernel<BN, STAGES, GATED, TY>;
+        auto kernel = gemm_tcgen05_kernel<BN, STAGES, GATED, TY, GROUPED>;
         value = 0;
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) == cudaSuccess &&
             cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) ==
@@ -738,12 +736,12 @@ int blocks_per_sm() {
     return value;
 }
 
-template <int BN, int STAGES, bool GATED, typename TY>
+template <int BN, int STAGES, bool GATED, typename TY, bool GROUPED = false>
 int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const CUtensorMap& map_y, const Params& p, int blocks,
            cudaStream_t stream) {
-    constexpr size_t shared = shared_bytes<BN, STAGES, TY>();
-    auto kernel = gemm_tcgen05_kernel<BN, STAGES, GATED, TY>;
-    const int per_sm = blocks_per_sm<BN, STAGES, GATED, TY>();
+    constexpr size_t shared = shared_bytes<BN, STAGES, GROUPED>();
+    auto kernel = gemm_tcgen05_kernel<BN, STAGES, GATED, TY, GROUPED>;
+    const int per_sm = blocks_per_sm<BN, STAGES, GATED, TY, GROUPED>();
     if (per_sm <= 0) return KIDI_REFUSED_SIZE;
     if (p.rounds > 0) {
         kernel<<<blocks, THREADS, shared, stream>>>(map_w, map_x, map_y, p);
@@ -913,7 +911,6 @@ KIDI_API int kidi_gemm_tcgen05(const void* x, const void* w, void* y, int y_dtyp
 KIDI_API int kidi_gemm_tcgen05_grouped(const void* x, const void* w, void* y, int tokens, int features, int K, long long ldx,
                                        long long ldy, int gated, int groups, const int* group_of_tile, const int* used, int* error,
                                        const GateShape* gate, cudaStream_t stream) {
-    constexpr int BN = 256;
     if (tokens <= 0 || features <= 0) return 0;
     const long long rows = (long long)groups * features * (gated ? 2 : 1);
     if (K <= 0 || (K & 7) || (ldx & 7) || (ldy & 7) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)y & 15) ||
@@ -949,8 +946,8 @@ KIDI_API int kidi_gemm_tcgen05_grouped(const void* x, const void* w, void* y, in
         int status = make_map(&map_w, w, rows, K, K, gated ? 64 : BM);
         if (!status) status = make_map(&map_x, from, p.tokens, K, ldx, GROUP_BOX);
         if (!status) status = make_store_map(&map_y, to, p.tokens, features, ldy, span);
-        if (!status) status = gated ? by_tokens<true, bf16>(BN, map_w, map_x, map_y, p, blocks, stream)
-                                    : by_tokens<false, bf16>(BN, map_w, map_x, map_y, p, blocks, stream);
+        if (!status) status = gated ? launch<256, 4, true, bf16, true>(map_w, map_x, map_y, p, blocks, stream)
+                                    : launch<256, 4, false, bf16, true>(map_w, map_x, map_y, p, blocks, stream);
         if (status) return status;
     }
     return 0;
