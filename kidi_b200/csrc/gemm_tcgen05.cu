@@ -266,12 +266,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         }
         __syncthreads();
         if (warp == 0) {
-            int count = 0;
+            int count = 0, run = 0;                    // pieces so far; where the run of the last tile's group begins
             for (int base = 0; base < p.token_tiles; base += 32) {
                 const int i = base + lane;
                 const int group = i < p.token_tiles ? pieces->group[i] : -1;
-                int first = i;                         // of the run of the tile's group
-                while (group >= 0 && first > 0 && pieces->group[first - 1] == group) --first;
+                const unsigned heads = __ballot_sync(0xffffffffu, i < p.token_tiles && (i == 0 || pieces->group[i - 1] != group)) &
+                                       (0xffffffffu >> (31 - lane));
+                const int first = heads ? base + 31 - __clz(heads) : run;      // of the run of the tile's group
+                run = __shfl_sync(0xffffffffu, first, 31);
                 const bool begins = group >= 0 && !((i - first) & 1) && pieces->wanted[i] > 0;
                 const unsigned all = __ballot_sync(0xffffffffu, begins);
                 if (begins) pieces->tile[count + __popc(all & ((1u << lane) - 1))] = (short)i;
