@@ -201,7 +201,7 @@ constexpr int GROUP_BOX = 64;        // tokens of a copy
 struct GroupPieces {
     int count;                       // pieces of work
     short tile[MOST_GROUP_TILES];    // a piece's first tile
-    short group[MOST_GROUP_TILES];   // of a tile (-1: none), then of a piece
+    int group[MOST_GROUP_TILES];     // of a tile (negative: none), then of a piece
     unsigned char wanted[MOST_GROUP_TILES];   // of a tile in rows, then of a piece in steps of 16 tokens
 };
 
@@ -261,7 +261,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     [[maybe_unused]] GroupPieces* pieces = reinterpret_cast<GroupPieces*>(tiles + shared_floor<BN, STAGES>());
     if constexpr (GROUPED) {
         for (int i = threadIdx.x; i < p.token_tiles; i += THREADS) {
-            pieces->group[i] = (short)p.group_of_tile[i];
+            pieces->group[i] = p.group_of_tile[i];
             pieces->wanted[i] = p.used_of_tile ? (unsigned char)min(max(p.used_of_tile[i], 0), GROUP_TILE) : GROUP_TILE;
         }
         __syncthreads();
@@ -284,7 +284,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         __syncthreads();
         // (a piece's number is at most its tile's: what is overwritten here has been read by then only if everybody reads first)
         constexpr int MINE = (MOST_GROUP_TILES + THREADS - 1) / THREADS;
-        short group[MINE];
+        int group[MINE];
         unsigned char wanted[MINE];
 #pragma unroll
         for (int k = 0; k < MINE; ++k) {
@@ -916,7 +916,7 @@ KIDI_API int kidi_gemm_tcgen05_grouped(const void* x, const void* w, void* y, in
     if (tokens <= 0 || features <= 0) return 0;
     const long long rows = (long long)groups * features * (gated ? 2 : 1);
     if (K <= 0 || (K & 7) || (ldx & 7) || (ldy & 7) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)y & 15) ||
-        groups <= 0 || groups > 32767 || rows > 0x7fffffffLL || tokens % GROUP_TILE || !group_of_tile || !error)
+        groups <= 0 || rows > 0x7fffffffLL || tokens % GROUP_TILE || !group_of_tile || !error)
         return KIDI_REFUSED_SIZE;
     const int span = gated ? 64 : BM;
     const int feature_tiles = (features + span - 1) / span;

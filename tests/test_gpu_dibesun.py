@@ -857,6 +857,21 @@ def test_products_over_groups_of_experts(rows, experts, top, hidden, inter, gate
         assert torch.allclose(got[128 * tile:128 * tile + 128], want, atol=2e-2, rtol=2e-2)
 
 
+def test_products_over_groups_of_any_number():
+    """Groups beyond 16 bits, and any negative number for a tile that holds nothing."""
+    from kidi_b200.kernels import tcgen05
+    generator = torch.Generator(device="cuda").manual_seed(4)
+    weight = torch.randn(70000, 8, 8, generator=generator, device="cuda").bfloat16()
+    tiles = torch.tensor([32768, 65537, -65536, 69999, 69999, -2 ** 31, 2], dtype=torch.int32, device="cuda")
+    x = torch.randn(tiles.numel() * 128, 8, generator=generator, device="cuda").bfloat16()
+    got = tcgen05.gemm_grouped(x, weight, tiles, False)
+    for tile, group in enumerate(tiles.tolist()):
+        rows = slice(tile * 128, tile * 128 + 128)
+        if group >= 0:         # sums of eight products in 32 bits, rounded once to bfloat16
+            want = x[rows].double() @ weight[group].double().t()
+            assert torch.allclose(got[rows].double(), want, atol=1e-5, rtol=2.0 ** -8)
+
+
 @pytest.mark.parametrize("gated", [True, False])
 @pytest.mark.parametrize("counts,hidden,inter", [((1, 16, 17, 127, 128, 129, 0, 255, 256, 257, 400, 513), 136, 72), ((300, 0, 40), 64, 136),
                                                  ((131000, 129, 1), 64, 64)])
