@@ -140,13 +140,22 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: t
 # heads of 128 x 64 the scan takes 15 us for 64 tokens, 26 for 128 and 229 for 1,300, the three kernels 20, 20 and 57 (16 heads
 # of 64 x 64: 11 and 17 at 64 tokens, 52 and 19 at 400).
 MIN_GATED_TOKENS = 96
+# (state rows, value width) pairs that it is compiled for, ahead of time like the scan that takes the others: a first prompt
+# must not wait for a compiler, or need one, that the scan does without.
+GATED_WIDTHS = ((128, 64), (64, 64), (128, 128), (16, 16))
+
+
+def gated_chunks_fit(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, coef: torch.Tensor, dim: int, vdim: int, longest: int) -> bool:
+    """Whether a step takes the chunked kernels with gates per token."""
+    return (0 < MIN_CHUNKED_TOKENS and MIN_GATED_TOKENS <= longest and (dim, vdim) in GATED_WIDTHS and coef.dim() == 3
+            and chunks_fit(q, k, v, dim, vdim, longest))
 
 
 def gated_recurrence(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: torch.Tensor, state: torch.Tensor, *, heads: int,
                      k_heads: int, q_heads: int, dim: int, vdim: int, tables, seqs: int, longest: int) -> torch.Tensor:
     """`scalar_recurrence` (S_t = a_t S_(t-1) + b_t k_t v_t^T, o_t = S_t^T q_t) of steps whose longest sequence brings
     `longest` tokens: in chunks on the tensor cores where the rows allow it, else as the scan."""
-    if not (0 < MIN_CHUNKED_TOKENS and MIN_GATED_TOKENS <= longest and coef.dim() == 3 and chunks_fit(q, k, v, dim, vdim, longest)):
+    if not gated_chunks_fit(q, k, v, coef, dim, vdim, longest):
         return scalar_recurrence.scalar_recurrence(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim,
                                                    vdim=vdim, tables=tables, seqs=seqs)
     scalar_recurrence.check(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim, vdim=vdim)

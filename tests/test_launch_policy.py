@@ -154,3 +154,17 @@ def test_work_beside_others_has_scratch_memory_of_its_own():
     with pytest.raises(ZeroDivisionError):
         ctx.beside(lambda: 1 / 0)
     assert ctx.workspace("sums", 8) is mine[0]
+
+
+def test_the_chunked_recurrence_is_taken_for_widths_that_are_compiled_ahead():
+    from kidi_b200.kernels import linear_attention
+
+    def fits(dim, vdim, longest=200, dtype=torch.bfloat16):
+        q, k, v = (torch.zeros(8, 2 * width, dtype=dtype) for width in (dim, dim, vdim))
+        return linear_attention.gated_chunks_fit(q, k, v, torch.zeros(8, 2, 2), dim, vdim, longest)
+
+    for pair in linear_attention.GATED_WIDTHS:
+        assert fits(*pair) and fits(*pair, longest=96) and not fits(*pair, longest=95) and not fits(*pair, dtype=torch.float32)
+    for dim in range(8, 264, 8):
+        for vdim in range(8, 264, 8):
+            assert fits(dim, vdim) == ((dim, vdim) in linear_attention.GATED_WIDTHS)
