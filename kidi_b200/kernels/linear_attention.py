@@ -145,9 +145,13 @@ MIN_GATED_TOKENS = 96
 GATED_WIDTHS = ((128, 64), (64, 64), (128, 128), (16, 16))
 
 
-def gated_chunks_fit(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, coef: torch.Tensor, dim: int, vdim: int, longest: int) -> bool:
+MOST_SEQUENCES = 65535          # blocks along a grid's third axis
+
+
+def gated_chunks_fit(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, coef: torch.Tensor, dim: int, vdim: int, longest: int,
+                     seqs: int = 1) -> bool:
     """Whether a step takes the chunked kernels with gates per token."""
-    return (0 < MIN_CHUNKED_TOKENS and MIN_GATED_TOKENS <= longest and (dim, vdim) in GATED_WIDTHS and coef.dim() == 3
+    return (0 < MIN_CHUNKED_TOKENS and seqs <= MOST_SEQUENCES and MIN_GATED_TOKENS <= longest and (dim, vdim) in GATED_WIDTHS and coef.dim() == 3
             and chunks_fit(q, k, v, dim, vdim, longest))
 
 
@@ -155,7 +159,7 @@ def gated_recurrence(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: to
                      k_heads: int, q_heads: int, dim: int, vdim: int, tables, seqs: int, longest: int) -> torch.Tensor:
     """`scalar_recurrence` (S_t = a_t S_(t-1) + b_t k_t v_t^T, o_t = S_t^T q_t) of steps whose longest sequence brings
     `longest` tokens: in chunks on the tensor cores where the rows allow it, else as the scan."""
-    if not gated_chunks_fit(q, k, v, coef, dim, vdim, longest):
+    if not gated_chunks_fit(q, k, v, coef, dim, vdim, longest, seqs):
         return scalar_recurrence.scalar_recurrence(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim,
                                                    vdim=vdim, tables=tables, seqs=seqs)
     scalar_recurrence.check(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim, vdim=vdim)

@@ -133,6 +133,8 @@ def test_32_bit_attention_counts_the_segments_that_a_row_can_see():
             for position in range(longest or 1100):
                 first = max(0, position - reach + 1)
                 assert position // 256 - first // 256 + 1 <= bound
+    assert ops.attention_f32_tiles(65535 * 64, 65535, 64, 64, 64, 4, 2, 148)
+    assert not ops.attention_f32_tiles(65536 * 64, 65536, 64, 64, 64, 4, 2, 148)
     for rows, segments in ((1, 160), (8, 160), (64, 160), (512, 64), (8, 1)):
         shares = ops.attention_f32_shares(rows, 32, 8, segments, 128, 148)
         assert 1 <= shares <= segments and (shares == 1 or rows * 32 * segments * 130 <= 1 << 26)
@@ -159,12 +161,13 @@ def test_work_beside_others_has_scratch_memory_of_its_own():
 def test_the_chunked_recurrence_is_taken_for_widths_that_are_compiled_ahead():
     from kidi_b200.kernels import linear_attention
 
-    def fits(dim, vdim, longest=200, dtype=torch.bfloat16):
+    def fits(dim, vdim, longest=200, dtype=torch.bfloat16, **more):
         q, k, v = (torch.zeros(8, 2 * width, dtype=dtype) for width in (dim, dim, vdim))
-        return linear_attention.gated_chunks_fit(q, k, v, torch.zeros(8, 2, 2), dim, vdim, longest)
+        return linear_attention.gated_chunks_fit(q, k, v, torch.zeros(8, 2, 2), dim, vdim, longest, **more)
 
     for pair in linear_attention.GATED_WIDTHS:
         assert fits(*pair) and fits(*pair, longest=96) and not fits(*pair, longest=95) and not fits(*pair, dtype=torch.float32)
+        assert fits(*pair, seqs=65535) and not fits(*pair, seqs=65536)       # (one axis of a grid)
     for dim in range(8, 264, 8):
         for vdim in range(8, 264, 8):
             assert fits(dim, vdim) == ((dim, vdim) in linear_attention.GATED_WIDTHS)
