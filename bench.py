@@ -450,7 +450,7 @@ KERNEL_CLASSES = (
 
 
 def kernel_class(name: str, decode: bool = False) -> str:
-    if name.startswith("diff_attention") or name == "attention":      # (`attention`: the general kernel)
+    if name.startswith(("diff_attention", "attention_f32")) or name == "attention":      # (`attention`: the general kernel)
         return "decode attention" if decode else "prompt attention"
     for label, prefixes in KERNEL_CLASSES:
         if name.startswith(prefixes):

@@ -75,4 +75,4 @@ def gemm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, bias: Optiona
     _check(_launch(x.data_ptr(), weight.data_ptr(), out.data_ptr(), dtype_code(out.dtype), rows, features, k, x.stride(0),
                    weight.stride(0), out.stride(0), bias.data_ptr() if bias is not None else 0, form, count,
                    parts.data_ptr() if parts is not None else 0, _stream()),
-           "gemm_simt", 1 if parts is None else 2)
+           "gemm_f32[tiles]" if form else "gemm_f32[rows]", 1 if parts is None else 2)

@@ -172,7 +172,7 @@ def gated_recurrence(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: to
             sums, before, tables.row_seq.data_ptr(), tables.seq_slot.data_ptr(), tables.seq_row0.data_ptr(),
             tables.seq_len.data_ptr(), seqs, heads, head0, here, -(-longest // CHUNK), coef=coef.data_ptr(),
             coef_width=coef.shape[2], k_heads=k_heads, q_heads=q_heads, keeps=keeps.data_ptr())
-        _check(lib.kidi_linear_chunks(ctypes.byref(args), ops._stream()), "scalar_recurrence", 3)
+        _check(lib.kidi_linear_chunks(ctypes.byref(args), ops._stream()), "scalar_recurrence[chunks]", 3)
     return out
 
 

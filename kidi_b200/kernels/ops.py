@@ -953,7 +953,8 @@ def attention_generic(qkv: torch.Tensor, out: torch.Tensor, *, heads: int, kv_he
         shares = 1 if tiles else attention_f32_shares(rows, heads, kv_heads, segments, value_dim, _sms(qkv.device))
         parts = ctx.workspace("attention_f32", rows * heads * segments * (value_dim + 2)) if shares > 1 else None
         more = AttentionF32Args(args, tables.seq_len.data_ptr(), plan.n_seqs, plan.max_new, segments, shares, _ptr(parts))
-        _check(core().kidi_attention_f32(ctypes.byref(more), 1 if tiles else 0, _stream()), "attention", 1 if parts is None else 2)
+        _check(core().kidi_attention_f32(ctypes.byref(more), 1 if tiles else 0, _stream()),
+               "attention_f32[tiles]" if tiles else "attention_f32[rows]", 1 if parts is None else 2)
         return
     _check(core().kidi_attention_generic(ctypes.byref(args), dtype_code(qkv.dtype), _stream()), "attention")
 

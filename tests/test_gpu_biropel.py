@@ -323,7 +323,7 @@ def test_the_recurrence_in_chunks(heads, k_heads, dim, vdim):
         want_state, want = loop(state[0])
         with ops.record_launches() as names:
             chunks = linear_attention.gated_recurrence(k, q, v, coef, state[0], longest=max(lengths), **common)
-        assert names == ["scalar_recurrence"]
+        assert names == ["scalar_recurrence[chunks]"]
         scan = scalar_recurrence.scalar_recurrence(k, q, v, coef, state[1], **common)
         # 32-bit sums of up to 200 tokens and 128 state rows, a rounding of at most 2^-24 a term in a random walk, and factors
         # in three parts that leave 2^-24: some 2^-24 sqrt(200) at the worst, 1.1e-7 and 1.4e-7 measured.

@@ -107,8 +107,10 @@ def test_gemm_32_bit_is_the_same_however_it_is_cut(shape):
           "32-bit product")
     for choice in choices:
         out = torch.full((M, N), float("nan"), device=DEVICE)
-        gemm_f32.gemm(x, w, out, bias, choice)
+        with ops.record_launches() as names:
+            gemm_f32.gemm(x, w, out, bias, choice)
         assert torch.equal(out, found), choice
+        assert set(names) == {"gemm_f32[tiles]" if choice[0] else "gemm_f32[rows]"}
     # Rows that start on no 16-byte boundary, results in bfloat16 and in a matrix with wider rows, and a row by itself.
     odd = torch.empty(M, K + 1, device=DEVICE)[:, 1:].copy_(x)
     assert torch.equal(ops.gemm_simt(odd, w, torch.float32, bias=bias), found)
@@ -568,9 +570,11 @@ def test_attention_in_32_bit_is_the_same_however_it_is_cut(heads, kv_heads, dim,
         if form:
             form["ctx"] = FakeContext(plan, tables)
         out = torch.full((len(rows), heads * vdim), float("nan"), device=DEVICE)
-        ops.attention_generic(qkv[rows], out, heads=heads, kv_heads=kv_heads, head_dim=dim, value_dim=vdim, scale=dim ** -0.5,
-                              window=130 if "window" in options else None, tables=tables, kv_view=view, keys_in_step=in_step,
-                              **extra, **{name: gate[rows] for name, gate in gates.items()}, **form)
+        with ops.record_launches() as names:
+            ops.attention_generic(qkv[rows], out, heads=heads, kv_heads=kv_heads, head_dim=dim, value_dim=vdim, scale=dim ** -0.5,
+                                  window=130 if "window" in options else None, tables=tables, kv_view=view, keys_in_step=in_step,
+                                  **extra, **{name: gate[rows] for name, gate in gates.items()}, **form)
+        assert set(names) == {("attention_f32[tiles]" if form["tiles"] else "attention_f32[rows]") if form else "attention"}
         return out
 
     everything = list(range(total))

@@ -200,6 +200,35 @@ def test_two_attention_mixers_side_by_side_in_a_captured_step(dtype):
     assert bool(expected.isfinite().all())
 
 
+def test_a_layer_names_the_form_of_its_kernels():
+    """32-bit attention on a prompt and on single tokens, a state-space mixer on prompts on either side of its chunks."""
+    from kidi_b200.kernels import ops
+    from kidi_b200.parts.registry import build_part
+    from kidi_b200.parts.spec import PartSpec
+
+    def names_of(spec, dtype, news):
+        part = build_part("mixer", spec, make_env(dtype))
+        part.bind({name: (t * 0.05).to(DEVICE) for name, t in random_tensors(part, dtype).items()})
+        part.bound()
+        cache, slots = step_context(part.cache_requests(), [0] * len(news[0]), None, dtype)
+        for step in news:
+            ctx, growth = run_step(cache, slots, [[0] * n for n in step], dtype)
+            with ops.record_launches() as names:
+                part.forward(torch.ones(sum(step), 128, dtype=dtype, device=DEVICE), ctx, cache.views(0), True)
+            cache.commit(growth)
+            yield names
+
+    attention = PartSpec("attention", {"hidden_size": 128, "num_heads": 4, "num_kv_heads": 2, "head_dim": 32})
+    prompt, one = names_of(attention, torch.float32, [(300, 200), (1, 1)])
+    assert prompt.count("gemm_f32[tiles]") == 2 and prompt.count("attention_f32[tiles]") == 1 and "attention" not in prompt
+    assert one.count("gemm_f32[rows]") == 2 and one.count("attention_f32[rows]") == 1 and "attention" not in one
+    mixer = PartSpec("mamba2", {"hidden_size": 128, "num_heads": 2, "vdim": 64, "state": 128, "conv": 4, "eps": 1e-5})
+    long, short, one = names_of(mixer, torch.bfloat16, [(96, 130), (95, 20), (1, 1)])
+    assert long.count("scalar_recurrence[chunks]") == 1 and "scalar_recurrence" not in long
+    for names in (short, one):
+        assert names.count("scalar_recurrence") == 1 and "scalar_recurrence[chunks]" not in names
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_part_with_biases(dtype):
     """The same mixer with a bias on the fused q/k/v projection (bound from q, k and v biases by
