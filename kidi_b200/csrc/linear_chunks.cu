@@ -71,6 +71,7 @@ struct LinearChunksArgs {
     const float* coef;      // [rows, heads, coef_width]: decay and write strength of a token first
     int coef_width, k_heads, q_heads;
     float* keeps;           // [chunks, group]: the product of a chunk's decays
+    int least;              // sequences of fewer tokens in the step are left to the scan
 };
 
 namespace {
@@ -183,7 +184,7 @@ struct Chunk {
     bool live;
     __device__ __forceinline__ Chunk(const LinearChunksArgs& a, int seq, int number) {
         const int row0 = a.seq_row0[seq], count = a.seq_len[seq];
-        live = number * CHUNK < count && a.row_seq[row0] >= 0;
+        live = number * CHUNK < count && count >= a.least && a.row_seq[row0] >= 0;
         tokens = min(CHUNK, count - number * CHUNK);
         row = row0 + number * CHUNK;
         index = first_chunk(row0, seq) + number;
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(WALK_THREADS) chunk_states_kernel(LinearChunks
     const int seq = blockIdx.z, head = a.head0 + blockIdx.y;
     const int row0 = a.seq_row0[seq], count = a.seq_len[seq];
     const long long at = 4 * ((long long)blockIdx.x * WALK_THREADS + threadIdx.x);
-    if (count <= 0 || a.row_seq[row0] < 0 || at >= D * E) return;
+    if (count <= 0 || count < a.least || a.row_seq[row0] < 0 || at >= D * E) return;
     const int chunks = (count + CHUNK - 1) / CHUNK;
     const long long stride = (long long)a.group * D * E;
     const float* sums = a.sums + ((long long)first_chunk(row0, seq) * a.group + blockIdx.y) * D * E + at;

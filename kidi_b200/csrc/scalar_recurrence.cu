@@ -16,8 +16,10 @@
 //
 // The state lives in 32-bit floats per cache slot and is carried from token to token; gates, decays, the state,
 // the read-out and the norms are 32-bit. The columns of a head's state are independent, so a block takes 32
-// columns of one (sequence, head) and walks the sequence's rows of the step in order: a token's result depends on
-// the sizes only, not on what else is in the step, nor on how the sequence was cut into steps.
+// columns of one (sequence, head) and walks the sequence's rows of the step in order: a token's state depends on
+// the sizes only, not on what else is in the step, nor on how the sequence was cut into steps. (The state-space mixer's
+// longer bfloat16 prompts go through linear_chunks.cu, whose sums follow the chunks of the sequence's portion: there a
+// token's result depends on how its prompt was cut, by roundings of 32-bit sums, but not on what else is in the step.)
 #include "common.cuh"
 
 struct ScalarRecurrenceArgs {
@@ -37,6 +39,7 @@ struct ScalarRecurrenceArgs {
     int seqs, heads, k_heads, q_heads, dim, vdim, extra, coef_width;
     float q_scale;         // q is multiplied by it
     const float* decay;    // [heads] or null: a_t is this number for every token and b_t is 1 (`coef` is not read)
+    int below;             // > 0: only sequences of fewer tokens in the step (linear_chunks.cu takes the others)
 };
 
 struct ShortConvArgs {
@@ -108,7 +111,7 @@ __global__ void __launch_bounds__(THREADS + 32) scalar_recurrence_kernel(ScalarR
     float* counted = partials + 2 * CHUNK * THREADS;               // [2][CHUNK][32]: the extra column's parts, a lane each
     const int seq = blockIdx.x, head = blockIdx.y;
     const int row0 = a.seq_row0[seq], count = a.seq_len[seq];
-    if (count <= 0 || a.row_seq[row0] < 0) return;        // a padding sequence touches no state
+    if (count <= 0 || a.row_seq[row0] < 0 || (a.below > 0 && count >= a.below)) return;        // a padding sequence touches no state
     const int dim = a.dim, vdim = a.vdim, vcols = a.vdim + a.extra;
     const bool walker = threadIdx.x < THREADS;
     const bool counter = !walker && a.extra && blockIdx.z == 0;    // the warp that keeps the extra column

@@ -36,7 +36,7 @@ class LinearChunksArgs(ctypes.Structure):
                 ("max_chunks", c_int), ("cos_table", c_void_p), ("sin_table", c_void_p), ("row_pos", c_void_p),
                 ("rotary_dim", c_int), ("key_scale", c_float), ("gate", c_void_p), ("ldg", c_longlong),
                 ("finished", c_void_p), ("ldf", c_longlong), ("eps", c_float), ("gate_silu", c_int), ("coef", c_void_p),
-                ("coef_width", c_int), ("k_heads", c_int), ("q_heads", c_int), ("keeps", c_void_p)]
+                ("coef_width", c_int), ("k_heads", c_int), ("q_heads", c_int), ("keeps", c_void_p), ("least", c_int)]
 
 
 # The chunked form on the tensor cores: steps whose longest sequence brings at least this many tokens (0: never).
@@ -136,7 +136,7 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: t
     return out
 
 
-# The fewest tokens of a step's longest sequence from which the chunked form with gates per token is the faster one: at 32
+# The fewest tokens of a sequence from which the chunked form with gates per token is the faster one: at 32
 # heads of 128 x 64 the scan takes 15 us for 64 tokens, 26 for 128 and 229 for 1,300, the three kernels 20, 20 and 57 (16 heads
 # of 64 x 64: 11 and 17 at 64 tokens, 52 and 19 at 400).
 MIN_GATED_TOKENS = 96
@@ -156,9 +156,11 @@ def gated_chunks_fit(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, coef: to
 
 
 def gated_recurrence(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: torch.Tensor, state: torch.Tensor, *, heads: int,
-                     k_heads: int, q_heads: int, dim: int, vdim: int, tables, seqs: int, longest: int) -> torch.Tensor:
-    """`scalar_recurrence` (S_t = a_t S_(t-1) + b_t k_t v_t^T, o_t = S_t^T q_t) of steps whose longest sequence brings
-    `longest` tokens: in chunks on the tensor cores where the rows allow it, else as the scan."""
+                     k_heads: int, q_heads: int, dim: int, vdim: int, tables, seqs: int, longest: int,
+                     shortest: int = 0) -> torch.Tensor:
+    """`scalar_recurrence` (S_t = a_t S_(t-1) + b_t k_t v_t^T, o_t = S_t^T q_t) of steps whose sequences bring `shortest` to
+    `longest` tokens: where the rows allow it in chunks on the tensor cores for the longer ones, else as the scan. A sequence's
+    own tokens choose, so that its state does not depend on what else is in the step."""
     if not gated_chunks_fit(q, k, v, coef, dim, vdim, longest, seqs):
         return scalar_recurrence.scalar_recurrence(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim,
                                                    vdim=vdim, tables=tables, seqs=seqs)
@@ -171,8 +173,11 @@ def gated_recurrence(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: to
             q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), 0, state.data_ptr(), out.data_ptr(),
             sums, before, tables.row_seq.data_ptr(), tables.seq_slot.data_ptr(), tables.seq_row0.data_ptr(),
             tables.seq_len.data_ptr(), seqs, heads, head0, here, -(-longest // CHUNK), coef=coef.data_ptr(),
-            coef_width=coef.shape[2], k_heads=k_heads, q_heads=q_heads, keeps=keeps.data_ptr())
+            coef_width=coef.shape[2], k_heads=k_heads, q_heads=q_heads, keeps=keeps.data_ptr(), least=MIN_GATED_TOKENS)
         _check(lib.kidi_linear_chunks(ctypes.byref(args), ops._stream()), "scalar_recurrence[chunks]", 3)
+    if shortest < MIN_GATED_TOKENS:
+        scalar_recurrence.scalar_recurrence(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim, vdim=vdim,
+                                            tables=tables, seqs=seqs, below=MIN_GATED_TOKENS, out=out)
     return out
 
 

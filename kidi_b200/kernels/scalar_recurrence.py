@@ -22,7 +22,7 @@ class ScalarRecurrenceArgs(ctypes.Structure):
                 ("ldv", c_longlong), ("coef", c_void_p), ("state", c_void_p), ("out", c_void_p), ("row_seq", c_void_p),
                 ("seq_slot", c_void_p), ("seq_row0", c_void_p), ("seq_len", c_void_p), ("seqs", c_int), ("heads", c_int),
                 ("k_heads", c_int), ("q_heads", c_int), ("dim", c_int), ("vdim", c_int), ("extra", c_int),
-                ("coef_width", c_int), ("q_scale", c_float), ("decay", c_void_p)]
+                ("coef_width", c_int), ("q_scale", c_float), ("decay", c_void_p), ("below", c_int)]
 
 
 class ShortConvArgs(ctypes.Structure):
@@ -95,22 +95,23 @@ def check(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: Optional[torc
 def scalar_recurrence(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: Optional[torch.Tensor],
                       state: torch.Tensor, *, heads: int, k_heads: int, q_heads: int, dim: int, vdim: int,
                       extra: int = 0, q_scale: float = 1.0, tables, seqs: int,
-                      decay: Optional[torch.Tensor] = None) -> torch.Tensor:
+                      decay: Optional[torch.Tensor] = None, below: int = 0, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """S_t = a_t S_(t-1) + b_t k_t (v_t, 1 if `extra`)^T and o_t = S_t^T (q_scale q_t) for every sequence's rows of
     the step, from and into `state` [slots + 1, heads, dim, vdim + extra] (float32). k [rows, k_heads * dim],
     q [rows, q_heads * dim], v [rows, heads * vdim] are views of the step's element type (head h reads key head
     h // (heads / k_heads), likewise q); coef float32 [rows, heads, >= 2] holds (a_t, b_t), or `decay`
     (float32 [heads], coef None) holds a_t for every token and b_t is 1. Returns the read-out, float32
-    [rows, heads * (vdim + extra)]."""
+    [rows, heads * (vdim + extra)]. `below` > 0: only the sequences that bring fewer tokens, into `out`."""
     check(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim, vdim=vdim, extra=extra, decay=decay)
     rows = v.shape[0]
-    out = torch.empty((rows, heads * (vdim + extra)), dtype=torch.float32, device=v.device)
+    if out is None:
+        out = torch.empty((rows, heads * (vdim + extra)), dtype=torch.float32, device=v.device)
     args = ScalarRecurrenceArgs(k.data_ptr(), k.stride(0), q.data_ptr(), q.stride(0), v.data_ptr(), v.stride(0),
                                 coef.data_ptr() if coef is not None else 0, state.data_ptr(), out.data_ptr(), tables.row_seq.data_ptr(),
                                 tables.seq_slot.data_ptr(), tables.seq_row0.data_ptr(), tables.seq_len.data_ptr(),
                                 seqs, heads, k_heads, q_heads, dim, vdim, extra,
                                 coef.shape[2] if coef is not None else 0, float(q_scale),
-                                decay.data_ptr() if decay is not None else 0)
+                                decay.data_ptr() if decay is not None else 0, below)
     _check(library().kidi_scalar_recurrence(ctypes.byref(args), dtype_code(v.dtype), ops._stream()), "scalar_recurrence")
     return out
 

@@ -287,11 +287,12 @@ def test_the_state_space_finish_in_pieces_of_eight_entries(heads, vdim, parts):
 
 @pytest.mark.parametrize("heads, k_heads, dim, vdim", [(4, 1, 128, 64), (6, 2, 64, 64), (3, 3, 16, 16), (2, 1, 128, 128)])
 def test_the_recurrence_in_chunks(heads, k_heads, dim, vdim):
-    """Chunks of 64 tokens on the tensor cores against the loop in 64 bits and beside the scan: lengths around a chunk, decays
-    of 0, 1 and everything between, a state that goes on from step to step, other slots' states left alone."""
+    """Chunks of 64 tokens on the tensor cores against the loop in 64 bits and beside the scan: lengths around two chunks and
+    below the fewest tokens (which the scan takes), decays of 0, 1 and everything between, a state that goes on from step to step,
+    other slots' states left alone."""
     from kidi_b200.kernels import linear_attention, ops, scalar_recurrence
     generator = torch.Generator().manual_seed(dim + heads)
-    lengths, slots = (65, 1, 200, 64, 129), (2, 0, 4, 5, 1)
+    lengths, slots = (96, 1, 200, 95, 129), (2, 0, 4, 5, 1)
     total = sum(lengths)
     k, q = (torch.randn(total, k_heads * dim, generator=generator).to(torch.bfloat16).cuda() for _ in range(2))
     v = torch.randn(total, heads * vdim, generator=generator).to(torch.bfloat16).cuda()
@@ -322,8 +323,8 @@ def test_the_recurrence_in_chunks(heads, k_heads, dim, vdim):
     for _ in range(2):              # the second step goes on from the first one's state
         want_state, want = loop(state[0])
         with ops.record_launches() as names:
-            chunks = linear_attention.gated_recurrence(k, q, v, coef, state[0], longest=max(lengths), **common)
-        assert names == ["scalar_recurrence[chunks]"]
+            chunks = linear_attention.gated_recurrence(k, q, v, coef, state[0], longest=max(lengths), shortest=min(lengths), **common)
+        assert names == ["scalar_recurrence[chunks]", "scalar_recurrence"]
         scan = scalar_recurrence.scalar_recurrence(k, q, v, coef, state[1], **common)
         # 32-bit sums of up to 200 tokens and 128 state rows, a rounding of at most 2^-24 a term in a random walk, and factors
         # in three parts that leave 2^-24: some 2^-24 sqrt(200) at the worst, 1.1e-7 and 1.4e-7 measured.
@@ -333,6 +334,29 @@ def test_the_recurrence_in_chunks(heads, k_heads, dim, vdim):
         for held in state[:1]:
             assert float((held.double() - want_state).norm() / want_state.norm()) <= 1e-6
         assert torch.equal(state[0][3], first[3])
+
+
+def test_a_sequence_takes_the_recurrence_of_its_own_length():
+    """Short and long portions in one step: every sequence's rows and state are, bit for bit, those of a step of its own."""
+    from kidi_b200.kernels import linear_attention
+    generator = torch.Generator().manual_seed(12)
+    heads, dim, vdim, lengths, slots = 5, 64, 64, (300, 10, 96, 95, 1), (1, 0, 3, 5, 2)
+    total = sum(lengths)
+    k, q = (torch.randn(total, dim, generator=generator).to(torch.bfloat16).cuda() for _ in range(2))
+    v = torch.randn(total, heads * vdim, generator=generator).to(torch.bfloat16).cuda()
+    coef = torch.rand(total, heads, 2, generator=generator).cuda()
+    first = torch.randn(6, heads, dim, vdim, generator=generator).cuda()
+    common = dict(heads=heads, k_heads=1, q_heads=1, dim=dim, vdim=vdim)
+    state = first.clone()
+    whole = linear_attention.gated_recurrence(k, q, v, coef, state, tables=step_tables(lengths, [0] * 5, slots), seqs=5,
+                                              longest=300, shortest=1, **common)
+    begin = 0
+    for count, slot in zip(lengths, slots):
+        rows, alone = slice(begin, begin + count), first.clone()
+        out = linear_attention.gated_recurrence(k[rows], q[rows], v[rows], coef[rows].contiguous(), alone, seqs=1, longest=count,
+                                                tables=step_tables([count], [0], [slot]), shortest=count, **common)
+        assert torch.equal(state[slot], alone[slot]) and torch.equal(whole[rows], out)
+        begin += count
 
 
 @pytest.mark.parametrize("form", ["gates per token", "one decay", "retention"])
