@@ -23,13 +23,15 @@ TILE_N = 128
 TIMES = {TILES_32: (0, 27, 38, 52, 70), TILES_64: (0, 40, 62, 80)}
 TILE_M = {TILES_32: 32, TILES_64: 64}
 PARTS_MAX = 1 << 27   # floats of the workspace (512 MB)
+PARTS_MB_PER_US = 4   # and the megabytes that a saved microsecond is worth
 
 
 @functools.lru_cache(maxsize=4096)
 def plan(rows: int, features: int, k: int, sms: int) -> Tuple[int, int]:
     """(form, chunks a block adds up): for tiles the height and the share of K with the smallest expected time, which is
     that of the SM with the most blocks, and what the chunks' sums cost on their way through the workspace (4 TB/s, and a
-    launch of 5 us). 301 rows of 4,096 x 12,288: a chunk a block 734 us, all 24 to a block 1,431; 512 rows of 24,576 x 4,096: 2,360 and 2,429."""
+    launch of 5 us) and in memory that is the caller's otherwise: 100 rows of 151,936 x 4,096 would take 464 MB of it to save
+    8 of 3,700 us. 301 rows of 4,096 x 12,288: a chunk a block 734 us, all 24 to a block 1,431."""
     chunks = -(-k // CHUNK)
     if rows <= ROWS_MAX and chunks <= ROWS_CHUNKS:
         return ROWS, chunks
@@ -43,7 +45,7 @@ def plan(rows: int, features: int, k: int, sms: int) -> Tuple[int, int]:
             rounds, rest = divmod(-(-tiles * splits // sms), len(times) - 1)
             cost = (rounds * times[-1] + times[rest]) * count
             if splits > 1:
-                cost += 5 + chunks * rows * features * 8 / 4e6
+                cost += 5 + chunks * rows * features * 8 / 4e6 + chunks * rows * features * 4 / 1e6 / PARTS_MB_PER_US
             if best_cost is None or cost < best_cost:
                 best, best_cost = (form, count), cost
     return best
@@ -71,7 +73,12 @@ def gemm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, bias: Optiona
     features = weight.shape[0]
     form, count = choice or plan(rows, features, k, sm_count(x.device))
     chunks = -(-k // CHUNK)
-    parts = torch.empty(chunks * rows * features, dtype=torch.float32, device=x.device) if form and count < chunks else None
+    parts = None
+    if form and count < chunks:
+        try:
+            parts = torch.empty(chunks * rows * features, dtype=torch.float32, device=x.device)
+        except torch.OutOfMemoryError:         # (the same sums take longer without it)
+            count = chunks
     _check(_launch(x.data_ptr(), weight.data_ptr(), out.data_ptr(), dtype_code(out.dtype), rows, features, k, x.stride(0),
                    weight.stride(0), out.stride(0), bias.data_ptr() if bias is not None else 0, form, count,
                    parts.data_ptr() if parts is not None else 0, _stream()),

@@ -477,6 +477,22 @@ def test_gemm_32_bit_with_more_features_than_a_grid_has_tiles():
         assert torch.equal(found[:, begin:end], ops.gemm_simt(x, w[begin:end], torch.float32, bias=bias[begin:end]))
 
 
+def test_a_32_bit_product_without_memory_for_its_workspace(monkeypatch):
+    from kidi_b200.kernels import gemm_f32
+    generator = torch.Generator().manual_seed(2)
+    x, w = torch.randn(33, 2100, generator=generator).to(DEVICE), torch.randn(130, 2100, generator=generator).to(DEVICE)
+    want, out = (torch.full((33, 130), float("nan"), device=DEVICE) for _ in range(2))
+    gemm_f32.gemm(x, w, want, choice=(gemm_f32.TILES_32, 1))
+
+    def none_left(*_, **__):
+        raise torch.OutOfMemoryError("no memory")
+
+    with monkeypatch.context() as patch:
+        patch.setattr(torch, "empty", none_left)
+        gemm_f32.gemm(x, w, out, choice=(gemm_f32.TILES_32, 1))
+    assert torch.equal(out, want) and not want.isnan().any()
+
+
 def test_32_bit_kernels_of_several_sizes_on_several_threads():
     """A launch that needs more shared memory beside another thread's that needs less, each on a stream of its own: no launch
     fails and every result keeps its bits."""

@@ -106,6 +106,13 @@ def test_a_32_bit_product_is_cut_into_whole_chunks_within_its_workspace(rows, fe
         assert chunks * rows * features <= gemm_f32.PARTS_MAX and rows <= 65535
 
 
+def test_a_32_bit_product_takes_memory_for_what_it_saves():
+    from kidi_b200.kernels import gemm_f32
+    assert gemm_f32.plan(100, 151936, 4096, 148)[1] == 8           # 464 MB would save 8 of 3,700 us
+    for rows, features, k in ((301, 4096, 12288), (301, 24576, 4096), (33, 4096, 12288)):
+        assert gemm_f32.plan(rows, features, k, 148)[1] < -(-k // gemm_f32.CHUNK)
+
+
 def test_the_32_bit_product_is_handed_out_with_its_types(monkeypatch):
     """Other threads call the library's function as soon as the module names it."""
     from kidi_b200.kernels import gemm_f32
