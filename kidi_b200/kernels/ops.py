@@ -950,11 +950,28 @@ def attention_generic(qkv: torch.Tensor, out: torch.Tensor, *, heads: int, kv_he
         if tiles is None:
             tiles = not plan.is_decode and attention_f32_tiles(rows, plan.n_seqs, plan.max_new, plan.max_total, reach, heads, kv_heads,
                                                                _sms(qkv.device))
-        shares = 1 if tiles else attention_f32_shares(rows, heads, kv_heads, segments, value_dim, _sms(qkv.device))
-        parts = ctx.workspace("attention_f32", rows * heads * segments * (value_dim + 2)) if shares > 1 else None
+        row_floats = heads * segments * (value_dim + 2)
+        at_once = rows if tiles else attention_f32_rows_at_once(rows, row_floats)
+        shares = 1 if tiles else attention_f32_shares(at_once, heads, kv_heads, segments, value_dim, _sms(qkv.device))
+        parts = None
+        if shares > 1:
+            try:
+                parts = ctx.workspace("attention_f32", at_once * row_floats)
+            except torch.OutOfMemoryError:         # (the same sums take longer without it)
+                pass
+        if parts is None:
+            at_once, shares = rows, 1
         more = AttentionF32Args(args, tables.seq_len.data_ptr(), plan.n_seqs, plan.max_new, segments, shares, _ptr(parts))
-        _check(core().kidi_attention_f32(ctypes.byref(more), 1 if tiles else 0, _stream()),
-               "attention_f32[tiles]" if tiles else "attention_f32[rows]", 1 if parts is None else 2)
+        for first in range(0, rows, at_once):
+            here = slice(first, min(rows, first + at_once))
+            part = more.a                              # (the rows' own operands; the step's keys stay those of all rows)
+            part.rows = here.stop - first
+            part.q, part.out = qkv[here].data_ptr(), out[here].data_ptr()
+            part.row_seq, part.row_pos = tables.row_seq[here].data_ptr(), tables.row_pos[here].data_ptr()
+            part.gate = gate[here].data_ptr() if gate is not None else 0
+            part.element_gate = element_gate[here].data_ptr() if element_gate is not None else 0
+            _check(core().kidi_attention_f32(ctypes.byref(more), 1 if tiles else 0, _stream()),
+                   "attention_f32[tiles]" if tiles else "attention_f32[rows]", 1 if parts is None else 2)
         return
     _check(core().kidi_attention_generic(ctypes.byref(args), dtype_code(qkv.dtype), _stream()), "attention")
 
@@ -973,9 +990,20 @@ def attention_f32_segments(longest: Optional[int], reach: int) -> int:
     return crossed if longest is None else min(-(-longest // 256), crossed)
 
 
+ATTENTION_F32_PARTS = 1 << 25         # floats of the segments' sums (128 MB)
+
+
+def attention_f32_rows_at_once(rows: int, row_floats: int) -> int:
+    """How many rows a launch takes: equal groups whose segments' sums stay below 128 MB, at least one (a row's sums are some
+    0.2% a query head of what its keys and values take in a cache of that length)."""
+    groups = -(-rows * row_floats // ATTENTION_F32_PARTS)
+    return max(1, -(-rows // max(1, groups)))
+
+
 def attention_f32_shares(rows: int, heads: int, kv_heads: int, segments: int, value_dim: int, sms: int) -> int:
-    """How many blocks share a row's segments: enough for four rounds of three blocks an SM (a block without a segment ends at
-    once, and the blocks of the first segments come first), while the segments' sums stay below 256 MB."""
+    """How many blocks share a row's segments, of the rows of a launch: enough for four rounds of three blocks an SM (a block
+    without a segment ends at once, and the blocks of the first segments come first), while the segments' sums stay below 256 MB
+    (a single row's go beyond that from 131,072 keys at 1,008 heads)."""
     blocks = rows * kv_heads * -(-(heads // kv_heads) // 8)
     if rows * heads * segments * (value_dim + 2) > 1 << 26:
         return 1

@@ -493,6 +493,52 @@ def test_a_32_bit_product_without_memory_for_its_workspace(monkeypatch):
     assert torch.equal(out, want) and not want.isnan().any()
 
 
+def test_32_bit_attention_with_less_memory_for_its_sums(monkeypatch):
+    """Rows in groups of any size, and no memory at all: the bits are those of one launch over all rows."""
+    from kidi_b200.cache.sequence_cache import KVRequest, SequenceCache
+    from kidi_b200.engine.plan import StepBatch, build_plan
+    from kidi_b200.kernels import ops
+    generator = torch.Generator().manual_seed(9)
+    draw = lambda *shape: torch.randn(*shape, generator=generator).to(DEVICE)
+    heads, kv_heads, dim, vdim, held = 9, 3, 20, 36, [900, 0, 255, 1500, 256, 700, 3]
+    cache = SequenceCache([[KVRequest(kv_heads, dim, None, value_dim=vdim)]], max_tokens=8192, max_positions=2048,
+                          dtype=torch.float32, device=torch.device(DEVICE))
+    slots = [cache.acquire() for _ in held]
+    cache.reserve([(slot, count + 1) for slot, count in zip(slots, held)])
+    cache.flush_tables()
+    view = cache.views(0)[0]
+    view.keys.copy_(draw(*view.keys.shape))
+    view.values.copy_(draw(*view.values.shape))
+    plan = build_plan(StepBatch(slots, [[0]] * len(held)), held, vocab_size=2)
+    tables = Tables()
+    for name in plan.FIELDS:
+        setattr(tables, name, torch.from_numpy(getattr(plan, name)).to(DEVICE))
+    tables.row_seq[1] = -1                            # a padding row
+    qkv, gates = draw(7, heads * dim + kv_heads * (dim + vdim)), {"gate": draw(7, heads), "element_gate": draw(7, heads * vdim)}
+
+    class NoMemory(FakeContext):
+        def workspace(self, name, count, zero=False):
+            raise torch.OutOfMemoryError("no memory")
+
+    def run(context=FakeContext):
+        out = torch.full((7, heads * vdim), float("nan"), device=DEVICE)
+        with ops.record_launches() as names:
+            ops.attention_generic(qkv, out, heads=heads, kv_heads=kv_heads, head_dim=dim, value_dim=vdim, scale=0.2, window=None,
+                                  tables=tables, kv_view=view, keys_in_step=False, ctx=context(plan, tables), **gates)
+        assert set(names) == {"attention_f32[rows]"}
+        return out, len(names)
+
+    want, launches = run()
+    assert launches == 1 and not want.isnan().any() and not want[1].any()
+    segments = view.table.shape[1] * view.page_size // 256
+    for rows in (1, 2, 3, 6):
+        monkeypatch.setattr(ops, "ATTENTION_F32_PARTS", rows * heads * segments * (vdim + 2))
+        found, launches = run()
+        assert torch.equal(found, want) and launches == -(-7 // -(-7 // -(-7 // rows)))
+    found, launches = run(NoMemory)
+    assert torch.equal(found, want) and launches == 1
+
+
 def test_32_bit_kernels_of_several_sizes_on_several_threads():
     """A launch that needs more shared memory beside another thread's that needs less, each on a stream of its own: no launch
     fails and every result keeps its bits."""

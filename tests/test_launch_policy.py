@@ -142,6 +142,14 @@ def test_32_bit_attention_counts_the_segments_that_a_row_can_see():
                 assert position // 256 - first // 256 + 1 <= bound
     assert ops.attention_f32_tiles(65535 * 64, 65535, 64, 64, 64, 4, 2, 148)
     assert not ops.attention_f32_tiles(65536 * 64, 65536, 64, 64, 64, 4, 2, 148)
+    # Sequences that may grow long share a launch's sums by rows: no row's segments fall to one block for it.
+    for rows, heads, kv_heads, capacity in ((8, 64, 8, 262144), (64, 32, 8, 40960), (3, 16, 1, 1048576), (1000, 32, 32, 8192)):
+        row_floats = heads * (capacity // 256) * 130
+        at_once = ops.attention_f32_rows_at_once(rows, row_floats)
+        assert 1 <= at_once <= rows and (at_once * row_floats <= 1 << 25 or at_once == 1)
+        shares = ops.attention_f32_shares(at_once, heads, kv_heads, capacity // 256, 128, 148)
+        assert at_once * kv_heads * -(-heads // kv_heads // 8) * shares >= 148
+    assert ops.attention_f32_rows_at_once(0, 100) == 1 and ops.attention_f32_rows_at_once(64, 32 * 160 * 130) == 32
     for rows, segments in ((1, 160), (8, 160), (64, 160), (512, 64), (8, 1)):
         shares = ops.attention_f32_shares(rows, 32, 8, segments, 128, 148)
         assert 1 <= shares <= segments and (shares == 1 or rows * 32 * segments * 130 <= 1 << 26)
