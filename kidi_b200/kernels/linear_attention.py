@@ -3,6 +3,7 @@ when a model with such a layer first runs."""
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Dict, Optional
 
@@ -161,23 +162,30 @@ def gated_recurrence(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, coef: to
     """`scalar_recurrence` (S_t = a_t S_(t-1) + b_t k_t v_t^T, o_t = S_t^T q_t) of steps whose sequences bring `shortest` to
     `longest` tokens: where the rows allow it in chunks on the tensor cores for the longer ones, else as the scan. A sequence's
     own tokens choose, so that its state does not depend on what else is in the step."""
+    scan = functools.partial(scalar_recurrence.scalar_recurrence, k, q, v, coef, state, heads=heads, k_heads=k_heads,
+                             q_heads=q_heads, dim=dim, vdim=vdim, tables=tables, seqs=seqs)
     if not gated_chunks_fit(q, k, v, coef, dim, vdim, longest, seqs):
-        return scalar_recurrence.scalar_recurrence(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim,
-                                                   vdim=vdim, tables=tables, seqs=seqs)
+        return scan()
     scalar_recurrence.check(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim, vdim=vdim)
     rows = v.shape[0]
     out = torch.empty((rows, heads * vdim), dtype=torch.float32, device=v.device)
-    for head0, here, sums, before, lib in _head_groups(rows, seqs, heads, dim, vdim, v.device, False, True):
-        keeps = torch.empty((rows // CHUNK + seqs + 1) * here, dtype=torch.float32, device=v.device)
+    groups = _head_groups(rows, seqs, heads, dim, vdim, v.device, False, True)
+    try:                               # (before the first launch: the kernels advance the state)
+        keeps = torch.empty((rows // CHUNK + seqs + 1) * heads, dtype=torch.float32, device=v.device)
+        group = next(groups)
+    except torch.OutOfMemoryError:     # (the scan needs none beside its result)
+        return scan(out=out)
+    while group is not None:
+        head0, here, sums, before, lib = group
         args = LinearChunksArgs(
             q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), 0, state.data_ptr(), out.data_ptr(),
             sums, before, tables.row_seq.data_ptr(), tables.seq_slot.data_ptr(), tables.seq_row0.data_ptr(),
             tables.seq_len.data_ptr(), seqs, heads, head0, here, -(-longest // CHUNK), coef=coef.data_ptr(),
             coef_width=coef.shape[2], k_heads=k_heads, q_heads=q_heads, keeps=keeps.data_ptr(), least=MIN_GATED_TOKENS)
         _check(lib.kidi_linear_chunks(ctypes.byref(args), ops._stream()), "scalar_recurrence[chunks]", 3)
+        group = next(groups, None)
     if shortest < MIN_GATED_TOKENS:
-        scalar_recurrence.scalar_recurrence(k, q, v, coef, state, heads=heads, k_heads=k_heads, q_heads=q_heads, dim=dim, vdim=vdim,
-                                            tables=tables, seqs=seqs, below=MIN_GATED_TOKENS, out=out)
+        scan(below=MIN_GATED_TOKENS, out=out)
     return out
 
 

@@ -359,6 +359,27 @@ def test_a_sequence_takes_the_recurrence_of_its_own_length():
         begin += count
 
 
+def test_the_recurrence_without_memory_for_its_chunks(monkeypatch):
+    """The chunked form's scratch memory cannot be had: the scan runs, once, over every head and sequence."""
+    from kidi_b200.kernels import linear_attention, ops, scalar_recurrence
+    generator = torch.Generator().manual_seed(3)
+    q, k, v = (torch.randn(150, width, generator=generator).to(torch.bfloat16).cuda() for width in (64, 64, 192))
+    coef, first = torch.rand(150, 3, 2, generator=generator).cuda(), torch.randn(3, 3, 64, 64, generator=generator).cuda()
+    common = dict(heads=3, k_heads=1, q_heads=1, dim=64, vdim=64, tables=step_tables([130, 20], [0, 0], [1, 0]), seqs=2)
+
+    def none_left(*_):
+        raise torch.OutOfMemoryError("no memory")
+        yield
+
+    monkeypatch.setattr(linear_attention, "_head_groups", none_left)
+    states = [first.clone(), first.clone()]
+    with ops.record_launches() as names:
+        found = linear_attention.gated_recurrence(k, q, v, coef, states[0], longest=130, shortest=20, **common)
+    assert names == ["scalar_recurrence"]
+    assert torch.equal(found, scalar_recurrence.scalar_recurrence(k, q, v, coef, states[1], **common))
+    assert torch.equal(*states)
+
+
 @pytest.mark.parametrize("form", ["gates per token", "one decay", "retention"])
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 def test_a_token_does_not_reach_earlier_ones_of_its_chunk(form, value):
