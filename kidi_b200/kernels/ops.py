@@ -29,10 +29,15 @@ def dtype_code(dtype: torch.dtype) -> int:
         raise unsupported(f"the kernels take float32 and bfloat16, not {dtype}") from None
 
 
+_raw_stream, _current_device = (getattr(torch._C, name, None) for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+
+
 def _stream() -> c_void_p:
-    """The current stream's handle. (Asked for once a launch: through `torch.cuda.current_stream()`, which makes a Python
-    object of it, that was 4 of a launch's 15 us on the host.)"""
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    """The current stream's handle. (Asked for once a launch: `torch.cuda.current_stream()`, which makes a Python object of it,
+    is 4 us of a launch's time on the host; it serves where the library does not hand the bare handle out.)"""
+    if _raw_stream is None or _current_device is None:
+        return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(_raw_stream(_current_device()))
 
 
 def _ptr(tensor: Optional[torch.Tensor]) -> c_void_p:

@@ -186,3 +186,16 @@ def test_the_chunked_recurrence_is_taken_for_widths_that_are_compiled_ahead():
     for dim in range(8, 264, 8):
         for vdim in range(8, 264, 8):
             assert fits(dim, vdim) == ((dim, vdim) in linear_attention.GATED_WIDTHS)
+
+
+def test_a_launch_finds_its_stream_by_the_documented_way_too(monkeypatch):
+    from types import SimpleNamespace
+    from kidi_b200.kernels import ops
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: SimpleNamespace(cuda_stream=4711))
+    monkeypatch.setattr(ops, "_current_device", lambda: 3)
+    monkeypatch.setattr(ops, "_raw_stream", lambda device: 100 + device)
+    assert ops._stream().value == 103
+    for name in ("_raw_stream", "_current_device"):
+        with monkeypatch.context() as patch:
+            patch.setattr(ops, name, None)
+            assert ops._stream().value == 4711
