@@ -12,12 +12,13 @@
 //    and 8 x 8 (8 x 4 for values of up to 64), operands by k in shared memory; keys are transposed on the way in, 16
 //    dimensions at a time, values are copied as they lie while the scores are computed. Bound by the multiply-adds and by
 //    what one warp a scheduler leaves idle (two blocks of four warps an SM: 250 registers a thread for two sets of sums):
-//    32 heads of 128 over 8, a prompt of 700 tokens 359 us (23 TFLOP/s), of 2,000 1,718 (a warp a row, head and key before:
-//    5,800 for 2,000).
+//    32 heads of 128 over 8, a prompt of 700 tokens 359 us (23 TFLOP/s), of 2,000 1,718 (attention_generic.cu, a warp a row,
+//    head and key: 5,800 for 2,000).
 //  * rows: decoding, and steps of a few tokens a sequence. A block takes one row, up to eight heads that share a key head,
 //    and every n-th segment, and leaves its sums in a workspace, which a second kernel merges (with one block a row the block
-//    merges them itself). The grid does not depend on how long the sequences are, so a captured step serves all lengths. Bound by the stream of keys and values, 64 KB a tile and block, three blocks an SM: 8 sequences of 1,030 tokens
-//    43 us (455 before), of 4,000 110 (2.4 TB/s).
+//    merges them itself). The grid does not depend on how long the sequences are, so a captured step serves all
+//    lengths. Bound by the stream of keys and values, 64 KB a tile and block, three blocks an SM: 8 sequences of 1,030 tokens
+//    43 us (attention_generic.cu: 455), of 4,000 110 (2.4 TB/s).
 #include <type_traits>
 
 #include "attention_args.cuh"

@@ -10,15 +10,16 @@
 //    four chunks at a time, eight lanes each, so that a lane has up to 4 features x 8 rows although the block's tile is small.
 //    Each warp fills a ring of its own with `cp.async`; there is no barrier of the block before the end. On a B200, weights
 //    of 24,576 x 4,096: 78 us for one row (5.1 TB/s), 106 for eight (3.8 TB/s), 156 for sixteen, where the tiles take 203
-//    and 206 and the 64 x 64 tiles of scalar loads that stood here before took 1,100.
+//    and 206.
 //  * tiles (more rows): bound by the multiply-adds. Where the tiles alone leave SMs idle, the chunks of K are dealt out over
 //    several blocks, whose sums meet in a workspace ([chunks, M, N]) and are added by a kernel of their own, in the same
-//    order. 301 rows of 24,576 x 4,096: 1,475 us, 41 TFLOP/s (a register-only loop of multiply-adds reaches 58 here), before
-//    2,900. Both operands lie in shared memory by k, transposed on the way in: with rows copied as they lie the operands of a
-//    multiply-add come out of 16-byte loads into the same register bank (every second instruction lost an issue slot, 28 to
-//    36 TFLOP/s whatever the tile). Global loads are four lanes a row: a row a lane cost the load/store pipe, which the
-//    shared-memory reads need, 32 lines an instruction (31 TFLOP/s). Packed multiply-adds (two features an instruction, the
-//    row's number stored twice) were no faster (35 to 40): what they save in issue slots they take in shared-memory reads.
+//    order. 301 rows of 24,576 x 4,096: 1,475 us, 41 TFLOP/s (148 x 128 lanes at 1.965 GHz: 74; the vendor's 32-bit product
+//    reaches 53 to 60 here). Both operands lie in shared memory by k, transposed on the way in: with rows copied as they lie
+//    the operands of a multiply-add come out of 16-byte loads into the same register bank (every second instruction lost an
+//    issue slot, 28 to 36 TFLOP/s whatever the tile). Global loads are four lanes a row: a row a lane cost the load/store
+//    pipe, which the shared-memory reads need, 32 lines an instruction (31 TFLOP/s). Packed multiply-adds (two features an
+//    instruction, the row's number stored twice) were no faster (35 to 40): what they save in issue slots they take in
+//    shared-memory reads.
 #include "common.cuh"
 
 namespace {
@@ -158,7 +159,8 @@ template <int PADDED, int EACH, int STAGES, bool ALIGNED, typename TY>
 int launch_rows(const float* x, const float* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
                 const float* bias, cudaStream_t stream) {
     const int chunks = (K + CHUNK - 1) / CHUNK, fours = (chunks + 3) / 4;
-    // As many warps as share the chunks evenly, at most MOST_WARPS (two such blocks fit an SM's shared memory).
+    // As many warps as share the chunks evenly, at most MOST_WARPS: two such blocks fit an SM's shared memory with up to 8
+    // rows, and with 9 to 16 rows up to 23 chunks (beyond, their sums leave room for one).
     const int turns = (fours + MOST_WARPS - 1) / MOST_WARPS, warps = (fours + turns - 1) / turns;
     const size_t bytes = ((size_t)warps * STAGES * 4 * (FEATURES + PADDED) * PITCH + (size_t)chunks * PADDED * FEATURES) * sizeof(float);
     if (bytes > MOST_SHARED) return KIDI_REFUSED_SIZE;
