@@ -945,7 +945,7 @@ def attention_generic(qkv: torch.Tensor, out: torch.Tensor, *, heads: int, kv_he
         value_dim, _ptr(sinks), _ptr(gate), gate.stride(0) if gate is not None else 0, _ptr(weight_bias), int(chunk or 0),
         float(out_scale), 1 if tied else 0, float(key_eps), *(distance_bias.fields(heads) if distance_bias is not None else (0, 0, 0)),
         _ptr(element_gate), element_gate.stride(0) if element_gate is not None else 0)
-    if ctx is not None and attention_f32_fits(qkv, head_dim, value_dim, tied):
+    if rows and ctx is not None and attention_f32_fits(qkv, head_dim, value_dim, tied):
         plan = ctx.plan
         # A captured step serves sequences of any length: its launch follows what a sequence may hold, not what it holds now.
         held = (window, chunk) if kv_view is not None and kv_view.ring_pages else (kv_view.table.shape[1] * kv_view.page_size,) \

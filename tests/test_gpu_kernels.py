@@ -539,6 +539,20 @@ def test_32_bit_attention_with_less_memory_for_its_sums(monkeypatch):
     assert torch.equal(found, want) and launches == 1
 
 
+def test_32_bit_attention_without_rows():
+    """A step without rows launches nothing, whatever form it asks for."""
+    from kidi_b200.engine.plan import StepBatch, build_plan
+    from kidi_b200.kernels import ops
+    plan = build_plan(StepBatch([0], [[0] * 2]), [0], vocab_size=2)
+    tables = Tables()
+    for name in plan.FIELDS:
+        setattr(tables, name, torch.from_numpy(getattr(plan, name)).to(DEVICE))
+    qkv, out = torch.zeros(0, 96, device=DEVICE), torch.zeros(0, 32, device=DEVICE)
+    for tiles in (None, False, True):
+        ops.attention_generic(qkv, out, heads=1, kv_heads=1, head_dim=32, scale=1.0, window=None, tables=tables, kv_view=None,
+                              keys_in_step=True, ctx=FakeContext(plan, tables), tiles=tiles)
+
+
 def test_32_bit_kernels_of_several_sizes_on_several_threads():
     """A launch that needs more shared memory beside another thread's that needs less, each on a stream of its own: no launch
     fails and every result keeps its bits."""
