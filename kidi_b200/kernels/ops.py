@@ -968,13 +968,13 @@ def attention_generic(qkv: torch.Tensor, out: torch.Tensor, *, heads: int, kv_he
             at_once, shares = rows, 1
         more = AttentionF32Args(args, tables.seq_len.data_ptr(), plan.n_seqs, plan.max_new, segments, shares, _ptr(parts))
         for first in range(0, rows, at_once):
-            here = slice(first, min(rows, first + at_once))
-            part = more.a                              # (the rows' own operands; the step's keys stay those of all rows)
-            part.rows = here.stop - first
-            part.q, part.out = qkv[here].data_ptr(), out[here].data_ptr()
-            part.row_seq, part.row_pos = tables.row_seq[here].data_ptr(), tables.row_pos[here].data_ptr()
-            part.gate = gate[here].data_ptr() if gate is not None else 0
-            part.element_gate = element_gate[here].data_ptr() if element_gate is not None else 0
+            if at_once < rows:                         # the rows' own operands (the step's keys stay those of all rows)
+                part, here = more.a, slice(first, min(rows, first + at_once))
+                part.rows = here.stop - first
+                part.q, part.out = qkv[here].data_ptr(), out[here].data_ptr()
+                part.row_seq, part.row_pos = tables.row_seq[here].data_ptr(), tables.row_pos[here].data_ptr()
+                part.gate = gate[here].data_ptr() if gate is not None else 0
+                part.element_gate = element_gate[here].data_ptr() if element_gate is not None else 0
             _check(core().kidi_attention_f32(ctypes.byref(more), 1 if tiles else 0, _stream()),
                    "attention_f32[tiles]" if tiles else "attention_f32[rows]", 1 if parts is None else 2)
         return
