@@ -547,8 +547,8 @@ template <int TN> int launch_tiles(const AttentionF32Args& args, cudaStream_t st
     auto needed = [](int stages) { return ((size_t)(stages + 2) * DEPTH * TILE + TILE * 16 * TN + TILE * TILE) * sizeof(float); };
     const size_t bytes = needed(stages);
     auto kernel = attention_f32_tiles_kernel<TN>;
-    // (One bound for heads of every width: another thread may be between setting its own and its launch.)
-    const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)needed(MOST_WIDE / DEPTH));
+    static std::atomic<unsigned long long> allowed{0};
+    const cudaError_t status = kidi_allow_shared(kernel, needed(MOST_WIDE / DEPTH), allowed);
     if (status != cudaSuccess) return (int)status;
     return kidi_launch(kernel, dim3((args.max_new + TILE - 1) / TILE, a.heads, args.seqs), dim3(THREADS), bytes, stream, args);
 }
@@ -574,8 +574,9 @@ KIDI_API int kidi_attention_f32(const AttentionF32Args* arguments, int tiles, cu
         a.kv_heads * blocks > 65535)
         return KIDI_REFUSED_SIZE;
     const size_t bytes = (size_t)TILE * (a.head_dim + KEY_PAD + vd) * sizeof(float);
-    constexpr size_t most = (size_t)TILE * (2 * MOST_WIDE + KEY_PAD) * sizeof(float);         // (as in launch_tiles)
-    const cudaError_t status = cudaFuncSetAttribute(attention_f32_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    constexpr size_t most = (size_t)TILE * (2 * MOST_WIDE + KEY_PAD) * sizeof(float);
+    static std::atomic<unsigned long long> allowed{0};
+    const cudaError_t status = kidi_allow_shared(attention_f32_rows_kernel, most, allowed);
     if (status != cudaSuccess) return (int)status;
     const int code = kidi_launch(attention_f32_rows_kernel, dim3(a.rows, a.kv_heads * blocks, args.shares), dim3(THREADS), bytes, stream, args);
     if (code || !args.parts) return code;

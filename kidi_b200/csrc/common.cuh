@@ -10,6 +10,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #define KIDI_API extern "C" __attribute__((visibility("default")))
 
 // Element type codes shared with the Python side.
@@ -98,6 +100,21 @@ __device__ __forceinline__ float gate_value(const GateShape& shape, float g, flo
 }
 
 static inline int kidi_launch_status() { return (int)cudaGetLastError(); }
+
+// Lets a kernel's blocks have up to `bytes` of dynamic shared memory: asked for once a device (`done`: a kernel's own bits), with
+// the most that any of its launches needs. A bound that followed each launch could be lowered by another thread between a
+// launch's setting and the launch itself.
+template <typename Kernel>
+static inline cudaError_t kidi_allow_shared(Kernel* kernel, size_t bytes, std::atomic<unsigned long long>& done) {
+    int device = 0;
+    cudaError_t status = cudaGetDevice(&device);
+    if (status != cudaSuccess) return status;
+    const unsigned long long bit = device < 64 ? 1ULL << device : 0;
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (status == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return status;
+}
 
 __device__ __forceinline__ void prefetch_l2(const void* pointer) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(pointer));

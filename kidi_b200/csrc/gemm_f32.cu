@@ -165,8 +165,8 @@ int launch_rows(const float* x, const float* w, void* y, int M, int N, int K, lo
     const size_t bytes = ((size_t)warps * STAGES * 4 * (FEATURES + PADDED) * PITCH + (size_t)chunks * PADDED * FEATURES) * sizeof(float);
     if (bytes > MOST_SHARED) return KIDI_REFUSED_SIZE;
     auto kernel = gemm_f32_rows_kernel<PADDED, EACH, STAGES, ALIGNED, TY>;
-    // (One bound for every launch: another thread may be between setting its own and its launch.)
-    const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST_SHARED);
+    static std::atomic<unsigned long long> allowed{0};
+    const cudaError_t status = kidi_allow_shared(kernel, MOST_SHARED, allowed);
     if (status != cudaSuccess) return (int)status;
     return kidi_launch(kernel, dim3((N + FEATURES - 1) / FEATURES), dim3(32 * warps), bytes, stream, x, w, (TY*)y, M, N, K, ldx,
                        ldw, ldy, bias);
@@ -341,7 +341,8 @@ int launch_tiles(const float* x, const float* w, void* y, int M, int N, int K, l
     const size_t most = (2 * S::stage + S::tm * S::tn * S::threads) * sizeof(float);
     const size_t bytes = chunks > 1 && !parts ? most : 2 * S::stage * sizeof(float);
     auto kernel = gemm_f32_tiles_kernel<S, ALIGNED, TY>;
-    const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    static std::atomic<unsigned long long> allowed{0};
+    const cudaError_t status = kidi_allow_shared(kernel, most, allowed);
     if (status != cudaSuccess) return (int)status;
     for (int n0 = 0; n0 < N; n0 += MOST * S::features) {       // (8.4 million features a launch)
         const int here = N - n0 < MOST * S::features ? N - n0 : MOST * S::features;
