@@ -29,15 +29,17 @@ def dtype_code(dtype: torch.dtype) -> int:
         raise unsupported(f"the kernels take float32 and bfloat16, not {dtype}") from None
 
 
-_raw_stream, _current_device = (getattr(torch._C, name, None) for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+def _stream_reader(library):
+    """A function that returns the current stream's handle. (Asked for once a launch: `torch.cuda.current_stream()`, which makes
+    a Python object of it, is 4 us of a launch's time on the host; it serves where `library`, the tensor library's compiled
+    module, does not hand the bare handle out.)"""
+    raw, device = (getattr(library, name, None) for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+    if raw is None or device is None:
+        return lambda: c_void_p(torch.cuda.current_stream().cuda_stream)
+    return lambda: c_void_p(raw(device()))
 
 
-def _stream() -> c_void_p:
-    """The current stream's handle. (Asked for once a launch: `torch.cuda.current_stream()`, which makes a Python object of it,
-    is 4 us of a launch's time on the host; it serves where the library does not hand the bare handle out.)"""
-    if _raw_stream is None or _current_device is None:
-        return c_void_p(torch.cuda.current_stream().cuda_stream)
-    return c_void_p(_raw_stream(_current_device()))
+_stream = _stream_reader(torch._C)
 
 
 def _ptr(tensor: Optional[torch.Tensor]) -> c_void_p:
@@ -955,8 +957,9 @@ def attention_generic(qkv: torch.Tensor, out: torch.Tensor, *, heads: int, kv_he
         if tiles is None:
             tiles = not plan.is_decode and attention_f32_tiles(rows, plan.n_seqs, plan.max_new, plan.max_total, reach, heads, kv_heads,
                                                                _sms(qkv.device))
-        row_floats = heads * segments * (value_dim + 2)
-        at_once = rows if tiles else attention_f32_rows_at_once(rows, row_floats)
+        row_floats, at_once = heads * segments * (value_dim + 2), rows
+        if not tiles and rows * row_floats > ATTENTION_F32_PARTS:
+            at_once = attention_f32_rows_at_once(rows, row_floats)
         shares = 1 if tiles else attention_f32_shares(at_once, heads, kv_heads, segments, value_dim, _sms(qkv.device))
         parts = None
         if shares > 1:

@@ -192,10 +192,7 @@ def test_a_launch_finds_its_stream_by_the_documented_way_too(monkeypatch):
     from types import SimpleNamespace
     from kidi_b200.kernels import ops
     monkeypatch.setattr(torch.cuda, "current_stream", lambda: SimpleNamespace(cuda_stream=4711))
-    monkeypatch.setattr(ops, "_current_device", lambda: 3)
-    monkeypatch.setattr(ops, "_raw_stream", lambda device: 100 + device)
-    assert ops._stream().value == 103
-    for name in ("_raw_stream", "_current_device"):
-        with monkeypatch.context() as patch:
-            patch.setattr(ops, name, None)
-            assert ops._stream().value == 4711
+    bare = {"_cuda_getCurrentRawStream": lambda device: 100 + device, "_cuda_getDevice": lambda: 3}
+    assert ops._stream_reader(SimpleNamespace(**bare))().value == 103
+    for name in bare:
+        assert ops._stream_reader(SimpleNamespace(**{name: bare[name]}))().value == 4711
