@@ -10,10 +10,10 @@
 //
 //  * tiles: prompts. A block takes 64 consecutive rows of a sequence for one head. Both products are register tiles of 8 x 4
 //    and 8 x 8 (8 x 4 for values of up to 64), operands by k in shared memory; keys are transposed on the way in, 16
-//    dimensions at a time, values are copied as they lie while the scores are computed. Bound by the multiply-adds and by
-//    what one warp a scheduler leaves idle (two blocks of four warps an SM: 250 registers a thread for two sets of sums):
-//    32 heads of 128 over 8, a prompt of 700 tokens 359 us (23 TFLOP/s), of 2,000 1,718 (attention_generic.cu, a warp a row,
-//    head and key: 5,800 for 2,000).
+//    dimensions at a time, values are copied as they lie while the scores are computed. Bound by what two warps a scheduler
+//    leave idle (two blocks of four warps an SM: 250 registers a thread for two sets of sums): 42% of issue slots are used,
+//    and the longest waits are for instructions, of which an unrolled tile is long. 32 heads of 128 over 8, a prompt of 700
+//    tokens 359 us (23 TFLOP/s), of 2,000 1,718 (attention_generic.cu, a warp a row, head and key: 5,800 for 2,000).
 //  * rows: decoding, and steps of a few tokens a sequence. A block takes one row, up to eight heads that share a key head,
 //    and every n-th segment, and leaves its sums in a workspace, which a second kernel merges (with one block a row the block
 //    merges them itself). The grid does not depend on how long the sequences are, so a captured step serves all

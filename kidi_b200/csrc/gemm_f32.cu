@@ -6,8 +6,9 @@
 // multiply-adds over ascending k that starts from zero; the chunks' sums are added in ascending order, then the bias.
 // Elements beyond K count as zeros.
 //
-//  * rows (up to 16 rows: decoding): bound by the stream of the weights. A block has 16 features and all of K. A warp takes
-//    four chunks at a time, eight lanes each, so that a lane has up to 4 features x 8 rows although the block's tile is small.
+//  * rows (up to 16 rows: decoding): the weights' stream, at 57% of the copy rate for eight rows, with 51% of issue slots
+//    used by six warps an SM (what a block's ring leaves room for). A block has 16 features and all of K. A warp takes four
+//    chunks at a time, eight lanes each, so that a lane has up to 4 features x 8 rows although the block's tile is small.
 //    Each warp fills a ring of its own with `cp.async`; there is no barrier of the block before the end. On a B200, weights
 //    of 24,576 x 4,096: 78 us for one row (5.1 TB/s), 106 for eight (3.8 TB/s), 156 for sixteen, where the tiles take 203
 //    and 206.

@@ -332,7 +332,7 @@ __global__ void short_conv_kernel(ShortConvArgs a) {
 }
 
 // The same for bfloat16 rows in 16-byte pieces: a thread takes eight channels of four neighbouring rows, whose taps it shares
-// (seven loads for sixteen), and their weights once. Bound by its instructions (32 exponentials and divisions): 1,800 rows of
+// (seven loads for sixteen), and their weights once. Bound by the wait for its loads (37% of issue slots used): 1,800 rows of
 // 2,304 channels 20 us as a launch of a step, a thread a channel and row 46.
 constexpr int CONV_ROWS = 4;
 template <int TAPS>
@@ -472,9 +472,9 @@ state_space_finish_kernel(const float* __restrict__ read, const T* __restrict__ 
         out[row * ldo + begin + i] = from_float<T>(staged[i] * inv * weight[begin + i]);
 }
 
-// The same in bfloat16 with a warp per (row, part) and eight neighbouring entries a lane at a time, in registers between the
-// two passes (PIECES of them): bound by the traffic, 37 MB for 1,800 rows of 2,048: 14 us as a launch of a step, a block
-// per part with an entry a thread 36.
+// The same in bfloat16 with a warp per (row, part) and eight neighbouring entries a lane at a time, in registers
+// between the two passes (PIECES of them): bound by the wait for its loads (37 MB for 1,800 rows of 2,048; 67% of issue
+// slots used): 14 us as a launch of a step, a block per part with an entry a thread 36.
 template <int PIECES>
 __global__ void __launch_bounds__(THREADS)
 state_space_finish_rows_kernel(const float* __restrict__ read, const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ z,
