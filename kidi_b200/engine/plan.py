@@ -19,6 +19,7 @@ places inside the new tokens.
 from __future__ import annotations
 
 import dataclasses
+import functools
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -52,6 +53,11 @@ class StepPlan:
     seq_len: np.ndarray   # int32 [n_seqs]
     seq_row0: np.ndarray  # int32 [n_seqs]
     want_rows: np.ndarray  # int32 [n_want]
+
+    @functools.cached_property
+    def min_new(self) -> int:
+        """Shortest T_b."""
+        return int(self.seq_len.min())
 
     FIELDS = ("tokens", "row_seq", "row_pos", "seq_slot", "seq_start", "seq_len", "seq_row0", "want_rows")
 

@@ -114,7 +114,7 @@ class StateSpaceMixer(Part):
         read = gated_recurrence(mixed[:, inner:inner + span], mixed[:, inner + span:], values, coef, views[0],
                                 heads=self.heads, k_heads=self.groups, q_heads=self.groups, dim=self.state,
                                 vdim=self.vdim, tables=ctx.tables, seqs=plan.n_seqs, longest=plan.max_new,
-                                shortest=int(plan.seq_len.min()))
+                                shortest=plan.min_new)
         gated = kernels.state_space_finish(read, values, z, self.skip, self.norm, heads=self.heads, vdim=self.vdim,
                                            parts=self.norm_groups, eps=self.eps)
         return self.out.forward(gated)

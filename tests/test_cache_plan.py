@@ -46,6 +46,11 @@ def test_groups_have_storage_of_their_own():
     assert cache.bytes() == 2 * full.keys.numel() * 4 + 2 * ring.keys.numel() * 4
 
 
+def test_a_plan_knows_its_shortest_and_longest_sequence():
+    plan = build_plan(StepBatch([3, 1, 2], [[0] * 5, [0] * 2, [0] * 9]), [7, 0, 1], vocab_size=2)
+    assert (plan.min_new, plan.max_new, plan.max_total) == (2, 9, 12)
+
+
 @pytest.mark.parametrize("grown", [[0], [0, 1, 2, 3], [1, 2, 4], [0, 2, 4, 5], [5]])
 def test_changed_rows_of_the_tables_reach_the_device(grown):
     """Every changed row is copied, whichever rows lie beside each other, and no other row."""
