@@ -39,7 +39,7 @@ COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-
 
 # The libraries of the package: name -> sources. Definitions are added per request.
 LIBRARIES: Dict[str, Tuple[str, ...]] = {
-    "core": ("elementwise.cu", "rowwise.cu", "gemm_simt.cu", "gemm_f32.cu", "gemm_skinny.cu", "gemm_tcgen05.cu",
+    "core": ("elementwise.cu", "rowwise.cu", "gemm_simt.cu", "gemm_f32.cu", "gemm_f32_tensor.cu", "gemm_skinny.cu", "gemm_tcgen05.cu",
              "attention_generic.cu", "attention_f32.cu", "sampling.cu", "lanes.cu"),
     # mixers that only some architectures have: built when a model with such a layer first runs
     "latent_attention": ("latent_attention.cu",),

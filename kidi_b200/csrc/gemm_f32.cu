@@ -1,5 +1,5 @@
-// y[M,N] = x[M,K] * W[N,K]^T (+ bias) with 32-bit operands and 32-bit multiply-adds on the CUDA cores: the products of
-// the 32-bit engine. No reduced-precision matrix mode.
+// y[M,N] = x[M,K] * W[N,K]^T (+ bias) with 32-bit operands and 32-bit multiply-adds on the CUDA cores: the 32-bit products of
+// weights with fewer than 1,024 features, fewer than 512 inputs or rows off 16 bytes (others: gemm_f32_tensor.cu).
 //
 // One order of additions for every shape, so that a row's result does not depend on how many other rows share the launch,
 // on where it falls in a tile, nor on which kernel below runs: K is cut in chunks of 512; a chunk's sum is one chain of fused

@@ -221,8 +221,8 @@ class Engine:
     def check_device_errors(self) -> None:
         """Raises if a kernel gave up a bounded wait (its result would be wrong). Kernels
         that wait on barriers record that instead of hanging; this reads the records."""
-        from ..kernels import tcgen05
-        code = tcgen05.error_code(self.device)
+        from ..kernels import gemm_f32_tensor, tcgen05
+        code = tcgen05.error_code(self.device) or gemm_f32_tensor.gave_up(self.device)
         if code or attention_kernels.timeout_flags():
             raise runtime_error(f"a kernel gave up waiting for its data (matrix product code {code}); "
                                 f"the results of this engine cannot be trusted")

@@ -1,4 +1,5 @@
-"""Matrix products with 32-bit operands and 32-bit multiply-adds (csrc/gemm_f32.cu): how a shape is cut.
+"""Matrix products with 32-bit operands and 32-bit multiply-adds (csrc/gemm_f32.cu): how a shape is cut. Large weights go to the
+tensor cores instead (gemm_f32_tensor).
 
 The result is the same bit for bit whatever is chosen here (see the kernels' order of additions), so a choice may depend on
 the number of rows."""
@@ -9,7 +10,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from . import ops
+from . import gemm_f32_tensor, ops
 from .attention import sm_count
 from .ops import _check, _stream, c_int, c_longlong, c_void_p, dtype_code
 
@@ -69,6 +70,8 @@ def gemm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, bias: Optiona
     """out = x @ weight.T (+ bias) for float32 x and weight with contiguous rows. `choice`: another plan (for tests)."""
     if _launch is None:
         _bind()
+    if choice is None and gemm_f32_tensor.fits(weight):
+        return gemm_f32_tensor.gemm(x, weight, out, bias)
     rows, k = x.shape
     features = weight.shape[0]
     form, count = choice or plan(rows, features, k, sm_count(x.device))

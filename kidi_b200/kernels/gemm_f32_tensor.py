@@ -1,0 +1,123 @@
+"""Matrix products with 32-bit operands on the tensor cores (csrc/gemm_f32_tensor.cu): which weights, and how a shape is cut.
+
+A row's result is the same bit for bit whatever is chosen from the number of rows here, and whether a weight comes here at all
+follows from the weight alone."""
+from __future__ import annotations
+
+import functools
+from typing import Optional, Tuple
+
+import torch
+
+from . import ops
+from .attention import sm_count
+from .ops import _check, _stream, c_int, c_longlong, c_void_p, dtype_code
+
+TILE_N = 128          # features of a tile
+STEP = 64             # k of a step
+# Weights from this size on (and with rows on 16 bytes): 1,024 x 512 is where one row is level with the multiply-adds of
+# gemm_f32 (10 against 12 us; 8 rows 10 against 20). The rule must not look at the number of rows, see above.
+MIN_FEATURES, MIN_K = 1024, 512
+PIECES = 148          # that the line of all steps is cut in (not the device's number of SMs: results would depend on it)
+MOST_HALVES = 1 << 25 # elements of x that are split at a time (128 MB of halves),
+MOST_ROWS = 32768     # and rows
+
+_launch = None
+
+
+def fits(weight: torch.Tensor) -> bool:
+    return (weight.shape[0] >= MIN_FEATURES and weight.shape[1] >= MIN_K and weight.stride(0) % 4 == 0
+            and weight.data_ptr() % 16 == 0)
+
+
+def _line(features: int, k: int) -> Tuple[int, int]:
+    """(tiles of features, steps of a tile)."""
+    return -(-features // TILE_N), -(-k // STEP)
+
+
+def pieces_of(features: int, k: int) -> int:
+    """How many pieces the line of all tiles' steps is cut in: at least four steps each."""
+    tiles, steps = _line(features, k)
+    return min(PIECES, max(1, tiles * steps // 4))
+
+
+@functools.lru_cache(maxsize=4096)
+def plan(rows: int, features: int, k: int, sms: int) -> Tuple[int, bool]:
+    """(rows of a tile, whether parts of a tile meet in memory): the smallest expected time, that of the SM with the most steps.
+    A step takes 0.77 us up to 64 rows and 1.05 at 128; parts cost a kernel (2 us) and their way through the L2 at 5 TB/s.
+    301 rows of 4,096 x 12,288: whole tiles of 80 rows 151 us, pieces with 112 rows 128; of 24,576 x 4,096: 238 by whole tiles
+    of 112, 252 by pieces."""
+    tiles, steps = _line(features, k)
+    pieces = pieces_of(features, k)
+    best, best_cost = None, None
+    for count in range(-(-rows // 128), max(2, -(-rows // 64) + 1)):
+        height = -(-(-(-rows // count)) // 16) * 16
+        count = -(-rows // height)
+        step = max(0.77, 0.5 + 0.0043 * height)
+        for meet in (False, True):
+            if meet:
+                cost = -(-pieces * count // sms) * -(-tiles * steps // pieces) * step
+                cost += 2 + (pieces + tiles) * rows * 1024 / 5e6
+            else:
+                cost = -(-tiles * count // sms) * steps * step
+            if best_cost is None or cost < best_cost:
+                best, best_cost = (height, meet), cost
+    return best
+
+
+def _bind():
+    """(Another thread takes `_launch` as soon as it is there: without its types, addresses would be passed in 32 bits.)"""
+    global _launch
+    launch = ops.core().kidi_gemm_f32_tensor
+    launch.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p,
+                       c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]
+    launch.restype = c_int
+    _launch = launch
+
+
+def gave_up(device: torch.device) -> int:
+    """The number of a bounded wait that ran out (0: none). Reading it synchronises with the device."""
+    if _launch is None:
+        return 0
+    with torch.cuda.device(device):
+        return int(ops.core().kidi_gemm_f32_tensor_gave_up())
+
+
+def _scratch(rows: int, features: int, k: int, meet: bool, device: torch.device) -> Tuple[torch.Tensor, int, int, int]:
+    """Memory of one call, and where in it the tiles' parts (0: none), x's halves and its rows' factors begin."""
+    halves = 4 * rows * (-(-k // 8) * 8)
+    for parts in ((4 * (pieces_of(features, k) + -(-features // TILE_N)) * rows * TILE_N, 0) if meet else (0,)):
+        try:
+            memory = torch.empty(parts + halves + 4 * rows, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:         # (without parts: the same sums by whole tiles)
+            continue
+        at = memory.data_ptr()
+        return memory, at if parts else 0, at + parts, at + parts + halves
+    raise torch.OutOfMemoryError("no memory for the operands of a 32-bit product")
+
+
+def gemm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
+         choice: Optional[Tuple[int, bool]] = None) -> None:
+    """out = x @ weight.T (+ bias) for float32 x and a weight that `fits`. `choice`: another plan (for tests)."""
+    if _launch is None:
+        _bind()
+    all_rows, k = x.shape
+    features = weight.shape[0]
+    sms, pieces = sm_count(x.device), pieces_of(features, k)
+    most = min(MOST_ROWS, max(128, MOST_HALVES // k // 128 * 128))
+    first = 0
+    while first < all_rows:
+        rows = min(most, all_rows - first)
+        height, meet = choice or plan(rows, features, k, sms)
+        try:
+            memory, parts, halves, factors = _scratch(rows, features, k, meet, x.device)
+        except torch.OutOfMemoryError:         # fewer rows at a time
+            if rows <= 16:
+                raise
+            most = rows // 2
+            continue
+        _check(_launch(x.data_ptr() + first * x.stride(0) * 4, weight.data_ptr(), out.data_ptr() + first * out.stride(0) * out.element_size(),
+                       dtype_code(out.dtype), rows, features, k, x.stride(0), weight.stride(0), out.stride(0),
+                       bias.data_ptr() if bias is not None else 0, pieces, height, halves, factors, parts, sms, _stream()),
+               "gemm_f32[tensor]", 3 if parts else 2)
+        first += rows

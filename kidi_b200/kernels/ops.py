@@ -800,7 +800,7 @@ def _gemm_f32():
 
 def gemm_simt(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype,
               out: Optional[torch.Tensor] = None, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """y = x @ weight.T (+ bias) with 32-bit fused multiply-adds, added in an order that depends on K and the types only."""
+    """y = x @ weight.T (+ bias) to 32-bit precision, added in an order that depends on the weight and the types only."""
     _need_cuda(x, weight, bias)
     check_bias(bias, weight.shape[0])
     if x.dim() != 2 or weight.dim() != 2 or x.shape[1] != weight.shape[1]:

@@ -121,6 +121,88 @@ def test_gemm_32_bit_is_the_same_however_it_is_cut(shape):
     assert torch.equal(ops.gemm_simt(x[M // 2:M // 2 + 1], w, torch.float32, bias=bias)[0], found[M // 2])
 
 
+# Edges of the tiles (128 features, 16 to 128 rows), of a step of 64 k, of the pieces that tiles are cut in, and of the rows
+# that are split at a time.
+@pytest.mark.parametrize("shape", [(1, 1024, 512), (3, 1153, 516), (16, 1030, 2052), (17, 1024, 576), (128, 1408, 1000),
+                                   (129, 1025, 640), (200, 4096, 4096), (270, 1100, 1284), (5, 20000, 512)])
+def test_gemm_32_bit_on_tensor_cores(shape, monkeypatch):
+    from kidi_b200.kernels import gemm_f32, gemm_f32_tensor, ops
+    M, N, K = shape
+    generator = torch.Generator().manual_seed(M + N)
+    x, w = torch.randn(M, K, generator=generator).to(DEVICE), torch.randn(N, K, generator=generator).to(DEVICE)
+    w *= torch.logspace(-3, 3, N, device=DEVICE)[:, None]                # features of several sizes
+    bias = torch.randn(N, generator=generator).to(DEVICE)
+    expected = x.double() @ w.double().T
+    with ops.record_launches() as names:
+        found = ops.gemm_simt(x, w, torch.float32)
+    assert names == ["gemm_f32[tensor]"]
+    # Against 64 bits, beside the size that a sum of such products has: no further off than the chains of multiply-adds.
+    size = (x.double().square() @ w.double().square().T).sqrt()
+    error = lambda y: float(((y.double() - expected) / size).square().mean().sqrt())
+    chains = torch.empty(M, N, device=DEVICE)
+    gemm_f32.gemm(x, w, chains, choice=gemm_f32.plan(M, N, K, 148))
+    assert error(found) < error(chains)
+    # A sum of K products whose operands are off by 2^-24.5 each and whose sums of 64 k are cut off four times, 2^-24 each.
+    assert error(found) < 2.0 ** -22
+    with_bias = ops.gemm_simt(x, w, torch.float32, bias=bias)
+    close(with_bias, found.double() + bias.double(), 2.0 ** -24, "bias")
+    for height in (16, 48, 128):
+        for meet in (False, True):
+            out = torch.full((M, N), float("nan"), device=DEVICE)
+            gemm_f32_tensor.gemm(x, w, out, bias, (height, meet))
+            assert torch.equal(out, with_bias), (height, meet)
+    odd = torch.empty(M, K + 1, device=DEVICE)[:, 1:].copy_(x)
+    assert torch.equal(ops.gemm_simt(odd, w, torch.float32, bias=bias), with_bias)
+    wide = torch.zeros(M, N + 3, device=DEVICE)
+    ops.gemm_simt(x, w, torch.float32, out=wide[:, :N], bias=bias)
+    assert torch.equal(wide[:, :N], with_bias) and not wide[:, N:].any()
+    assert torch.equal(ops.gemm_simt(x, w, torch.bfloat16, bias=bias), with_bias.to(torch.bfloat16))
+    assert torch.equal(ops.gemm_simt(x[M // 2:M // 2 + 1], w, torch.float32, bias=bias)[0], with_bias[M // 2])
+    monkeypatch.setattr(gemm_f32_tensor, "MOST_HALVES", 128 * K)         # the rows 128 at a time
+    assert torch.equal(ops.gemm_simt(x, w, torch.float32, bias=bias), with_bias)
+    assert gemm_f32_tensor.gave_up(torch.device(DEVICE)) == 0
+
+
+def test_gemm_32_bit_on_tensor_cores_with_values_of_any_size():
+    """Infinities, NaNs and overflows come out as multiply-adds have them; rows and blocks of very large and very small values keep
+    their precision; zeros stay zeros."""
+    from kidi_b200.kernels import gemm_f32, gemm_f32_tensor, ops
+    generator = torch.Generator().manual_seed(4)
+    M, N, K = 20, 1100, 700
+    x, w = torch.randn(M, K, generator=generator).to(DEVICE), torch.randn(N, K, generator=generator).to(DEVICE)
+    x[1] *= 2.0 ** 60
+    x[2] *= 2.0 ** -100
+    x[3] = 0
+    x[4, ::2] *= 2.0 ** 30
+    w[5] *= 2.0 ** -100
+    w[6, 64:128] *= 2.0 ** 40
+    w[7] = 0
+    expected = x.double() @ w.double().T
+    found = ops.gemm_simt(x, w, torch.float32)
+    assert not found[3].any() and not found[:, 7].any()
+    for i in range(M):
+        for rows in (slice(0, 5), slice(5, 6), slice(6, 7), slice(8, N)):
+            size = float(expected[i, rows].norm())
+            if size > 2.0 ** -115:                                       # (below, 32 bits themselves are coarser)
+                assert float((found[i, rows].double() - expected[i, rows]).norm()) < 2.0 ** -20 * size, (i, rows)
+    x[11], w[12] = 3e38, 3e38                                            # sums beyond the largest number, not always products
+    expected = (x.double() @ w.double().T).float()
+    found = ops.gemm_simt(x, w, torch.float32)
+    assert torch.equal(found.isinf(), expected.isinf()) and torch.equal(found[found.isinf()], expected[found.isinf()])
+    x[11], w[12] = 0, 0
+    x[8, 100], x[9, 3], x[10, 5], x[12, 7], x[12, 8] = math.inf, -math.inf, math.nan, math.inf, -math.inf
+    w[9, 100], w[10, 3], w[11, 1], w[13, 100] = 0, math.inf, math.nan, 1
+    chains = torch.empty(M, N, device=DEVICE)
+    gemm_f32.gemm(x, w, chains, choice=gemm_f32.plan(M, N, K, 148))
+    for height, meet in ((32, False), (32, True), (16, True)):
+        out = torch.empty(M, N, device=DEVICE)
+        gemm_f32_tensor.gemm(x, w, out, None, (height, meet))
+        assert torch.equal(out.isnan(), chains.isnan())
+        assert torch.equal(out.isinf(), chains.isinf()) and torch.equal(out[chains.isinf()], chains[chains.isinf()])
+        clean = [i for i in range(M) if i not in (8, 9, 10, 11, 12)]
+        assert torch.equal(out[clean][:, 14:], found[clean][:, 14:])
+
+
 @pytest.mark.parametrize("rows", [1, 3, 8, 9, 16, 31, 64])
 @pytest.mark.parametrize("shape", [(389, 96), (100, 200), (4096, 1024), (40, 4104)])
 @pytest.mark.parametrize("row_tiles", [1, 2])

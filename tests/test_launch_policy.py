@@ -113,6 +113,19 @@ def test_a_32_bit_product_takes_memory_for_what_it_saves():
         assert gemm_f32.plan(rows, features, k, 148)[1] < -(-k // gemm_f32.CHUNK)
 
 
+@pytest.mark.parametrize("rows", [1, 16, 17, 129, 301, 4000])
+@pytest.mark.parametrize("features, k", [(1024, 512), (4096, 12288), (151936, 4096), (1100, 60000)])
+def test_a_32_bit_product_on_tensor_cores_is_cut_by_its_weight(rows, features, k):
+    from kidi_b200.kernels import gemm_f32_tensor
+    height, meet = gemm_f32_tensor.plan(rows, features, k, 148)
+    assert height % 16 == 0 and 16 <= height <= 128 and meet in (False, True)
+    pieces, line = gemm_f32_tensor.pieces_of(features, k), -(-features // 128) * -(-k // 64)
+    assert 1 <= pieces <= 148 and line // pieces >= 4
+    weight = torch.empty(features, k, device="meta")
+    assert gemm_f32_tensor.fits(weight) and not gemm_f32_tensor.fits(weight[:1023]) and not gemm_f32_tensor.fits(weight[:, :508])
+    assert not gemm_f32_tensor.fits(torch.empty(2048, 1002, device="meta"))
+
+
 def test_the_32_bit_product_is_handed_out_with_its_types(monkeypatch):
     """Other threads call the library's function as soon as the module names it."""
     from kidi_b200.kernels import gemm_f32
