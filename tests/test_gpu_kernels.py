@@ -185,9 +185,15 @@ def test_gemm_32_bit_on_tensor_cores_with_values_of_any_size():
             size = float(expected[i, rows].norm())
             if size > 2.0 ** -115:                                       # (below, 32 bits themselves are coarser)
                 assert float((found[i, rows].double() - expected[i, rows]).norm()) < 2.0 ** -20 * size, (i, rows)
-    x[11], w[12] = 3e38, 3e38                                            # sums beyond the largest number, not always products
+    # Sums beyond the largest number: with a row of such size only the result overflows, with a feature the sums on the way do,
+    # and then it is what the chains make of it.
+    x[11], w[12] = 3e38, 3e38
     expected = (x.double() @ w.double().T).float()
+    chains = torch.empty(M, N, device=DEVICE)
+    gemm_f32.gemm(x, w, chains, choice=gemm_f32.plan(M, N, K, 148))
+    expected[:, 12] = chains[:, 12]
     found = ops.gemm_simt(x, w, torch.float32)
+    assert torch.equal(found.isnan(), expected.isnan())
     assert torch.equal(found.isinf(), expected.isinf()) and torch.equal(found[found.isinf()], expected[found.isinf()])
     x[11], w[12] = 0, 0
     x[8, 100], x[9, 3], x[10, 5], x[12, 7], x[12, 8] = math.inf, -math.inf, math.nan, math.inf, -math.inf
