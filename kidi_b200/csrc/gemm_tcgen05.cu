@@ -64,6 +64,18 @@ __device__ __forceinline__ bool mbarrier_try_wait(unsigned long long* bar, unsig
         : "memory");
     return done != 0;
 }
+// One thread of a warp that is here as a whole. Instructions that take their operands from the warp's shared registers (copies,
+// matrix instructions) are issued at their full rate from such code; from a branch on the lane's number a matrix instruction
+// took 50 to 140 cycles, whatever its size (64 at 128 tokens is what it needs).
+__device__ __forceinline__ bool elect_one() {
+    unsigned elected = 0;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "@p mov.u32 %0, 1;\n\t}"
+        : "+r"(elected));
+    return elected != 0;
+}
 // Bounded wait: false when the limit was reached or another thread has given up.
 __device__ __forceinline__ bool mbarrier_wait(unsigned long long* bar, unsigned parity, volatile int* gave_up) {
     for (unsigned spin = 0; spin < SPIN_LIMIT; ++spin) {
@@ -71,6 +83,12 @@ __device__ __forceinline__ bool mbarrier_wait(unsigned long long* bar, unsigned 
         if ((spin & 1023u) == 1023u && *gave_up) return false;
     }
     return false;
+}
+
+// The same for a whole warp, whose lanes go on together or not at all.
+__device__ __forceinline__ bool mbarrier_wait_warp(unsigned long long* bar, unsigned parity, volatile int* gave_up) {
+    if (__builtin_expect(__all_sync(0xffffffffu, mbarrier_try_wait(bar, parity)), 1)) return true;
+    return __all_sync(0xffffffffu, mbarrier_wait(bar, parity, gave_up));
 }
 
 __device__ __forceinline__ void tma_load_2d(void* smem, const CUtensorMap* map, unsigned long long* bar, int x, int y) {
@@ -108,14 +126,14 @@ __host__ __device__ constexpr unsigned make_instr_desc(int bn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bn >> 3) << 17) | ((unsigned)(BM >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_bf16(unsigned tmem_d, unsigned long long desc_a, unsigned long long desc_b,
-                                          unsigned idesc, unsigned accumulate) {
+template <bool ACCUMULATE>
+__device__ __forceinline__ void umma_bf16(unsigned tmem_d, unsigned long long desc_a, unsigned long long desc_b, unsigned idesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         :
-        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "n"(ACCUMULATE ? 1 : 0)
         : "memory");
 }
 __device__ __forceinline__ void umma_commit(unsigned long long* bar) {
@@ -246,7 +264,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     __shared__ unsigned tmem_base_slot;
     __shared__ int gave_up, is_last;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // Where block c's piece of the line begins, and which block holds k-block g of the line.
     auto begin_of = [&](long long c) -> long long { return c * p.share + (c < p.extra ? c : p.extra); };   // in the tail's line
     auto block_of = [&](long long g) -> int {
@@ -348,9 +366,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const unsigned tmem_base = tmem_base_slot;
     volatile int* abort_flag = &gave_up;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ------------------------------------------------------------ producer
         int issued = 0;                                   // stages filled so far
+        bool ok = true;                                   // (the same in all lanes)
         auto load = [&](long long tile, int kb_first, int kb_count) {
             int token_tile, feature_tile;
             locate(tile, token_tile, feature_tile);
@@ -358,79 +377,91 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             const int boxes = (columns_of(token_tile) + GROUP_BOX - 1) / GROUP_BOX;
             for (int i = 0; i < kb_count; ++i, ++issued) {
                 const int s = issued % STAGES;
-                if (issued >= STAGES && !mbarrier_wait(&empty_bar[s], ((issued / STAGES) - 1) & 1, abort_flag)) {
-                    if (!*abort_flag) { *abort_flag = 1; atomicExch(p.error, 1); }
+                if (issued >= STAGES) ok = mbarrier_wait_warp(&empty_bar[s], ((issued / STAGES) - 1) & 1, abort_flag);
+                if (!ok) {
+                    if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.error, 1); }
                     return;
                 }
-                unsigned char* stage = tiles + (size_t)s * STAGE_BYTES;
-                mbarrier_expect_tx(&full_bar[s], GROUPED ? A_BYTES + boxes * GROUP_BOX * BK * 2 : STAGE_BYTES);
-                const int k = (kb_first + i) * BK;
-                if (GATED) {
-                    tma_load_2d(stage, &map_w, &full_bar[s], k, f0);                            // 64 gate rows
-                    tma_load_2d(stage + A_BYTES / 2, &map_w, &full_bar[s], k, p.features + f0);  // 64 up rows
-                } else {
-                    tma_load_2d(stage, &map_w, &full_bar[s], k, f0);
+                if (elect_one()) {
+                    unsigned char* stage = tiles + (size_t)s * STAGE_BYTES;
+                    mbarrier_expect_tx(&full_bar[s], GROUPED ? A_BYTES + boxes * GROUP_BOX * BK * 2 : STAGE_BYTES);
+                    const int k = (kb_first + i) * BK;
+                    if (GATED) {
+                        tma_load_2d(stage, &map_w, &full_bar[s], k, f0);                            // 64 gate rows
+                        tma_load_2d(stage + A_BYTES / 2, &map_w, &full_bar[s], k, p.features + f0);  // 64 up rows
+                    } else {
+                        tma_load_2d(stage, &map_w, &full_bar[s], k, f0);
+                    }
+                    if (GROUPED)
+                        for (int box = 0; box < boxes; ++box)
+                            tma_load_2d(stage + A_BYTES + box * GROUP_BOX * BK * 2, &map_x, &full_bar[s], k, t0 + box * GROUP_BOX);
+                    else
+                        tma_load_2d(stage + A_BYTES, &map_x, &full_bar[s], k, t0);
                 }
-                if (GROUPED)
-                    for (int box = 0; box < boxes; ++box)
-                        tma_load_2d(stage + A_BYTES + box * GROUP_BOX * BK * 2, &map_x, &full_bar[s], k, t0 + box * GROUP_BOX);
-                else
-                    tma_load_2d(stage + A_BYTES, &map_x, &full_bar[s], k, t0);
+                __syncwarp();
             }
         };
-        for (int round = 0; round < rounds && !*abort_flag; ++round)
+        for (int round = 0; round < rounds && ok; ++round)
             if (blockIdx.x + (long long)round * gridDim.x < whole_tiles)
                 load(blockIdx.x + (long long)round * gridDim.x, 0, p.k_blocks);
-        for (long long g = piece_begin; g < piece_end && !*abort_flag;) {
+        for (long long g = piece_begin; g < piece_end && ok;) {
             const long long tile = g / p.k_blocks;
             const int kb_first = (int)(g - tile * p.k_blocks);
             const int kb_count = (int)min((long long)(p.k_blocks - kb_first), piece_end - g);
             load(p.tail_first + tile, kb_first, kb_count);
             g += kb_count;
         }
-        if (*abort_flag) {  // let the copies in flight land before the block leaves
+        if (!ok) {  // let the copies in flight land before the block leaves
             for (int i = max(0, issued - STAGES); i < issued; ++i)
                 for (unsigned spin = 0; spin < SPIN_LIMIT; ++spin)
                     if (mbarrier_try_wait(&full_bar[i % STAGES], (i / STAGES) & 1)) break;
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // -------------------------------------------------------------- issuer
         int consumed = 0, done = 0;                        // stages read, accumulators finished
+        bool ok = true;                                    // (the same in all lanes)
+        const unsigned memory = __shfl_sync(0xffffffffu, tmem_base, 0);
         auto multiply = [&](int kb_count, int columns) {
             const unsigned idesc = make_instr_desc(columns);
             const int buffer = done & 1;
             // The accumulator's last reader (two pieces of work ago) must have read it out.
-            if (done >= 2 && !mbarrier_wait(&drained_bar[buffer], ((done >> 1) - 1) & 1, abort_flag)) {
-                if (!*abort_flag) { *abort_flag = 1; atomicExch(p.error, 4); }
+            if (done >= 2) ok = mbarrier_wait_warp(&drained_bar[buffer], ((done >> 1) - 1) & 1, abort_flag);
+            if (!ok) {
+                if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.error, 4); }
                 return;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned accumulator = tmem_base + buffer * BUFFER_COLUMNS;
+            const unsigned accumulator = memory + buffer * BUFFER_COLUMNS;
             for (int i = 0; i < kb_count; ++i, ++consumed) {
                 const int s = consumed % STAGES;
-                if (!mbarrier_wait(&full_bar[s], (consumed / STAGES) & 1, abort_flag)) {
-                    if (!*abort_flag) { *abort_flag = 1; atomicExch(p.error, 2); }
-                    break;
+                ok = mbarrier_wait_warp(&full_bar[s], (consumed / STAGES) & 1, abort_flag);
+                if (!ok) {
+                    if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.error, 2); }
+                    return;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                unsigned char* stage = tiles + (size_t)s * STAGE_BYTES;
+                const unsigned char* stage = tiles + (size_t)s * STAGE_BYTES;
                 const unsigned long long desc_a = make_smem_desc(stage), desc_b = make_smem_desc(stage + A_BYTES);
+                if (elect_one()) {      // (32 bytes further inside the swizzle span: +2 in 16-byte units)
+                    if (i == 0) umma_bf16<false>(accumulator, desc_a, desc_b, idesc);
+                    else umma_bf16<true>(accumulator, desc_a, desc_b, idesc);
 #pragma unroll
-                for (int k = 0; k < BK / UMMA_K; ++k)  // 32 bytes further inside the swizzle span: +2 in 16-byte units
-                    umma_bf16(accumulator, desc_a + 2 * k, desc_b + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-                umma_commit(&empty_bar[s]);  // arrives when these instructions have read the stage
+                    for (int k = 1; k < BK / UMMA_K; ++k) umma_bf16<true>(accumulator, desc_a + 2 * k, desc_b + 2 * k, idesc);
+                    umma_commit(&empty_bar[s]);  // arrives when these instructions have read the stage
+                    if (i == kb_count - 1) umma_commit(&ready_bar[buffer]);  // arrives when the accumulator is complete
+                }
+                __syncwarp();
             }
-            umma_commit(&ready_bar[buffer]);  // arrives when the accumulator is complete
             ++done;
         };
-        for (int round = 0; round < rounds && !*abort_flag; ++round) {
+        for (int round = 0; round < rounds && ok; ++round) {
             const long long tile = blockIdx.x + (long long)round * gridDim.x;
             if (tile >= whole_tiles) break;
             int token_tile = 0, feature_tile;
             if (GROUPED) locate(tile, token_tile, feature_tile);
             multiply(p.k_blocks, columns_of(token_tile));
         }
-        for (long long g = piece_begin; g < piece_end && !*abort_flag;) {
+        for (long long g = piece_begin; g < piece_end && ok;) {
             const int kb_first = (int)(g % p.k_blocks);
             const int kb_count = (int)min((long long)(p.k_blocks - kb_first), piece_end - g);
             multiply(kb_count, BN);
