@@ -19,7 +19,7 @@
 // are there (the blocks are launched cooperatively, so they are resident together), the block that
 // brought the i-th part adds the i-th share of the tile's token columns over all parts, in their
 // order along k, so that the result does not depend on timing, and stores it: the sum and the
-// stores are spread over the blocks. Epilogues: store (bfloat16 or float32), or the SiLU gate of a
+// stores are spread over the blocks. From 1,024 tokens on, two SMs have a tile (below). Epilogues: store (bfloat16 or float32), or the SiLU gate of a
 // fused [gate | up] projection, for which a tile is 64 gate rows and the 64 matching up rows.
 //
 // Every wait on an mbarrier is bounded: when the limit is reached the block records a
@@ -197,6 +197,7 @@ struct Params {
     long long ldy;
     int tokens, features;  // features: width of y (for the gated form the weight has 2 * features rows)
     int k_blocks;          // ceil(K / 64): the k-blocks of one tile
+    int columns;           // tokens of a tile (two SMs on a tile)
     int token_tiles;
     long long tiles;
     int rounds;            // whole tiles a block takes for itself: tiles b, b + blocks, ... (while there are)
@@ -228,6 +229,69 @@ struct GroupPieces {
 template <int BN, int STAGES> __host__ __device__ constexpr size_t shared_floor() {
     constexpr int columns = epilogue_columns<BN>();
     return (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 64 * (columns + 1) * sizeof(float) + 2 * columns * BM * sizeof(bf16);
+}
+
+// A tile's results from the accumulator to y, by 128 threads (threads 64 to 191 of the block; `row`: a thread's feature within the
+// tile, or of the gated form its gate or up row). `ok` false: there are none, zeros go out.
+template <bool GATED, int CW, typename TY>
+__device__ __forceinline__ void store_tile(const Params& p, const CUtensorMap& map_y, unsigned accumulator, int f0, int t0, int columns,
+                                           bool ok, int row, float* exchange, bf16* staging, int& staged_chunks) {
+    constexpr int SPAN = GATED ? 64 : BM;
+    TY* y = (TY*)p.y;
+#pragma unroll 1
+    for (int c = 0; c < columns; c += CW) {
+        float v[CW];
+        if (ok) tmem_load<CW>(accumulator + c, v);
+        else
+#pragma unroll
+            for (int i = 0; i < CW; ++i) v[i] = 0.f;
+        // The thread's feature within the tile and its columns of the chunk (gated: half of them).
+        const int feature = GATED ? row & 63 : row;
+        const int first = GATED && row >= 64 ? CW / 2 : 0;
+        constexpr int COUNT = GATED ? CW / 2 : CW;
+        const bool mine = f0 + feature < p.features;
+        if (GATED) {
+            // Rows 64..127 hold the up projection of the features in rows 0..63. The two threads of a feature
+            // share its columns: one takes the first half and gets their up values, the other takes the second
+            // half and gets their gates.
+            float* shared_row = exchange + feature * (CW + 1);
+#pragma unroll
+            for (int i = 0; i < CW / 2; ++i) shared_row[(CW / 2 - first) + i] = row < 64 ? v[CW / 2 + i] : v[i];
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < CW / 2; ++i) {
+                const float other = shared_row[first + i];
+                v[i] = row < 64 ? gate_value_near(p.gate, v[i], other) : gate_value_near(p.gate, other, v[CW / 2 + i]);
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+        } else if (p.bias && mine) {
+            const float shift = p.bias[f0 + row];
+#pragma unroll
+            for (int i = 0; i < CW; ++i) v[i] += shift;
+        }
+        if (sizeof(TY) == 2 && p.staged) {
+            bf16* out = staging + (staged_chunks & 1) * (CW * SPAN);
+            // The copy that read this buffer two chunks ago must be through with it.
+            if (threadIdx.x == 64 && staged_chunks >= 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < COUNT; ++i) out[(first + i) * SPAN + feature] = __float2bfloat16_rn(v[i]);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the copy reads what these threads wrote
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (threadIdx.x == 64) {
+                tma_store_2d(&map_y, out, f0, t0 + c);
+                if (CW > 16 && c + 16 < columns) tma_store_2d(&map_y, out + 16 * SPAN, f0, t0 + c + 16);
+                tma_store_commit();
+            }
+            ++staged_chunks;
+        } else if (mine) {
+#pragma unroll
+            for (int i = 0; i < COUNT; ++i) {
+                const int token = t0 + c + first + i;
+                if (token < p.tokens) y[token * p.ldy + f0 + feature] = from_float<TY>(v[i]);
+            }
+        }
+    }
 }
 
 // Tiles are numbered so that the blocks at work at one time share few weight tiles and few token
@@ -519,65 +583,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 }
                 return;
             }
-            {
-                TY* y = (TY*)p.y;
-#pragma unroll 1
-                for (int c = 0; c < columns; c += CW) {
-                    float v[CW];
-                    if (ok) tmem_load<CW>(accumulator + c, v);
-                    else
-#pragma unroll
-                        for (int i = 0; i < CW; ++i) v[i] = 0.f;
-                    // The thread's feature within the tile and its columns of the chunk (gated: half of them).
-                    const int feature = GATED ? row & 63 : row;
-                    const int first = GATED && row >= 64 ? CW / 2 : 0;
-                    constexpr int COUNT = GATED ? CW / 2 : CW;
-                    const bool mine = f0 + feature < p.features;
-                    if (GATED) {
-                        // Rows 64..127 hold the up projection of the features in rows 0..63. The two threads of a feature
-                        // share its columns: one takes the first half and gets their up values, the other takes the second
-                        // half and gets their gates.
-                        float* shared_row = exchange + feature * (CW + 1);
-#pragma unroll
-                        for (int i = 0; i < CW / 2; ++i) shared_row[(CW / 2 - first) + i] = row < 64 ? v[CW / 2 + i] : v[i];
-                        asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll
-                        for (int i = 0; i < CW / 2; ++i) {
-                            const float other = shared_row[first + i];
-                            v[i] = row < 64 ? gate_value_near(p.gate, v[i], other) : gate_value_near(p.gate, other, v[CW / 2 + i]);
-                        }
-                        asm volatile("bar.sync 1, 128;" ::: "memory");
-                    } else if (p.bias && mine) {
-                        const float shift = p.bias[f0 + row];
-#pragma unroll
-                        for (int i = 0; i < CW; ++i) v[i] += shift;
-                    }
-                    if (sizeof(TY) == 2 && p.staged) {
-                        bf16* out = staging + (staged_chunks & 1) * (CW * SPAN);
-                        // The copy that read this buffer two chunks ago must be through with it.
-                        if (threadIdx.x == 64 && staged_chunks >= 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                        asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll
-                        for (int i = 0; i < COUNT; ++i) out[(first + i) * SPAN + feature] = __float2bfloat16_rn(v[i]);
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the copy reads what these threads wrote
-                        asm volatile("bar.sync 1, 128;" ::: "memory");
-                        if (threadIdx.x == 64) {
-                            tma_store_2d(&map_y, out, f0, t0 + c);
-                            if (CW > 16 && (!GROUPED || c + 16 < columns)) tma_store_2d(&map_y, out + 16 * SPAN, f0, t0 + c + 16);
-                            tma_store_commit();
-                        }
-                        ++staged_chunks;
-                    } else if (mine) {
-#pragma unroll
-                        for (int i = 0; i < COUNT; ++i) {
-                            const int token = t0 + c + first + i;
-                            if (token < p.tokens) y[token * p.ldy + f0 + feature] = from_float<TY>(v[i]);
-                        }
-                    }
-                }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbarrier_arrive(&drained_bar[buffer]);
-            }
+            store_tile<GATED, CW, TY>(p, map_y, accumulator, f0, t0, columns, ok, row, exchange, staging, staged_chunks);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            mbarrier_arrive(&drained_bar[buffer]);
         };
         // A shared tile's second phase: when all its parts have arrived (the blocks of a call are
         // resident together: a cooperative launch), the block that brought the i-th part adds, in the
@@ -674,6 +682,192 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     if (warp == 0) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLUMNS));
     }
+}
+
+// ----------------------------------------------------------------------------------------------- two SMs on a tile (prompts)
+// A pair of blocks has a tile of 2 x 128 features by up to 256 tokens: each loads its own features' weights and half of the
+// tokens, and the first one issues instructions that work on both (`cta_group::2`). What comes from the L2 is a third less than
+// with a block a tile (32 KB an SM and step instead of 48). Tiles are `columns` tokens high, whichever height leaves the least
+// idle in the last round. Bound by the tensor cores at the clock that the power cap leaves (82% of their cycles at 1.5 GHz for
+// 1,801 rows of 24,576 x 4,096). Microseconds, a block a tile and this: 24,576 x 4,096 with 1,801 rows 281 and 272, 4,096 rows
+// 559 and 530; 4,096 x 12,288 with 1,100 rows 154 and 100, 1,801 rows 157 and 141; 6,144 x 4,096 with 1,801 rows 76 and 69;
+// 2,048 x 2,048 with 1,024 rows 26 and 13.
+constexpr int PAIR_STAGES = 6, PAIR_COLUMNS = 256, PAIR_CW = 32;
+constexpr int PAIR_STAGE_BYTES = BM * BK * 2 + PAIR_COLUMNS / 2 * BK * 2;
+constexpr size_t pair_shared_bytes() {
+    return 1024 + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + 64 * (PAIR_CW + 1) * sizeof(float) + 2 * PAIR_CW * BM * sizeof(bf16);
+}
+
+// Both blocks' copies report to the first one's barrier.
+__device__ __forceinline__ void tma_load_pair(void* smem, const CUtensorMap* map, unsigned long long* bar, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        :
+        : "r"(smem_u32(smem)), "l"((unsigned long long)map), "r"(smem_u32(bar) & 0xFEFFFFFFu), "r"(x), "r"(y)
+        : "memory");
+}
+template <bool ACCUMULATE>
+__device__ __forceinline__ void umma_pair(unsigned tmem_d, unsigned long long desc_a, unsigned long long desc_b, unsigned idesc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        :
+        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "n"(ACCUMULATE ? 1 : 0)
+        : "memory");
+}
+// Arrives at both blocks' barriers when the instructions issued so far have been carried out.
+__device__ __forceinline__ void umma_commit_pair(unsigned long long* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"((unsigned short)3)
+                 : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <bool GATED, typename TY>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_tcgen05_pairs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                          const __grid_constant__ CUtensorMap map_y, Params p) {
+    constexpr int A_BYTES = BM * BK * 2, SPAN = GATED ? 64 : BM;
+    extern __shared__ unsigned char raw[];
+    unsigned char* tiles = (unsigned char*)(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
+    float* exchange = reinterpret_cast<float*>(tiles + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES);
+    bf16* staging = reinterpret_cast<bf16*>(exchange + 64 * (PAIR_CW + 1));
+    __shared__ unsigned long long full_bar[PAIR_STAGES], empty_bar[PAIR_STAGES], ready_bar[2], drained_bar[2];
+    __shared__ unsigned tmem_base_slot;
+    __shared__ int gave_up;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    volatile int* abort_flag = &gave_up;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < PAIR_STAGES; ++s) {
+            mbarrier_init(&full_bar[s], 1);
+            mbarrier_init(&empty_bar[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbarrier_init(&ready_bar[b], 1);
+            mbarrier_init(&drained_bar[b], 8);     // the epilogue warps of both blocks (the first one's barrier)
+        }
+        gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
+                     "r"(2 * PAIR_COLUMNS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_barrier();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned tmem_base = tmem_base_slot;
+
+    // Tiles in columns of eight token tiles, as above.
+    const int tall = (int)(p.tiles / p.token_tiles);
+    auto locate = [&](int tile, int& t0, int& f0) {
+        const int column = tile / (8 * tall), within = tile - column * 8 * tall, wide = min(8, p.token_tiles - column * 8);
+        t0 = (column * 8 + within % wide) * p.columns;
+        f0 = (within / wide * 2 + rank) * SPAN;
+    };
+    const int half = p.columns / 2;
+    bool ok = true;                                        // (the same in all lanes)
+    if (warp == 0) {
+        // ------------------------------------------------------------ producer: this block's features, its half of the tokens
+        int issued = 0;
+        for (int tile = pair; tile < p.tiles && ok; tile += pairs) {
+            int t0, f0;
+            locate(tile, t0, f0);
+            for (int kb = 0; kb < p.k_blocks; ++kb, ++issued) {
+                const int s = issued % PAIR_STAGES, k = kb * BK;
+                if (issued >= PAIR_STAGES) ok = mbarrier_wait_warp(&empty_bar[s], ((issued / PAIR_STAGES) - 1) & 1, abort_flag);
+                if (!ok) {
+                    if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.error, 1); }
+                    break;
+                }
+                if (elect_one()) {
+                    unsigned char* stage = tiles + (size_t)s * PAIR_STAGE_BYTES;
+                    if (rank == 0) mbarrier_expect_tx(&full_bar[s], 2 * (A_BYTES + half * BK * 2));
+                    if (GATED) {
+                        tma_load_pair(stage, &map_w, &full_bar[s], k, f0);
+                        tma_load_pair(stage + A_BYTES / 2, &map_w, &full_bar[s], k, p.features + f0);
+                    } else {
+                        tma_load_pair(stage, &map_w, &full_bar[s], k, f0);
+                    }
+                    tma_load_pair(stage + A_BYTES, &map_x, &full_bar[s], k, t0 + rank * half);
+                }
+                __syncwarp();
+            }
+        }
+        for (int i = max(0, issued - PAIR_STAGES); i < issued && ok; ++i)   // (what arrives here from the other block has arrived)
+            ok = mbarrier_wait_warp(&empty_bar[i % PAIR_STAGES], (i / PAIR_STAGES) & 1, abort_flag);
+        if (!ok && rank == 0)                              // copies in flight land before the blocks leave
+            for (int i = max(0, issued - PAIR_STAGES); i < issued; ++i)
+                for (unsigned spin = 0; spin < SPIN_LIMIT; ++spin)
+                    if (mbarrier_try_wait(&full_bar[i % PAIR_STAGES], (i / PAIR_STAGES) & 1)) break;
+    } else if (warp == 1) {
+        // -------------------------------------------------------------- issuer: the first block's, for both
+        const unsigned memory = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const unsigned idesc = make_instr_desc(p.columns) + ((unsigned)(BM >> 4) << 24);           // M = 256
+        int consumed = 0, done = 0;
+        for (int tile = pair; rank == 0 && tile < p.tiles && ok; tile += pairs, ++done) {
+            const int buffer = done & 1;
+            if (done >= 2) ok = mbarrier_wait_warp(&drained_bar[buffer], ((done >> 1) - 1) & 1, abort_flag);
+            if (!ok) {
+                if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.error, 4); }
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const unsigned accumulator = memory + buffer * PAIR_COLUMNS;
+            for (int kb = 0; kb < p.k_blocks; ++kb, ++consumed) {
+                const int s = consumed % PAIR_STAGES;
+                ok = mbarrier_wait_warp(&full_bar[s], (consumed / PAIR_STAGES) & 1, abort_flag);
+                if (!ok) {
+                    if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.error, 2); }
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const unsigned char* stage = tiles + (size_t)s * PAIR_STAGE_BYTES;
+                const unsigned long long desc_a = make_smem_desc(stage), desc_b = make_smem_desc(stage + A_BYTES);
+                if (elect_one()) {
+                    if (kb == 0) umma_pair<false>(accumulator, desc_a, desc_b, idesc);
+                    else umma_pair<true>(accumulator, desc_a, desc_b, idesc);
+#pragma unroll
+                    for (int k = 1; k < BK / UMMA_K; ++k) umma_pair<true>(accumulator, desc_a + 2 * k, desc_b + 2 * k, idesc);
+                    umma_commit_pair(&empty_bar[s]);
+                    if (kb == p.k_blocks - 1) umma_commit_pair(&ready_bar[buffer]);
+                }
+                __syncwarp();
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ epilogue: this block's features, all tokens
+        const int quarter = warp & 3, row = quarter * 32 + lane;
+        unsigned drained[2];
+        for (int b = 0; b < 2; ++b)
+            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(drained[b]) : "r"(smem_u32(&drained_bar[b])));
+        int done = 0, staged_chunks = 0;
+        for (int tile = pair; tile < p.tiles; tile += pairs, ++done) {
+            int t0, f0;
+            locate(tile, t0, f0);
+            const int buffer = done & 1;
+            const unsigned accumulator = tmem_base + buffer * PAIR_COLUMNS + ((unsigned)(quarter * 32) << 16);
+            ok = ok && mbarrier_wait_warp(&ready_bar[buffer], (done >> 1) & 1, abort_flag);
+            if (!ok && lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.error, 3); }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // (all four warps take part, whatever they found: they meet at barriers)
+            if (f0 < p.features) store_tile<GATED, PAIR_CW, TY>(p, map_y, accumulator, f0, t0, p.columns, ok, row, exchange, staging, staged_chunks);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(drained[buffer]) : "memory");
+        }
+        if (threadIdx.x == 64) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_barrier();                                     // neither leaves while the other may still reach its memory
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * PAIR_COLUMNS));
 }
 
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -807,6 +1001,38 @@ int by_tokens(int bn, const CUtensorMap& map_w, const CUtensorMap& map_x, const 
     }
     return KIDI_REFUSED_SIZE;
 }
+
+// Tokens from which on two SMs take a tile.
+constexpr int PAIR_TOKENS = 1024;
+
+// The height of those tiles: the least rounds times steps. A step of 64 k took 0.388 us at 256 tokens, 0.355 at 224, 0.310 at 192,
+// 0.275 at 160, 0.239 at 128 (2,048 rows of 24,576 x 4,096, under the power cap): as much as 78 tokens for the weights, and the
+// tokens. 1,500 rows of 4,096 x 12,288: six tiles of 256 tokens 173 us, eight of 192 133, two rounds either way.
+int pair_columns(int tokens, int features, int span) {
+    const int pairs = sm_count_of_current_device() / 2, tall = (features + 2 * span - 1) / (2 * span);
+    int best = PAIR_COLUMNS;
+    long long best_cost = 0;
+    for (int columns = PAIR_COLUMNS; columns >= 96; columns -= 32) {
+        const long long rounds = ((long long)tall * ((tokens + columns - 1) / columns) + pairs - 1) / pairs;
+        if (columns == PAIR_COLUMNS || rounds * (columns + 78) < best_cost) {
+            best = columns;
+            best_cost = rounds * (columns + 78);
+        }
+    }
+    return best;
+}
+
+template <bool GATED, typename TY>
+int launch_pairs(const CUtensorMap& map_w, const CUtensorMap& map_x, const CUtensorMap& map_y, const Params& p, cudaStream_t stream) {
+    constexpr size_t shared = pair_shared_bytes();
+    static_assert(shared <= 226 * 1024, "the stages fit an SM's shared memory");
+    auto kernel = gemm_tcgen05_pairs_kernel<GATED, TY>;
+    static std::atomic<unsigned long long> allowed{0};
+    const cudaError_t status = kidi_allow_shared(kernel, shared, allowed);
+    if (status != cudaSuccess) return (int)status;
+    const long long most = sm_count_of_current_device() / 2, pairs = p.tiles < most ? p.tiles : most;
+    return kidi_launch_clusters(kernel, dim3((unsigned)(2 * pairs)), dim3(THREADS), shared, stream, 2, map_w, map_x, map_y, p);
+}
 }  // namespace
 
 // The token tile that fits `tokens` rows.
@@ -912,16 +1138,27 @@ KIDI_API int kidi_gemm_tcgen05(const void* x, const void* w, void* y, int y_dtyp
     const long long tail = (tiles - p.tail_first) * p.k_blocks;   // dealt out in k-blocks
     p.share = (int)(tail / blocks);
     p.extra = (int)(tail % blocks);
+    p.columns = pair_columns(tokens, features, span);
+    // (One round of the widest tiles either way: a block a tile begins 1.2 us sooner, 18.9 against 20.1 us for 2,048 rows of
+    // 2,048 x 2,048. Shared tiles are slower than pairs.)
+    const bool one_round = p.columns == PAIR_COLUMNS && blocks == tiles && 2 * tiles > sm_count_of_current_device();
+    const bool paired = tokens >= PAIR_TOKENS && splits == 0 && !one_round;
+    if (paired) {
+        p.token_tiles = (tokens + p.columns - 1) / p.columns;
+        p.tiles = (long long)((features + 2 * span - 1) / (2 * span)) * p.token_tiles;
+        if (p.tiles > 0x7fffffffLL) return KIDI_REFUSED_SIZE;
+    }
     if (!workspace || !counters || !error) return KIDI_REFUSED_SIZE;
     CUtensorMap map_w, map_x;
     int status = make_map(&map_w, w, gated ? 2LL * features : features, K, ldw, gated ? 64 : BM);
     if (status) return status;
-    status = make_map(&map_x, x, tokens, K, ldx, bn);
+    status = make_map(&map_x, x, tokens, K, ldx, paired ? p.columns / 2 : bn);
     if (status) return status;
-    // bfloat16 results whose rows 16-byte copies can write leave through shared memory and TMA stores.
+    // bfloat16 results whose rows 16-byte copies can write, to the last, leave through shared memory and TMA stores (which write
+    // whole 16 bytes: what stands behind a row of a wider matrix would not stay).
     CUtensorMap map_y;
     memset(&map_y, 0, sizeof(map_y));
-    p.staged = y_dtype == KIDI_BF16 && !(ldy & 7) && !((uintptr_t)y & 15);
+    p.staged = y_dtype == KIDI_BF16 && !(ldy & 7) && !(features & 7) && !((uintptr_t)y & 15);
     if (p.staged) {
         status = make_store_map(&map_y, y, tokens, features, ldy, span);
         if (status) return status;
@@ -929,8 +1166,11 @@ KIDI_API int kidi_gemm_tcgen05(const void* x, const void* w, void* y, int y_dtyp
     if (gated) {
         if (y_dtype != KIDI_BF16) return KIDI_REFUSED_DTYPE;
         if (bias) return KIDI_REFUSED_SIZE;
+        if (paired) return launch_pairs<true, bf16>(map_w, map_x, map_y, p, stream);
         return by_tokens<true, bf16>(bn, map_w, map_x, map_y, p, blocks, stream);
     }
+    if (paired && y_dtype == KIDI_BF16) return launch_pairs<false, bf16>(map_w, map_x, map_y, p, stream);
+    if (paired && y_dtype == KIDI_F32) return launch_pairs<false, float>(map_w, map_x, map_y, p, stream);
     if (y_dtype == KIDI_BF16) return by_tokens<false, bf16>(bn, map_w, map_x, map_y, p, blocks, stream);
     if (y_dtype == KIDI_F32) return by_tokens<false, float>(bn, map_w, map_x, map_y, p, blocks, stream);
     return KIDI_REFUSED_DTYPE;

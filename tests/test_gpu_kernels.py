@@ -258,6 +258,30 @@ def test_gemm_tcgen05(rows, shape, splits):
     assert tcgen05.error_code(torch.device(DEVICE)) == 0
 
 
+# Two SMs on a tile: heights of 96 to 256 tokens, odd numbers of 128 features (the last pair's second half is empty), ragged edges
+# in all dimensions, several rounds, results in 32 bits and in rows that copies can't write.
+@pytest.mark.parametrize("rows", [1024, 1025, 1500, 1801, 3000])
+@pytest.mark.parametrize("shape", [(389, 96), (100, 200), (4096, 1024), (130, 4104), (2176, 64), (9000, 128)])
+def test_gemm_tcgen05_by_pairs_of_blocks(rows, shape):
+    from kidi_b200.kernels import tcgen05
+    N, K = shape
+    generator = torch.Generator(device=DEVICE).manual_seed(rows + N)
+    x = torch.randn(rows, K, generator=generator, device=DEVICE).to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=generator, device=DEVICE) / math.sqrt(K) * 2).to(torch.bfloat16)
+    bias = torch.randn(N, generator=generator, device=DEVICE)
+    for out_dtype in (torch.float32, torch.bfloat16):
+        alone = torch.cat([tcgen05.gemm(part, w, out_dtype, splits=1, bias=bias) for part in x.split(1000)])
+        out = torch.full((rows, N + 3), 7.0, dtype=out_dtype, device=DEVICE)
+        tcgen05.gemm(x, w, out_dtype, out=out[:, :N], bias=bias)          # (a block a tile adds in the same order)
+        assert torch.equal(out[:, :N], alone) and bool((out[:, N:] == 7).all())
+        assert torch.equal(tcgen05.gemm(x, w, out_dtype, bias=bias), alone)
+    close(tcgen05.gemm(x, w, torch.float32), x.double() @ w.double().T, 2e-5, f"{rows}x{N}x{K}")
+    if N % 2 == 0:
+        alone = torch.cat([tcgen05.gemm_silu_gate(part, w, splits=1) for part in x.split(1000)])
+        assert torch.equal(tcgen05.gemm_silu_gate(x, w), alone)
+    assert tcgen05.error_code(torch.device(DEVICE)) == 0
+
+
 @pytest.mark.parametrize("rows", [1, 17, 64, 150])
 @pytest.mark.parametrize("splits", [1, 2])
 def test_gemm_tcgen05_silu_gate(rows, splits):
