@@ -11,14 +11,17 @@
 //  * tiles: prompts. A block takes 64 consecutive rows of a sequence for one head. Both products are register tiles of 8 x 4
 //    and 8 x 8 (8 x 4 for values of up to 64), operands by k in shared memory; keys are transposed on the way in, 16
 //    dimensions at a time, values are copied as they lie while the scores are computed. Bound by what two warps a scheduler
-//    leave idle (two blocks of four warps an SM: 250 registers a thread for two sets of sums): 42% of issue slots are used,
-//    and the longest waits are for instructions, of which an unrolled tile is long. 32 heads of 128 over 8, a prompt of 700
-//    tokens 359 us (23 TFLOP/s), of 2,000 1,718 (attention_generic.cu, a warp a row, head and key: 5,800 for 2,000).
+//    can issue (two blocks of four warps an SM: 250 registers a thread for two sets of sums): 61% of issue slots are used. Loops
+//    are unrolled only as far as the instruction caches hold them (8 KB a scheduler: behind that every instruction waits), and
+//    what a tile needs besides the two products is done element by element. Rows' blocks are started longest first over all
+//    heads. 32 heads of 128 over 8, a prompt of 700 tokens 258 us (371 with everything unrolled), of 2,000 1,202 (1,775;
+//    attention_generic.cu, a warp a row, head and key: 5,800).
 //  * rows: decoding, and steps of a few tokens a sequence. A block takes one row, up to eight heads that share a key head,
 //    and every n-th segment, and leaves its sums in a workspace, which a second kernel merges (with one block a row the block
 //    merges them itself). The grid does not depend on how long the sequences are, so a captured step serves all
-//    lengths. Bound by the stream of keys and values, 64 KB a tile and block, three blocks an SM: 8 sequences of 1,030 tokens
-//    43 us (attention_generic.cu: 455), of 4,000 110 (2.4 TB/s).
+//    lengths. Bound by the instructions of a tile (half of the issue slots are used) and by a segment's four tiles one behind
+//    the other, three blocks an SM. Eight warps a block: 8 sequences of 1,030 tokens 42 us (four warps 48,
+//    attention_generic.cu 455), of 4,000 93 (116), one of 1,030 30 (38).
 #include <type_traits>
 
 #include "attention_args.cuh"
@@ -112,9 +115,10 @@ __device__ __forceinline__ void key_at(const AttentionArgs& a, int u, int start,
 
 // ------------------------------------------------------------------------------------------------------------------ rows
 constexpr int GROUP = 8;         // heads of a block
+constexpr int ROWS_THREADS = 256, KEY_TEAMS = ROWS_THREADS / TILE, VALUE_TEAMS = ROWS_THREADS / MOST_WIDE;
 constexpr int KEY_PAD = 4;       // floats between the keys of a tile: eight keys' 16-byte pieces meet no bank twice
 
-__global__ void __launch_bounds__(THREADS) attention_f32_rows_kernel(AttentionF32Args args) {
+__global__ void __launch_bounds__(ROWS_THREADS) attention_f32_rows_kernel(AttentionF32Args args) {
     const AttentionArgs& a = args.a;
     extern __shared__ __align__(16) float shared[];
     __shared__ const float* keys_at[TILE];
@@ -129,18 +133,22 @@ __global__ void __launch_bounds__(THREADS) attention_f32_rows_kernel(AttentionF3
     const int seq = a.row_seq[row];
     if (seq < 0) {
         if (!args.parts)
-            for (int i = t; i < heads * vd; i += THREADS) ((float*)a.out)[row * a.ldo + (long long)head0 * vd + i] = 0.f;
+            for (int i = t; i < heads * vd; i += ROWS_THREADS) ((float*)a.out)[row * a.ldo + (long long)head0 * vd + i] = 0.f;
         return;
     }
     const int position = a.row_pos[row], first = first_visible(position, a.window, a.chunk);
     const int first_segment = first / SEGMENT, last_segment = position / SEGMENT;
     if (first_segment + (int)blockIdx.z > last_segment) return;
     const int slot = a.seq_slot[seq], start = a.k_step ? a.seq_start[seq] : 0x7fffffff, row0 = a.seq_row0[seq];
-    for (int i = t; i < heads * d; i += THREADS) query[i / d][i % d] = ((const float*)a.q)[row * a.ldq + (long long)head0 * d + i];
-    float acc[GROUP], total[GROUP];
-    Merged merged[GROUP];
+    for (int i = t; i < heads * d; i += ROWS_THREADS) query[i / d][i % d] = ((const float*)a.q)[row * a.ldq + (long long)head0 * d + i];
+    static_assert(GROUP == 2 * KEY_TEAMS, "a thread's heads of a key");
+    // A thread's share of the weighted sums: a column of every VALUE_TEAMS-th head.
+    constexpr int MINE = GROUP / VALUE_TEAMS;
+    const int column = t % MOST_WIDE, team = t / MOST_WIDE;
+    float acc[MINE], total[MINE];
+    Merged merged[MINE];
 #pragma unroll
-    for (int h = 0; h < GROUP; ++h) total[h] = 0.f;
+    for (int i = 0; i < MINE; ++i) total[i] = 0.f;
 
     int low = 0, high = 0;                            // the keys of the segment that the row sees
     auto locate = [&](int tile) {
@@ -152,11 +160,19 @@ __global__ void __launch_bounds__(THREADS) attention_f32_rows_kernel(AttentionF3
             values_at[t] = value;
         }
     };
+    // (A thread's pieces: from one to the next ROWS_THREADS pieces on, `down` keys and `across` pieces.)
     auto copy = [&](const float* const* from, float* to, int width, int stride) {
-        const int pieces = width / 4;
-        for (int i = t; i < TILE * pieces; i += THREADS) {
-            const int key = i / pieces, c = (i - key * pieces) * 4;
-            copy16(to + key * stride + c, from[key] ? from[key] + c : nullptr, (const float*)a.q);
+        const int pieces = width / 4, down = ROWS_THREADS / pieces, across = ROWS_THREADS - down * pieces;
+        int key = t / pieces, c = t - key * pieces;
+#pragma unroll 2
+        while (key < TILE) {
+            copy16(to + key * stride + 4 * c, from[key] ? from[key] + 4 * c : nullptr, (const float*)a.q);
+            key += down;
+            c += across;
+            if (c >= pieces) {
+                c -= pieces;
+                ++key;
+            }
         }
         commit_copies();
     };
@@ -169,7 +185,7 @@ __global__ void __launch_bounds__(THREADS) attention_f32_rows_kernel(AttentionF3
             sum[t] = 0.f;
         }
 #pragma unroll
-        for (int h = 0; h < GROUP; ++h) acc[h] = 0.f;
+        for (int i = 0; i < MINE; ++i) acc[i] = 0.f;
         const int last = high / TILE;
         locate(low / TILE);
         __syncthreads();
@@ -180,26 +196,28 @@ __global__ void __launch_bounds__(THREADS) attention_f32_rows_kernel(AttentionF3
             __syncthreads();                              // the keys are there (and the query)
             {
                 const int key = t % TILE, u = tile * TILE + key;
-                float dots[GROUP / 2];
+                float dots[GROUP / KEY_TEAMS];
 #pragma unroll
-                for (int i = 0; i < GROUP / 2; ++i) dots[i] = 0.f;
-                for (int k = 0; k < d; k += 4) {
-                    const float4 b = *reinterpret_cast<const float4*>(keys + key * pitch + k);
+                for (int i = 0; i < GROUP / KEY_TEAMS; ++i) dots[i] = 0.f;
+                auto multiply = [&](auto count) {
+#pragma unroll 4
+                    for (int k = 0; k < d; k += 4) {
+                        const float4 b = *reinterpret_cast<const float4*>(keys + key * pitch + k);
 #pragma unroll
-                    for (int i = 0; i < GROUP / 2; ++i) {
-                        const int h = t / TILE + 2 * i;
-                        if (h < heads) {
-                            const float4 q = *reinterpret_cast<const float4*>(&query[h][k]);
+                        for (int i = 0; i < decltype(count)::value; ++i) {
+                            const float4 q = *reinterpret_cast<const float4*>(&query[t / TILE + KEY_TEAMS * i][k]);
                             dots[i] = fmaf(q.x, b.x, dots[i]);
                             dots[i] = fmaf(q.y, b.y, dots[i]);
                             dots[i] = fmaf(q.z, b.z, dots[i]);
                             dots[i] = fmaf(q.w, b.w, dots[i]);
                         }
                     }
-                }
+                };
+                if (t / TILE + KEY_TEAMS < heads) multiply(std::integral_constant<int, 2>());
+                else if (t / TILE < heads) multiply(std::integral_constant<int, 1>());
 #pragma unroll
-                for (int i = 0; i < GROUP / 2; ++i) {
-                    const int h = t / TILE + 2 * i;
+                for (int i = 0; i < GROUP / KEY_TEAMS; ++i) {
+                    const int h = t / TILE + KEY_TEAMS * i;
                     if (h < heads) scores[h][key] = u >= low && u <= high ? score_of(a, dots[i], head0 + h, position, u) : -INFINITY;
                 }
             }
@@ -225,7 +243,7 @@ __global__ void __launch_bounds__(THREADS) attention_f32_rows_kernel(AttentionF3
                 }
             }
             __syncthreads();
-            for (int i = t; i < heads * TILE; i += THREADS)
+            for (int i = t; i < heads * TILE; i += ROWS_THREADS)
                 scores[i / TILE][i % TILE] = weight_of(a, scores[i / TILE][i % TILE], head0 + i / TILE, top[i / TILE]);
             wait_copies<1>();
             __syncthreads();                              // the weights and the values are there
@@ -238,55 +256,66 @@ __global__ void __launch_bounds__(THREADS) attention_f32_rows_kernel(AttentionF3
                 part = __fadd_rn(part, __shfl_xor_sync(0xffffffffu, part, 2));
                 if ((t & 3) == 0 && t >> 2 < heads) sum[h] = __fmaf_rn(sum[h], scale[h], part);
             }
-            if (t < vd) {
+            if (column < vd) {
 #pragma unroll
-                for (int h = 0; h < GROUP; ++h)
-                    if (h < heads) acc[h] = __fmul_rn(acc[h], scale[h]);
+                for (int i = 0; i < MINE; ++i)
+                    if (team + VALUE_TEAMS * i < heads) acc[i] = __fmul_rn(acc[i], scale[team + VALUE_TEAMS * i]);
                 // (keys outside the row's reach have zero weights and zero values)
+#pragma unroll 4
                 for (int key = 0; key < TILE; key += 4) {
-                    const float v[4] = {values[key * vd + t], values[(key + 1) * vd + t], values[(key + 2) * vd + t], values[(key + 3) * vd + t]};
+                    const float* from = values + key * vd + column;
+                    const float v[4] = {from[0], from[vd], from[2 * vd], from[3 * vd]};
 #pragma unroll
-                    for (int h = 0; h < GROUP; ++h)
-                        if (h < heads) {
-                            const float4 p = *reinterpret_cast<const float4*>(&scores[h][key]);
-                            acc[h] = fmaf(p.x, v[0], acc[h]);
-                            acc[h] = fmaf(p.y, v[1], acc[h]);
-                            acc[h] = fmaf(p.z, v[2], acc[h]);
-                            acc[h] = fmaf(p.w, v[3], acc[h]);
+                    for (int i = 0; i < MINE; ++i)
+                        if (team + VALUE_TEAMS * i < heads) {
+                            const float4 p = *reinterpret_cast<const float4*>(&scores[team + VALUE_TEAMS * i][key]);
+                            acc[i] = fmaf(p.x, v[0], acc[i]);
+                            acc[i] = fmaf(p.y, v[1], acc[i]);
+                            acc[i] = fmaf(p.z, v[2], acc[i]);
+                            acc[i] = fmaf(p.w, v[3], acc[i]);
                         }
                 }
             }
             __syncthreads();                              // weights, values and statistics are free again
         }
         if (args.parts) {
-            float* part = args.parts + (((long long)row * a.heads + head0) * args.segments + segment - first_segment) * (vd + 2);
+            float* part = args.parts + (((long long)row * a.heads + head0 + team) * args.segments + segment - first_segment) * (vd + 2);
 #pragma unroll
-            for (int h = 0; h < GROUP; ++h, part += (long long)args.segments * (vd + 2))
+            for (int i = 0; i < MINE; ++i, part += (long long)VALUE_TEAMS * args.segments * (vd + 2)) {
+                const int h = team + VALUE_TEAMS * i;
                 if (h < heads) {
-                    if (t < vd) part[t] = acc[h];
-                    if (t == 0) {
+                    if (column < vd) part[column] = acc[i];
+                    if (column == 0) {
                         part[vd] = top[h];
                         part[vd + 1] = sum[h];
                     }
                 }
+            }
         } else {
 #pragma unroll
-            for (int h = 0; h < GROUP; ++h)
+            for (int i = 0; i < MINE; ++i) {
+                const int h = team + VALUE_TEAMS * i;
                 if (h < heads) {
-                    merged[h].add(top[h], sum[h]);
-                    total[h] = merge(total[h], acc[h], merged[h].old, merged[h].fresh);
+                    merged[i].add(top[h], sum[h]);
+                    total[i] = merge(total[i], acc[i], merged[i].old, merged[i].fresh);
                 }
+            }
         }
         __syncthreads();                                  // the statistics are free again
     }
-    if (!args.parts && t < vd)
-#pragma unroll
-        for (int h = 0; h < GROUP; ++h)
+    if (!args.parts && column < vd)
+#pragma unroll 1
+        for (int i = 0; i < MINE; ++i) {
+            const int h = team + VALUE_TEAMS * i;
             if (h < heads) {
-                float factor, divisor;
-                closing(a, head0 + h, merged[h].top, merged[h].sum, factor, divisor);
-                put(a, row, head0 + h, vd, t, total[h], factor, divisor);
+                float factor, divisor, value = total[0], top_of = merged[0].top, sum_of = merged[0].sum;
+#pragma unroll
+                for (int j = 1; j < MINE; ++j)
+                    if (i == j) { value = total[j]; top_of = merged[j].top; sum_of = merged[j].sum; }
+                closing(a, head0 + h, top_of, sum_of, factor, divisor);
+                put(a, row, head0 + h, vd, column, value, factor, divisor);
             }
+        }
 }
 
 __global__ void __launch_bounds__(THREADS) attention_f32_merge_kernel(AttentionF32Args args) {
@@ -321,6 +350,10 @@ __device__ __forceinline__ int moved(int k) { return (k >> 2 & 3) * 8; }
 // Weights by key: four neighbouring rows stand in group (row / 4) ^ (key / 4 % 8).
 __device__ __forceinline__ int weight_place(int key, int row) { return key * TILE + ((row >> 2 ^ (key >> 2 & 7)) << 2 | (row & 3)); }
 
+// What stands in the place of a key's score that a row does not see: a NaN of this kernel's own (a maximum leaves it out), whose
+// weight is -0. That adds nothing to a sum, and no weight of a key that is seen is -0.
+constexpr unsigned UNSEEN = 0xffc0deadu;
+
 // TN: values of a thread (the value heads are at most 16 TN wide).
 template <int TN>
 __global__ void __launch_bounds__(THREADS, 2) attention_f32_tiles_kernel(AttentionF32Args args) {
@@ -329,6 +362,7 @@ __global__ void __launch_bounds__(THREADS, 2) attention_f32_tiles_kernel(Attenti
     __shared__ const float* keys_at[2][TILE];
     __shared__ const float* values_at[2][TILE];
     __shared__ float exchange[2][TILE], scale[TILE], old_factor[TILE], new_factor[TILE];
+    __shared__ int low_of[TILE];                              // the first key that a row sees
     constexpr int COLUMNS = 16 * TN;
     const int d = a.head_dim, vd = a.value_dim ? a.value_dim : d, stages = (d + DEPTH - 1) / DEPTH;
     float* query = shared;                                    // [stages * DEPTH][TILE]
@@ -336,8 +370,8 @@ __global__ void __launch_bounds__(THREADS, 2) attention_f32_tiles_kernel(Attenti
     float* values = stage + 2 * DEPTH * TILE;                 // [TILE][COLUMNS]
     float* weights = values + TILE * COLUMNS;                 // [key][row]: scores, then weights
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const int seq = blockIdx.z, head = blockIdx.y, kv_head = head / (a.heads / a.kv_heads);
-    const int length = args.seq_len[seq], tile0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * TILE;      // longest walks first
+    const int seq = blockIdx.z, head = blockIdx.x, kv_head = head / (a.heads / a.kv_heads);
+    const int length = args.seq_len[seq], tile0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * TILE;      // longest walks first
     if (tile0 >= length) return;
     const int row0 = a.seq_row0[seq], sequence_start = a.seq_start[seq], slot = a.seq_slot[seq];
     const int start = a.k_step ? sequence_start : 0x7fffffff;
@@ -349,6 +383,8 @@ __global__ void __launch_bounds__(THREADS, 2) attention_f32_tiles_kernel(Attenti
     }
     const int low = first_visible(position0, a.window, a.chunk), high = position0 + count - 1;
 
+    if (t < TILE) low_of[t] = t < count ? first_visible(position0 + t, a.window, a.chunk) : 0x7fffffff;
+    const bool plain = !(a.softcap > 0.f) && !a.slopes && !a.distance_bias;       // scores are products times a number
     const int piece_k = t % 4 * 4, piece_row = t / 4;         // (of a stage: two rows, 32 apart)
     for (int s = 0; s < stages; ++s)
 #pragma unroll
@@ -422,32 +458,46 @@ __global__ void __launch_bounds__(THREADS, 2) attention_f32_tiles_kernel(Attenti
             else if (tile < last_tile) locate(tile + 1);
             __syncthreads();
             const float* rows = query + st * DEPTH * TILE;
+#pragma unroll 1
+            for (int k4 = 0; k4 < DEPTH; k4 += 4) {           // (unrolled in full, 9 KB of instructions would not fit their cache)
+                const float* q_at = rows + k4 * TILE + (first_row ^ moved(k4));
+                const float* b_at = current + k4 * TILE + (first_key ^ moved(k4));
+                const int other = (first_row ^ moved(k4) ^ 16) - (first_row ^ moved(k4));
 #pragma unroll
-            for (int k = 0; k < DEPTH; ++k) {
-                float q[8], b[4];
-                *reinterpret_cast<float4*>(q) = *reinterpret_cast<const float4*>(rows + k * TILE + (first_row ^ moved(k)));
-                *reinterpret_cast<float4*>(q + 4) = *reinterpret_cast<const float4*>(rows + k * TILE + (first_row ^ moved(k) ^ 16));
-                *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(current + k * TILE + (first_key ^ moved(k)));
+                for (int k = 0; k < 4; ++k) {
+                    float q[8], b[4];
+                    *reinterpret_cast<float4*>(q) = *reinterpret_cast<const float4*>(q_at + k * TILE);
+                    *reinterpret_cast<float4*>(q + 4) = *reinterpret_cast<const float4*>(q_at + k * TILE + other);
+                    *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(b_at + k * TILE);
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < 4; ++j)
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) s[i][j] = fmaf(q[i], b[j], s[i][j]);
+                        for (int i = 0; i < 8; ++i) s[i][j] = fmaf(q[i], b[j], s[i][j]);
+                }
             }
         }
+        // A tile whose keys not every row sees: a key that a row does not see is left out of its sum (its value may be anything).
+        const bool whole = tile * TILE + TILE - 1 <= position0 && tile * TILE >= first_visible(high, a.window, a.chunk) && count == TILE;
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const int u = tile * TILE + first_key + j;
                 float four[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int r = first_row + 16 * h + i, position = position0 + r;
-                    const bool seen = r < count && u <= position && u >= first_visible(position, a.window, a.chunk);
-                    four[i] = seen ? score_of(a, s[4 * h + i][j], head, position, u) : -INFINITY;
-                }
+                for (int i = 0; i < 4; ++i) four[i] = plain ? __fmul_rn(s[4 * h + i][j], a.scale) : s[4 * h + i][j];
                 *reinterpret_cast<float4*>(weights + weight_place(first_key + j, first_row + 16 * h)) = make_float4(four[0], four[1], four[2], four[3]);
             }
+        // What is left to do to a thread's scores, one by one: such loops unrolled would push the products out of the instruction
+        // caches.
+        if (!plain || !whole) {
+#pragma unroll 1
+            for (int e = 0; e < 32; ++e) {
+                const int r = first_row + (e & 16) + (e & 3), key = first_key + (e >> 2 & 3), u = tile * TILE + key, position = position0 + r;
+                float* place = weights + weight_place(key, r);
+                if (u > position || u < low_of[r]) *place = __uint_as_float(UNSEEN);
+                else if (!plain) *place = score_of(a, *place, head, position, u);
+            }
+        }
         __syncthreads();
         float highest = -INFINITY;
 #pragma unroll 8
@@ -461,14 +511,25 @@ __global__ void __launch_bounds__(THREADS, 2) attention_f32_tiles_kernel(Attenti
         if (!half) scale[own_row] = factor;
         float parts[2] = {0.f, 0.f};
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll 8
-            for (int key = 0; key < 16; ++key) {
-                float* place = weights + weight_place(half * 32 + j * 16 + key, own_row);
-                const float weight = weight_of(a, *place, head, top);
-                *place = weight;
-                parts[j] = __fadd_rn(parts[j], weight);
+        for (int j = 0; j < 2; ++j) {
+            if (a.weight_bias) {
+#pragma unroll 1
+                for (int key = 0; key < 16; ++key) {
+                    float* place = weights + weight_place(half * 32 + j * 16 + key, own_row);
+                    const float score = *place;
+                    *place = __float_as_uint(score) == UNSEEN ? -0.f : weight_of(a, score, head, top);
+                }
+            } else {
+#pragma unroll 4
+                for (int key = 0; key < 16; ++key) {
+                    float* place = weights + weight_place(half * 32 + j * 16 + key, own_row);
+                    const float score = *place;
+                    *place = __float_as_uint(score) == UNSEEN ? -0.f : score == -INFINITY ? 0.f : expf(__fsub_rn(score, top));
+                }
             }
+#pragma unroll 4
+            for (int key = 0; key < 16; ++key) parts[j] = __fadd_rn(parts[j], weights[weight_place(half * 32 + j * 16 + key, own_row)]);
+        }
         const float mine = __fadd_rn(parts[0], parts[1]);
         __syncthreads();                                      // (the maxima have been read)
         exchange[half][own_row] = mine;
@@ -482,8 +543,6 @@ __global__ void __launch_bounds__(THREADS, 2) attention_f32_tiles_kernel(Attenti
 #pragma unroll
             for (int j = 0; j < TN; ++j) acc[i][j] = __fmul_rn(acc[i][j], c);
         }
-        // A tile whose keys not every row sees: a key that a row does not see is left out of its sum (its value may be anything).
-        const bool whole = tile * TILE + TILE - 1 <= position0 && tile * TILE >= first_visible(high, a.window, a.chunk) && count == TILE;
         auto accumulate = [&](auto masked) {
 #pragma unroll 4
             for (int key = 0; key < TILE; ++key) {
@@ -494,10 +553,8 @@ __global__ void __launch_bounds__(THREADS, 2) attention_f32_tiles_kernel(Attenti
                 for (int g = 0; g < TN; g += 4) *reinterpret_cast<float4*>(v + g) = *reinterpret_cast<const float4*>(values + key * COLUMNS + first_value + 8 * g);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    if constexpr (decltype(masked)::value) {
-                        const int position = position0 + first_row + (i / 4) * 16 + i % 4, u = tile * TILE + key;
-                        if (u > position || u < first_visible(position, a.window, a.chunk)) continue;
-                    }
+                    if constexpr (decltype(masked)::value)
+                        if (__float_as_int(p[i]) < 0) continue;          // (-0)
 #pragma unroll
                     for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(p[i], v[j], acc[i][j]);
                 }
@@ -528,16 +585,19 @@ __global__ void __launch_bounds__(THREADS, 2) attention_f32_tiles_kernel(Attenti
         __syncthreads();                                      // weights and values are free again
     }
     if (!half) closing(a, head, merged.top, merged.sum, old_factor[own_row], new_factor[own_row]);
-    __syncthreads();
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int r = first_row + (i / 4) * 16 + i % 4;
-        if (r >= count) continue;
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int c = first_value + (j / 4) * 32 + j % 4;
-            if (c < vd) put(a, row0 + tile0 + r, head, vd, c, total[i][j], old_factor[r], new_factor[r]);
-        }
+        for (int j = 0; j < TN; j += 4)
+            *reinterpret_cast<float4*>(values + r * COLUMNS + first_value + 8 * j) =
+                make_float4(total[i][j], total[i][j + 1], total[i][j + 2], total[i][j + 3]);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int i = t; i < count * vd; i += THREADS) {
+        const int r = i / vd, c = i - r * vd;
+        put(a, row0 + tile0 + r, head, vd, c, values[r * COLUMNS + c], old_factor[r], new_factor[r]);
     }
 }
 
@@ -550,7 +610,7 @@ template <int TN> int launch_tiles(const AttentionF32Args& args, cudaStream_t st
     static std::atomic<unsigned long long> allowed{0};
     const cudaError_t status = kidi_allow_shared(kernel, needed(MOST_WIDE / DEPTH), allowed);
     if (status != cudaSuccess) return (int)status;
-    return kidi_launch(kernel, dim3((args.max_new + TILE - 1) / TILE, a.heads, args.seqs), dim3(THREADS), bytes, stream, args);
+    return kidi_launch(kernel, dim3(a.heads, (args.max_new + TILE - 1) / TILE, args.seqs), dim3(THREADS), bytes, stream, args);
 }
 }  // namespace
 
@@ -566,7 +626,7 @@ KIDI_API int kidi_attention_f32(const AttentionF32Args* arguments, int tiles, cu
         (a.distance_bias && (a.bias_last < 0 || a.bias_stride <= a.bias_last)) || args.seqs <= 0)
         return KIDI_REFUSED_SIZE;
     if (tiles) {
-        if (args.seqs > 65535 || args.max_new <= 0) return KIDI_REFUSED_SIZE;
+        if (args.seqs > 65535 || args.max_new <= 0 || args.max_new > 65535 * TILE) return KIDI_REFUSED_SIZE;
         return vd <= 64 ? launch_tiles<4>(args, stream) : launch_tiles<8>(args, stream);
     }
     const int group = a.heads / a.kv_heads, blocks = (group + GROUP - 1) / GROUP;
@@ -578,7 +638,7 @@ KIDI_API int kidi_attention_f32(const AttentionF32Args* arguments, int tiles, cu
     static std::atomic<unsigned long long> allowed{0};
     const cudaError_t status = kidi_allow_shared(attention_f32_rows_kernel, most, allowed);
     if (status != cudaSuccess) return (int)status;
-    const int code = kidi_launch(attention_f32_rows_kernel, dim3(a.rows, a.kv_heads * blocks, args.shares), dim3(THREADS), bytes, stream, args);
+    const int code = kidi_launch(attention_f32_rows_kernel, dim3(a.rows, a.kv_heads * blocks, args.shares), dim3(ROWS_THREADS), bytes, stream, args);
     if (code || !args.parts) return code;
     return kidi_launch(attention_f32_merge_kernel, dim3(a.rows, a.heads), dim3(THREADS), 0, stream, args);
 }
