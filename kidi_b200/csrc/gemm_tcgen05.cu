@@ -186,7 +186,16 @@ __device__ __forceinline__ void tmem_load(unsigned address, float (&v)[N]) {
 
 // Token columns that the epilogue takes at a time: its barriers and copies are paid for once a piece. (Small tiles have
 // two blocks an SM and no shared memory to spare.)
-template <int BN> constexpr int epilogue_columns() { return BN >= 128 ? 32 : 16; }
+// The gate's arithmetic is long: 32 columns of it, unrolled, do not fit the instruction caches (12 instead of 5 us a tile of 256).
+template <int BN, bool GATED> constexpr int epilogue_columns() { return BN >= 128 && !GATED ? 32 : 16; }
+// What the epilogue has of shared memory: the gated form's exchange (two buffers), then two buffers of results on their way out.
+template <bool GATED> constexpr size_t exchange_bytes() { return GATED ? 2 * 64 * (16 + 1) * sizeof(float) : 0; }
+template <int BN, bool GATED> __host__ __device__ constexpr size_t epilogue_bytes() {
+    return exchange_bytes<GATED>() + 2 * epilogue_columns<BN, GATED>() * (GATED ? 64 : BM) * sizeof(bf16);
+}
+template <int BN> __host__ __device__ constexpr size_t most_epilogue_bytes() {
+    return epilogue_bytes<BN, true>() > epilogue_bytes<BN, false>() ? epilogue_bytes<BN, true>() : epilogue_bytes<BN, false>();
+}
 
 struct Params {
     void* y;               // [tokens, ldy]
@@ -224,11 +233,10 @@ struct GroupPieces {
     unsigned char wanted[MOST_GROUP_TILES];   // of a tile in rows, then of a piece in steps of 16 tokens
 };
 
-// Shared memory of a block: the stages, the gated epilogue's exchange buffer and two buffers of results on their way out;
+// Shared memory of a block: the stages and the epilogue's buffers;
 // behind them (`pieces`, in the build for weights in groups) what a block knows of those.
 template <int BN, int STAGES> __host__ __device__ constexpr size_t shared_floor() {
-    constexpr int columns = epilogue_columns<BN>();
-    return (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 64 * (columns + 1) * sizeof(float) + 2 * columns * BM * sizeof(bf16);
+    return (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + most_epilogue_bytes<BN>();
 }
 
 // A tile's results from the accumulator to y, by 128 threads (threads 64 to 191 of the block; `row`: a thread's feature within the
@@ -238,6 +246,12 @@ __device__ __forceinline__ void store_tile(const Params& p, const CUtensorMap& m
                                            bool ok, int row, float* exchange, bf16* staging, int& staged_chunks) {
     constexpr int SPAN = GATED ? 64 : BM;
     TY* y = (TY*)p.y;
+    const bool staged = sizeof(TY) == 2 && p.staged;
+    // The thread's feature within the tile and its columns of a chunk (gated: half of them).
+    const int feature = GATED ? row & 63 : row;
+    const int first = GATED && row >= 64 ? CW / 2 : 0;
+    constexpr int COUNT = GATED ? CW / 2 : CW;
+    const bool mine = f0 + feature < p.features;
 #pragma unroll 1
     for (int c = 0; c < columns; c += CW) {
         float v[CW];
@@ -245,35 +259,32 @@ __device__ __forceinline__ void store_tile(const Params& p, const CUtensorMap& m
         else
 #pragma unroll
             for (int i = 0; i < CW; ++i) v[i] = 0.f;
-        // The thread's feature within the tile and its columns of the chunk (gated: half of them).
-        const int feature = GATED ? row & 63 : row;
-        const int first = GATED && row >= 64 ? CW / 2 : 0;
-        constexpr int COUNT = GATED ? CW / 2 : CW;
-        const bool mine = f0 + feature < p.features;
+        bf16* out = staging + (staged_chunks & 1) * (CW * SPAN);
+        // The copy that read this buffer two chunks ago must be through with it.
+        if (staged && threadIdx.x == 64 && staged_chunks >= 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
         if (GATED) {
             // Rows 64..127 hold the up projection of the features in rows 0..63. The two threads of a feature
             // share its columns: one takes the first half and gets their up values, the other takes the second
-            // half and gets their gates.
-            float* shared_row = exchange + feature * (CW + 1);
+            // half and gets their gates. (Two buffers in turn: one barrier a chunk is enough.)
+            float* shared_row = exchange + (staged_chunks & 1) * 64 * (CW + 1) + feature * (CW + 1);
 #pragma unroll
             for (int i = 0; i < CW / 2; ++i) shared_row[(CW / 2 - first) + i] = row < 64 ? v[CW / 2 + i] : v[i];
             asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll
             for (int i = 0; i < CW / 2; ++i) {
                 const float other = shared_row[first + i];
-                v[i] = row < 64 ? gate_value_near(p.gate, v[i], other) : gate_value_near(p.gate, other, v[CW / 2 + i]);
+                v[i] = gate_value_near(p.gate, row < 64 ? v[i] : other, row < 64 ? other : v[CW / 2 + i]);
             }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-        } else if (p.bias && mine) {
-            const float shift = p.bias[f0 + row];
+        } else {
+            if (p.bias && mine) {
+                const float shift = p.bias[f0 + row];
 #pragma unroll
-            for (int i = 0; i < CW; ++i) v[i] += shift;
+                for (int i = 0; i < CW; ++i) v[i] += shift;
+            }
+            if (staged) asm volatile("bar.sync 1, 128;" ::: "memory");
         }
-        if (sizeof(TY) == 2 && p.staged) {
-            bf16* out = staging + (staged_chunks & 1) * (CW * SPAN);
-            // The copy that read this buffer two chunks ago must be through with it.
-            if (threadIdx.x == 64 && staged_chunks >= 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+        ++staged_chunks;
+        if (staged) {
 #pragma unroll
             for (int i = 0; i < COUNT; ++i) out[(first + i) * SPAN + feature] = __float2bfloat16_rn(v[i]);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the copy reads what these threads wrote
@@ -283,7 +294,6 @@ __device__ __forceinline__ void store_tile(const Params& p, const CUtensorMap& m
                 if (CW > 16 && c + 16 < columns) tma_store_2d(&map_y, out + 16 * SPAN, f0, t0 + c + 16);
                 tma_store_commit();
             }
-            ++staged_chunks;
         } else if (mine) {
 #pragma unroll
             for (int i = 0; i < COUNT; ++i) {
@@ -317,13 +327,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     constexpr int SPAN = GATED ? 64 : BM;                  // output features per tile
     extern __shared__ unsigned char raw[];
     unsigned char* tiles = (unsigned char*)(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
-    // The gated epilogue passes the up rows of a chunk of columns between warps (64 x (columns + 1) floats).
+    // The gated epilogue passes the up rows of a chunk of columns between warps (two buffers of 64 x 17 floats).
     float* exchange = reinterpret_cast<float*>(tiles + (size_t)STAGES * STAGE_BYTES);
     // Results on their way out (p.staged): two buffers of CW tokens x SPAN features, which TMA stores
     // write to y in whole lines (a thread holds one feature of CW tokens: stored directly, every
     // token's 32 features of a warp would be a 64-byte piece of its own).
-    constexpr int CW = epilogue_columns<BN>();
-    bf16* staging = reinterpret_cast<bf16*>(tiles + (size_t)STAGES * STAGE_BYTES + 64 * (CW + 1) * sizeof(float));
+    constexpr int CW = epilogue_columns<BN, GATED>();
+    bf16* staging = reinterpret_cast<bf16*>(tiles + (size_t)STAGES * STAGE_BYTES + exchange_bytes<GATED>());
     __shared__ unsigned long long full_bar[STAGES], empty_bar[STAGES], ready_bar[2], drained_bar[2];
     __shared__ unsigned tmem_base_slot;
     __shared__ int gave_up, is_last;
@@ -692,10 +702,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 // 1,801 rows of 24,576 x 4,096). Microseconds, a block a tile and this: 24,576 x 4,096 with 1,801 rows 281 and 272, 4,096 rows
 // 559 and 530; 4,096 x 12,288 with 1,100 rows 154 and 100, 1,801 rows 157 and 141; 6,144 x 4,096 with 1,801 rows 76 and 69;
 // 2,048 x 2,048 with 1,024 rows 26 and 13.
-constexpr int PAIR_STAGES = 6, PAIR_COLUMNS = 256, PAIR_CW = 32;
+constexpr int PAIR_STAGES = 6, PAIR_COLUMNS = 256;
 constexpr int PAIR_STAGE_BYTES = BM * BK * 2 + PAIR_COLUMNS / 2 * BK * 2;
 constexpr size_t pair_shared_bytes() {
-    return 1024 + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + 64 * (PAIR_CW + 1) * sizeof(float) + 2 * PAIR_CW * BM * sizeof(bf16);
+    return 1024 + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + most_epilogue_bytes<PAIR_COLUMNS>();
 }
 
 // Both blocks' copies report to the first one's barrier.
@@ -734,7 +744,7 @@ gemm_tcgen05_pairs_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     extern __shared__ unsigned char raw[];
     unsigned char* tiles = (unsigned char*)(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
     float* exchange = reinterpret_cast<float*>(tiles + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES);
-    bf16* staging = reinterpret_cast<bf16*>(exchange + 64 * (PAIR_CW + 1));
+    bf16* staging = reinterpret_cast<bf16*>(tiles + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + exchange_bytes<GATED>());
     __shared__ unsigned long long full_bar[PAIR_STAGES], empty_bar[PAIR_STAGES], ready_bar[2], drained_bar[2];
     __shared__ unsigned tmem_base_slot;
     __shared__ int gave_up;
@@ -857,7 +867,7 @@ gemm_tcgen05_pairs_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             if (!ok && lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.error, 3); }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // (all four warps take part, whatever they found: they meet at barriers)
-            if (f0 < p.features) store_tile<GATED, PAIR_CW, TY>(p, map_y, accumulator, f0, t0, p.columns, ok, row, exchange, staging, staged_chunks);
+            if (f0 < p.features) store_tile<GATED, epilogue_columns<PAIR_COLUMNS, GATED>(), TY>(p, map_y, accumulator, f0, t0, p.columns, ok, row, exchange, staging, staged_chunks);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(drained[buffer]) : "memory");
