@@ -38,7 +38,9 @@ MIN_FEATURES = 16384                    # the dispatcher uses this kernel for we
 TALL_FEATURES = 65536
 MAX_ROWS_TALL = int(os.environ.get("KIDI_B200_TCGEN05_MAX_ROWS_TALL", "64"))
 MIN_GATED_ROWS = 9                      # and its fused SiLU gate from this many rows on (below: the skinny kernel)
-# The most rows for the fused gate (and within MAX_ROWS): beyond, the product followed by the gate kernel is faster.
+# The most rows for the fused gate (and within MAX_ROWS): beyond, the product followed by the gate kernel is faster, up to prompts
+# (`fits_prompt`), whose epilogues run beside the next tile's products: 1,801 rows of 2 x 12,288 x 4,096 270 us against 296,
+# of 2 x 2,816 x 2,048 38 against 43.
 MAX_GATED_ROWS = int(os.environ.get("KIDI_B200_TCGEN05_MAX_GATED_ROWS", "32"))
 COUNTERS = 4096                         # two per block of a launch (two blocks an SM at most)
 
@@ -118,7 +120,8 @@ def _run(x, weight, out, features: int, gated: bool, splits: Optional[int], bias
         _ptr(x), _ptr(weight), _ptr(out), dtype_code(out.dtype), rows, features, K, x.stride(0), weight.stride(0),
         out.stride(0), 1 if gated else 0, splits, _ptr(workspace), _ptr(counters), _ptr(error), _ptr(bias),
         _stream()),
-        "gemm_silu_gate[tcgen05]" if gated else "gemm_tcgen05")
+        # (a prompt's product bears the kernel's name with and without the gate in its epilogue)
+        "gemm_silu_gate[tcgen05]" if gated and not 0 < PROMPT_ROWS <= rows else "gemm_tcgen05")
 
 
 def gemm(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, out: Optional[torch.Tensor] = None,

@@ -191,6 +191,8 @@ class RoutedExperts(Part):
         up, down = self._shared
         if skinny.fits(x, up.weight) and up.bias is None:            # few rows: the activation in the epilogue
             mid = skinny.gemm_silu_gate(x, up.weight, shape=self.shared_shape) if self.gated else skinny.gemm(x, up.weight, x.dtype, activation="gelu")
+        elif self.gated and self.shared_shape is None and up.bias is None and tcgen05.fits_prompt(x, up.weight):
+            mid = tcgen05.gemm_silu_gate(x, up.weight)
         else:
             mid = self._activate(up.forward(x), self.shared_shape)
         return down.forward(mid)

@@ -491,3 +491,28 @@ def test_a_toy_mixer_with_state_of_its_own(tmp_path):
     for held in [bystander, *slots]:
         engine.release(held)
     engine.cache.check()
+
+
+@pytest.mark.parametrize("rows", [1023, 1024, 1300])
+@pytest.mark.parametrize("kind", ["gated_mlp", "routed_experts"])
+def test_a_prompt_has_its_gate_in_the_product(kind, rows):
+    """From 1,024 rows on gate and up projections and the gate are one launch, of the layer's feed-forward and of a shared expert."""
+    from kidi_b200.kernels import ops
+    from kidi_b200.parts.registry import build_part
+    from kidi_b200.parts.spec import PartSpec
+    params = {"hidden_size": 128, "intermediate_size": 200, "activation": "silu"} if kind == "gated_mlp" else \
+        {"hidden_size": 128, "expert_size": 64, "experts": 4, "top": 2, "score": "softmax", "renormalise": True, "weight_on": "output",
+         "shared_size": 200}
+    part = build_part("feed_forward", PartSpec(kind, params, "mlp."), make_env(torch.bfloat16))
+    tensors = {name: (t * 3).to(DEVICE) for name, t in random_tensors(part, torch.bfloat16).items()}
+    part.bind(tensors)
+    part.bound()
+    cache, slots = step_context([], [0], None, torch.bfloat16, max_positions=4096)
+    ctx, _ = run_step(cache, slots, [[0] * rows], torch.bfloat16)
+    x = torch.randn(rows, 128, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16).to(DEVICE)
+    with ops.record_launches() as names:
+        found = part.forward(x, ctx)
+    assert ("silu_gate" in names) == (rows < 1024) and names.count("gemm_tcgen05") == (2 if rows >= 1024 else 0), names
+    few = torch.cat([part.forward(piece, run_step(cache, slots, [[0] * len(piece)], torch.bfloat16)[0]) for piece in x.split(500)])
+    # bfloat16 results of up to three products behind one another: 2^-9 each, of sums whose terms are rounded likewise.
+    assert float((found.double() - few.double()).norm() / few.double().norm()) < 6 * 2.0 ** -9
