@@ -110,6 +110,21 @@ __device__ __forceinline__ bool mbarrier_wait(unsigned long long* bar, unsigned 
     kidi_attention_timeout = 1;
     return false;
 }
+// The same for a whole warp, whose lanes go on together or not at all.
+__device__ __forceinline__ bool mbarrier_wait_warp(unsigned long long* bar, unsigned parity, volatile int* gave_up) {
+    return __all_sync(0xffffffffu, mbarrier_wait(bar, parity, gave_up));
+}
+// One thread of a warp that is here as a whole: copies and matrix instructions, whose operands stand in the warp's shared
+// registers, are issued at their full rate from such code; from a branch on the lane's number one took 50 to 140 cycles.
+__device__ __forceinline__ bool elect_one() {
+    unsigned elected = 0;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "@p mov.u32 %0, 1;\n\t}"
+        : "+r"(elected));
+    return elected != 0;
+}
 __device__ __forceinline__ void tma_load_2d(void* smem, const CUtensorMap* map, unsigned long long* bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -145,14 +160,14 @@ __host__ __device__ constexpr unsigned instr_desc(int n, bool b_mn_major) {
 }
 // The instruction is ordered with the barriers around it by tcgen05.commit and the
 // tcgen05 fences, which carry the memory clobbers.
-__device__ __forceinline__ void umma(unsigned tmem_d, unsigned long long a, unsigned long long b, unsigned idesc,
-                                     bool accumulate) {
+template <bool ACCUMULATE>
+__device__ __forceinline__ void umma(unsigned tmem_d, unsigned long long a, unsigned long long b, unsigned idesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         :
-        : "r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"((unsigned)accumulate));
+        : "r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "n"(ACCUMULATE ? 1 : 0));
 }
 __device__ __forceinline__ void umma_commit(unsigned long long* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
@@ -485,7 +500,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const 
     const Place first_look(p);
     if (first_look.q0 >= first_look.count) return;
     const int heads_here = first_look.heads_here;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         mbarrier_init(&ctl.q_full, 1);
@@ -529,53 +544,56 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const 
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CONTROL_REGISTERS));
         if (warp < HEADS) {
             const int h = warp;
-            if (lane == 0 && h < heads_here) {
+            if (h < heads_here) {
                 const Place at(p);
                 const int tiles = at.tiles;
-                // ------------------------------ matrix instructions of head h (one thread a head)
+                // ------------------------------ matrix instructions of head h (one thread of a warp a head)
                 // The operand descriptors are built once; a step along k adds to the address field
                 // (16-byte units; a shared-memory address never carries out of its 14 bits).
                 constexpr unsigned idesc_s = instr_desc(BN, false), idesc_o = instr_desc(D, true);
                 const unsigned long long q_desc = desc_k_major(q_tiles + h * QKV_TILE), k_desc = desc_k_major(k_tile);
                 const unsigned long long p_desc = desc_k_major(p_tiles + h * P_TILE);
-                const unsigned tmem_s = tmem + h * 128, tmem_o = tmem + 256 + h * 128;
-                // (The loops over k stay rolled: this thread runs with few registers, and an
-                // instruction takes longer to be accepted than its operands to be computed.)
+                const unsigned memory = __shfl_sync(0xffffffffu, tmem, 0);
+                const unsigned tmem_s = memory + h * 128, tmem_o = memory + 256 + h * 128;
+                auto along = [](int kk) { return (unsigned)((kk >> 2) * (SPAN_BYTES >> 4) + (kk & 3) * 2); };
                 auto scores = [&]() {                   // S_h = Q_h K^T
-#pragma unroll 1
-                    for (int kk = 0; kk < D / 16; ++kk) {
-                        const unsigned offset = (kk >> 2) * (SPAN_BYTES >> 4) + (kk & 3) * 2;
-                        umma(tmem_s, q_desc + offset, k_desc + offset, idesc_s, kk > 0);
+                    if (elect_one()) {
+                        umma<false>(tmem_s, q_desc, k_desc, idesc_s);
+#pragma unroll
+                        for (int kk = 1; kk < D / 16; ++kk) umma<true>(tmem_s, q_desc + along(kk), k_desc + along(kk), idesc_s);
+                        umma_commit(&ctl.s_ready[h]);
+                        umma_commit(&ctl.k_free);
                     }
-                    umma_commit(&ctl.s_ready[h]);
-                    umma_commit(&ctl.k_free);
+                    __syncwarp();
                 };
-                bool ok = mbarrier_wait(&ctl.q_full, 0, abort_flag) && mbarrier_wait(&ctl.k_full, 0, abort_flag);
+                bool ok = mbarrier_wait_warp(&ctl.q_full, 0, abort_flag) && mbarrier_wait_warp(&ctl.k_full, 0, abort_flag);
                 if (ok) scores();
                 for (int j = 0; j < tiles && ok; ++j) {
                     if (j + 1 < tiles) {             // the head's next scores, as soon as the softmax warps hold these
-                        ok = mbarrier_wait(&ctl.k_full, (j + 1) & 1, abort_flag) &&
-                             mbarrier_wait(&ctl.s_free[h], j & 1, abort_flag);
+                        ok = mbarrier_wait_warp(&ctl.k_full, (j + 1) & 1, abort_flag) &&
+                             mbarrier_wait_warp(&ctl.s_free[h], j & 1, abort_flag);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         scores();
                     }
-                    ok = mbarrier_wait(&ctl.v_full[j & 1], (j >> 1) & 1, abort_flag);
-                    ok = ok && mbarrier_wait(&ctl.p_ready[h], j & 1, abort_flag);
+                    ok = mbarrier_wait_warp(&ctl.v_full[j & 1], (j >> 1) & 1, abort_flag);
+                    ok = ok && mbarrier_wait_warp(&ctl.p_ready[h], j & 1, abort_flag);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned long long v_desc = desc_mn_major(v_tiles + (j & 1) * QKV_TILE, SPAN_BYTES);
-#pragma unroll 1
-                    for (int kk = 0; kk < BN / 16; ++kk) {
-                        const unsigned a_offset = (kk >> 2) * (SPAN_BYTES >> 4) + (kk & 3) * 2;
-                        umma(tmem_o, p_desc + a_offset, v_desc + kk * (2048 >> 4), idesc_o, j > 0 || kk > 0);
+                    if (elect_one()) {
+                        if (j == 0) umma<false>(tmem_o, p_desc, v_desc, idesc_o);
+                        else umma<true>(tmem_o, p_desc, v_desc, idesc_o);
+#pragma unroll
+                        for (int kk = 1; kk < BN / 16; ++kk) umma<true>(tmem_o, p_desc + along(kk), v_desc + kk * (2048 >> 4), idesc_o);
+                        umma_commit(&ctl.pv_done[h]);
+                        umma_commit(&ctl.v_free[j & 1]);
                     }
-                    umma_commit(&ctl.pv_done[h]);
-                    umma_commit(&ctl.v_free[j & 1]);
+                    __syncwarp();
                 }
             }
         } else if (warp == HEADS) {
-            if (lane == 0) {
+            {
                 // -------------------------------------------------------------- copies
                 const Place at(p);
                 const int tiles = at.tiles, tile_low = at.tile_low, row0 = at.row0, q0 = at.q0, head0 = at.head0;
@@ -606,22 +624,27 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const 
                     if (p.from_cache) load_pages(v_tiles + (j & 1) * QKV_TILE, &ctl.v_full[j & 1], &v_map, j);
                     else load_tile(v_tiles + (j & 1) * QKV_TILE, &ctl.v_full[j & 1], v_col, row0 + (tile_low + j) * BN, &map);
                 };
-                mbarrier_expect_tx(&ctl.q_full, heads_here * QKV_TILE);
-                for (int h = 0; h < heads_here; ++h)
-                    load_tile(q_tiles + h * QKV_TILE, &ctl.q_full, (head0 + h) * D, row0 + q0, &map);
-                load_k(0);
-                load_v(0);
-                if (tiles > 1) load_v(1);
+                if (elect_one()) {
+                    mbarrier_expect_tx(&ctl.q_full, heads_here * QKV_TILE);
+                    for (int h = 0; h < heads_here; ++h)
+                        load_tile(q_tiles + h * QKV_TILE, &ctl.q_full, (head0 + h) * D, row0 + q0, &map);
+                    load_k(0);
+                    load_v(0);
+                    if (tiles > 1) load_v(1);
+                }
+                __syncwarp();
                 bool ok = true;
                 for (int j = 0; j + 1 < tiles && ok; ++j) {
                     // Both heads' scores of tile j are done (they were issued a tile ago): K_{j+1} follows.
-                    ok = mbarrier_wait(&ctl.k_free, j & 1, abort_flag);
+                    ok = mbarrier_wait_warp(&ctl.k_free, j & 1, abort_flag);
                     if (!ok) break;
-                    load_k(j + 1);
+                    if (elect_one()) load_k(j + 1);
+                    __syncwarp();
                     if (j >= 1) {                    // both heads' P V_{j-1} are done: the buffer takes V_{j+1}
-                        ok = mbarrier_wait(&ctl.v_free[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag);
+                        ok = mbarrier_wait_warp(&ctl.v_free[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag);
                         if (!ok) break;
-                        load_v(j + 1);
+                        if (elect_one()) load_v(j + 1);
+                        __syncwarp();
                     }
                 }
             }
