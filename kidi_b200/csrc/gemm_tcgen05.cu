@@ -213,25 +213,76 @@ struct Params {
     long long tail_first;  // the first tile of the tail
     int share, extra;      // of the tail's k-blocks a block takes `share`, the first `extra` blocks one more
     int staged;            // results leave through shared memory and TMA stores (bfloat16 y, 16-byte aligned rows)
-    const int* group_of_tile;   // [token tiles] (GROUPED): the tile's tokens take the weight rows from group * group_rows on
+    const int* group_of_tile;   // [tiles of 128 tokens] (weights in groups): the tile's tokens take the weight rows from group * group_rows on
                                 // (a tile whose group is negative holds no tokens and is left out)
     int group_rows;
     const int* used_of_tile;    // [token tiles] or null (all of them): the rows of a tile that are wanted, from its first one on
     GateShape gate;             // the gated form's activation (all zero: SiLU)
 };
 
-// Weights in groups: the rows' tiles are 128 tokens high. A block takes two neighbouring tiles of one group at once (the
-// weights are loaded once for both, and at 128 tokens a tile the operands' way from the L2 is what bounds it: 32 KB for 256
-// cycles of matrix instructions against 48 KB for 512), and of those the tokens that are wanted, in steps of 16. Which tiles
-// begin such a piece of work every block finds out for itself, in shared memory.
+// Weights in groups: the rows' tiles are 128 tokens high. A pair of blocks takes two neighbouring tiles of one group at once (the
+// weights are loaded once for both), and of those the tokens that are wanted, in steps of 16. Which tiles begin such a piece of
+// work every block finds out for itself, in shared memory.
 constexpr int GROUP_TILE = 128, MOST_GROUP_TILES = 1024;
-constexpr int GROUP_BOX = 64;        // tokens of a copy
+constexpr int GROUP_BOX = 32;        // tokens of a copy
 struct GroupPieces {
     int count;                       // pieces of work
     short tile[MOST_GROUP_TILES];    // a piece's first tile
     int group[MOST_GROUP_TILES];     // of a tile (negative: none), then of a piece
     unsigned char wanted[MOST_GROUP_TILES];   // of a tile in rows, then of a piece in steps of 16 tokens
 };
+
+// Which tiles begin a piece of work, its group and the steps of 16 tokens it has: found by the whole block.
+__device__ __forceinline__ void find_pieces(const Params& p, GroupPieces* pieces, int warp, int lane) {
+    for (int i = threadIdx.x; i < p.token_tiles; i += THREADS) {
+        pieces->group[i] = p.group_of_tile[i];
+        pieces->wanted[i] = p.used_of_tile ? (unsigned char)min(max(p.used_of_tile[i], 0), GROUP_TILE) : GROUP_TILE;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int count = 0, run = 0;                    // pieces so far; where the run of the last tile's group begins
+        for (int base = 0; base < p.token_tiles; base += 32) {
+            const int i = base + lane;
+            const int group = i < p.token_tiles ? pieces->group[i] : -1;
+            const unsigned heads = __ballot_sync(0xffffffffu, i < p.token_tiles && (i == 0 || pieces->group[i - 1] != group)) &
+                                   (0xffffffffu >> (31 - lane));
+            const int first = heads ? base + 31 - __clz(heads) : run;      // of the run of the tile's group
+            run = __shfl_sync(0xffffffffu, first, 31);
+            const bool begins = group >= 0 && !((i - first) & 1) && pieces->wanted[i] > 0;
+            const unsigned all = __ballot_sync(0xffffffffu, begins);
+            if (begins) pieces->tile[count + __popc(all & ((1u << lane) - 1))] = (short)i;
+            count += __popc(all);
+        }
+        if (lane == 0) pieces->count = count;
+    }
+    __syncthreads();
+    // (a piece's number is at most its tile's: what is overwritten here has been read by then only if everybody reads first)
+    constexpr int MINE = (MOST_GROUP_TILES + THREADS - 1) / THREADS;
+    int group[MINE];
+    unsigned char wanted[MINE];
+#pragma unroll
+    for (int k = 0; k < MINE; ++k) {
+        const int i = threadIdx.x + k * THREADS;
+        group[k] = -1;
+        wanted[k] = 0;
+        if (i < pieces->count) {
+            const int tile = pieces->tile[i];
+            const bool two = tile + 1 < p.token_tiles && pieces->group[tile + 1] == pieces->group[tile] && pieces->wanted[tile + 1] > 0;
+            group[k] = pieces->group[tile];
+            wanted[k] = (unsigned char)((two ? GROUP_TILE + pieces->wanted[tile + 1] + 15 : pieces->wanted[tile] + 15) / 16);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < MINE; ++k) {
+        const int i = threadIdx.x + k * THREADS;
+        if (i < pieces->count) {
+            pieces->group[i] = group[k];
+            pieces->wanted[i] = wanted[k];
+        }
+    }
+    __syncthreads();
+}
 
 // Shared memory of a block: the stages and the epilogue's buffers;
 // behind them (`pieces`, in the build for weights in groups) what a block knows of those.
@@ -315,9 +366,7 @@ __device__ __forceinline__ void store_tile(const Params& p, const CUtensorMap& m
 // A block keeps its ring of operand stages full across the borders of tiles, and the accumulator
 // is double-buffered in tensor memory (2 x BN columns): while the four epilogue warps read one
 // piece of work out, the tensor core is at the next.
-// GROUPED: weights in groups, a build of its own, so that the others carry neither its tables nor its widths of a tile that are
-// known at run time only (with them 1,801 rows through gate, up and down of 4,096 x 12,288 took 557 us instead of 531 to 548).
-template <int BN, int STAGES, bool GATED, typename TY, bool GROUPED = false>
+template <int BN, int STAGES, bool GATED, typename TY>
 __global__ void __launch_bounds__(THREADS, BN <= 64 ? 2 : 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     const __grid_constant__ CUtensorMap map_y, Params p) {
@@ -350,60 +399,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     // feature tile (the blocks at work at one time share few weight tiles and eight token tiles,
     // however long the prompt), column after column.
     const int feature_tiles = (int)(p.tiles / p.token_tiles);
-    [[maybe_unused]] GroupPieces* pieces = reinterpret_cast<GroupPieces*>(tiles + shared_floor<BN, STAGES>());
-    if constexpr (GROUPED) {
-        for (int i = threadIdx.x; i < p.token_tiles; i += THREADS) {
-            pieces->group[i] = p.group_of_tile[i];
-            pieces->wanted[i] = p.used_of_tile ? (unsigned char)min(max(p.used_of_tile[i], 0), GROUP_TILE) : GROUP_TILE;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            int count = 0, run = 0;                    // pieces so far; where the run of the last tile's group begins
-            for (int base = 0; base < p.token_tiles; base += 32) {
-                const int i = base + lane;
-                const int group = i < p.token_tiles ? pieces->group[i] : -1;
-                const unsigned heads = __ballot_sync(0xffffffffu, i < p.token_tiles && (i == 0 || pieces->group[i - 1] != group)) &
-                                       (0xffffffffu >> (31 - lane));
-                const int first = heads ? base + 31 - __clz(heads) : run;      // of the run of the tile's group
-                run = __shfl_sync(0xffffffffu, first, 31);
-                const bool begins = group >= 0 && !((i - first) & 1) && pieces->wanted[i] > 0;
-                const unsigned all = __ballot_sync(0xffffffffu, begins);
-                if (begins) pieces->tile[count + __popc(all & ((1u << lane) - 1))] = (short)i;
-                count += __popc(all);
-            }
-            if (lane == 0) pieces->count = count;
-        }
-        __syncthreads();
-        // (a piece's number is at most its tile's: what is overwritten here has been read by then only if everybody reads first)
-        constexpr int MINE = (MOST_GROUP_TILES + THREADS - 1) / THREADS;
-        int group[MINE];
-        unsigned char wanted[MINE];
-#pragma unroll
-        for (int k = 0; k < MINE; ++k) {
-            const int i = threadIdx.x + k * THREADS;
-            group[k] = -1;
-            wanted[k] = 0;
-            if (i < pieces->count) {
-                const int tile = pieces->tile[i];
-                const bool two = tile + 1 < p.token_tiles && pieces->group[tile + 1] == pieces->group[tile] && pieces->wanted[tile + 1] > 0;
-                group[k] = pieces->group[tile];
-                wanted[k] = (unsigned char)((two ? GROUP_TILE + pieces->wanted[tile + 1] + 15 : pieces->wanted[tile] + 15) / 16);
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < MINE; ++k) {
-            const int i = threadIdx.x + k * THREADS;
-            if (i < pieces->count) {
-                pieces->group[i] = group[k];
-                pieces->wanted[i] = wanted[k];
-            }
-        }
-        __syncthreads();
-    }
-    const int token_tiles = GROUPED ? pieces->count : p.token_tiles;
-    const long long whole_tiles = GROUPED ? (long long)token_tiles * feature_tiles : p.tail_first;
-    const int rounds = GROUPED ? (int)((whole_tiles + gridDim.x - 1) / gridDim.x) : p.rounds;
+    const int token_tiles = p.token_tiles, rounds = p.rounds;
+    const long long whole_tiles = p.tail_first;
     auto locate = [&](long long tile, int& token_tile, int& feature_tile) {
         const long long column = tile / (8LL * feature_tiles), within = tile - column * 8 * feature_tiles;
         const int wide = min(8, token_tiles - (int)column * 8);
@@ -412,9 +409,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     };
     // A tile's first token, its tokens (in steps of 16) and, with weights in groups (the experts of a routed feed-forward), its
     // group's first weight row.
-    auto first_token = [&](int token_tile) { return GROUPED ? pieces->tile[token_tile] * GROUP_TILE : token_tile * BN; };
-    auto columns_of = [&](int token_tile) { return GROUPED ? pieces->wanted[token_tile] * 16 : BN; };
-    auto group_begin = [&](int token_tile) { return GROUPED ? pieces->group[token_tile] * p.group_rows : 0; };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -447,8 +441,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         auto load = [&](long long tile, int kb_first, int kb_count) {
             int token_tile, feature_tile;
             locate(tile, token_tile, feature_tile);
-            const int f0 = group_begin(token_tile) + feature_tile * SPAN, t0 = first_token(token_tile);
-            const int boxes = (columns_of(token_tile) + GROUP_BOX - 1) / GROUP_BOX;
+            const int f0 = feature_tile * SPAN, t0 = token_tile * BN;
             for (int i = 0; i < kb_count; ++i, ++issued) {
                 const int s = issued % STAGES;
                 if (issued >= STAGES) ok = mbarrier_wait_warp(&empty_bar[s], ((issued / STAGES) - 1) & 1, abort_flag);
@@ -458,7 +451,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 }
                 if (elect_one()) {
                     unsigned char* stage = tiles + (size_t)s * STAGE_BYTES;
-                    mbarrier_expect_tx(&full_bar[s], GROUPED ? A_BYTES + boxes * GROUP_BOX * BK * 2 : STAGE_BYTES);
+                    mbarrier_expect_tx(&full_bar[s], STAGE_BYTES);
                     const int k = (kb_first + i) * BK;
                     if (GATED) {
                         tma_load_2d(stage, &map_w, &full_bar[s], k, f0);                            // 64 gate rows
@@ -466,11 +459,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     } else {
                         tma_load_2d(stage, &map_w, &full_bar[s], k, f0);
                     }
-                    if (GROUPED)
-                        for (int box = 0; box < boxes; ++box)
-                            tma_load_2d(stage + A_BYTES + box * GROUP_BOX * BK * 2, &map_x, &full_bar[s], k, t0 + box * GROUP_BOX);
-                    else
-                        tma_load_2d(stage + A_BYTES, &map_x, &full_bar[s], k, t0);
+                    tma_load_2d(stage + A_BYTES, &map_x, &full_bar[s], k, t0);
                 }
                 __syncwarp();
             }
@@ -495,8 +484,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         int consumed = 0, done = 0;                        // stages read, accumulators finished
         bool ok = true;                                    // (the same in all lanes)
         const unsigned memory = __shfl_sync(0xffffffffu, tmem_base, 0);
-        auto multiply = [&](int kb_count, int columns) {
-            const unsigned idesc = make_instr_desc(columns);
+        auto multiply = [&](int kb_count) {
+            constexpr unsigned idesc = make_instr_desc(BN);
             const int buffer = done & 1;
             // The accumulator's last reader (two pieces of work ago) must have read it out.
             if (done >= 2) ok = mbarrier_wait_warp(&drained_bar[buffer], ((done >> 1) - 1) & 1, abort_flag);
@@ -531,14 +520,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         for (int round = 0; round < rounds && ok; ++round) {
             const long long tile = blockIdx.x + (long long)round * gridDim.x;
             if (tile >= whole_tiles) break;
-            int token_tile = 0, feature_tile;
-            if (GROUPED) locate(tile, token_tile, feature_tile);
-            multiply(p.k_blocks, columns_of(token_tile));
+            multiply(p.k_blocks);
         }
         for (long long g = piece_begin; g < piece_end && ok;) {
             const int kb_first = (int)(g % p.k_blocks);
             const int kb_count = (int)min((long long)(p.k_blocks - kb_first), piece_end - g);
-            multiply(kb_count, BN);
+            multiply(kb_count);
             g += kb_count;
         }
     } else if (warp >= 2) {
@@ -554,7 +541,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         auto finish = [&](long long tile, long long tail_tile, int kb_first, int kb_count) {
             int token_tile, feature_tile;
             locate(tile, token_tile, feature_tile);
-            const int f0 = feature_tile * SPAN, t0 = first_token(token_tile), columns = columns_of(token_tile);
+            const int f0 = feature_tile * SPAN, t0 = token_tile * BN;
             const int buffer = done & 1;
             const unsigned accumulator = tmem_base + buffer * BUFFER_COLUMNS + ((unsigned)(quarter * 32) << 16);
             bool ok = !*abort_flag && mbarrier_wait(&ready_bar[buffer], (done >> 1) & 1, abort_flag);
@@ -593,7 +580,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 }
                 return;
             }
-            store_tile<GATED, CW, TY>(p, map_y, accumulator, f0, t0, columns, ok, row, exchange, staging, staged_chunks);
+            store_tile<GATED, CW, TY>(p, map_y, accumulator, f0, t0, BN, ok, row, exchange, staging, staged_chunks);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             mbarrier_arrive(&drained_bar[buffer]);
         };
@@ -704,8 +691,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 // 2,048 x 2,048 with 1,024 rows 26 and 13.
 constexpr int PAIR_STAGES = 6, PAIR_COLUMNS = 256;
 constexpr int PAIR_STAGE_BYTES = BM * BK * 2 + PAIR_COLUMNS / 2 * BK * 2;
-constexpr size_t pair_shared_bytes() {
-    return 1024 + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + most_epilogue_bytes<PAIR_COLUMNS>();
+template <bool GROUPED> constexpr size_t pair_shared_bytes() {
+    return (GROUPED ? sizeof(GroupPieces) : 0) + 1024 + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + most_epilogue_bytes<PAIR_COLUMNS>();
 }
 
 // Both blocks' copies report to the first one's barrier.
@@ -736,7 +723,7 @@ __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <bool GATED, typename TY>
+template <bool GATED, typename TY, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tcgen05_pairs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                           const __grid_constant__ CUtensorMap map_y, Params p) {
@@ -774,21 +761,26 @@ gemm_tcgen05_pairs_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem_base = tmem_base_slot;
 
-    // Tiles in columns of eight token tiles, as above.
-    const int tall = (int)(p.tiles / p.token_tiles);
-    auto locate = [&](int tile, int& t0, int& f0) {
-        const int column = tile / (8 * tall), within = tile - column * 8 * tall, wide = min(8, p.token_tiles - column * 8);
-        t0 = (column * 8 + within % wide) * p.columns;
-        f0 = (within / wide * 2 + rank) * SPAN;
+    GroupPieces* pieces = reinterpret_cast<GroupPieces*>(tiles + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + most_epilogue_bytes<PAIR_COLUMNS>());
+    if (GROUPED) find_pieces(p, pieces, warp, lane);
+    // Tiles in columns of eight token tiles, as above. A tile's first token, its tokens (a multiple of 32), its first feature and
+    // its first weight row.
+    const int token_tiles = GROUPED ? pieces->count : p.token_tiles;
+    const int tall = (p.features + 2 * SPAN - 1) / (2 * SPAN), count = token_tiles * tall;
+    struct Tile { int t0, columns, f0, w0; };
+    auto locate = [&](int tile) {
+        const int column = tile / (8 * tall), within = tile - column * 8 * tall, wide = min(8, token_tiles - column * 8);
+        const int which = column * 8 + within % wide, f0 = (within / wide * 2 + rank) * SPAN;
+        if (GROUPED) return Tile{pieces->tile[which] * GROUP_TILE, (pieces->wanted[which] + 1) / 2 * 32, f0, pieces->group[which] * p.group_rows + f0};
+        return Tile{which * p.columns, p.columns, f0, f0};
     };
-    const int half = p.columns / 2;
     bool ok = true;                                        // (the same in all lanes)
     if (warp == 0) {
         // ------------------------------------------------------------ producer: this block's features, its half of the tokens
         int issued = 0;
-        for (int tile = pair; tile < p.tiles && ok; tile += pairs) {
-            int t0, f0;
-            locate(tile, t0, f0);
+        for (int tile = pair; tile < count && ok; tile += pairs) {
+            const Tile at = locate(tile);
+            const int half = at.columns / 2, boxes = GROUPED ? (half + GROUP_BOX - 1) / GROUP_BOX : 1, box_rows = GROUPED ? GROUP_BOX : half;
             for (int kb = 0; kb < p.k_blocks; ++kb, ++issued) {
                 const int s = issued % PAIR_STAGES, k = kb * BK;
                 if (issued >= PAIR_STAGES) ok = mbarrier_wait_warp(&empty_bar[s], ((issued / PAIR_STAGES) - 1) & 1, abort_flag);
@@ -798,14 +790,15 @@ gemm_tcgen05_pairs_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                 }
                 if (elect_one()) {
                     unsigned char* stage = tiles + (size_t)s * PAIR_STAGE_BYTES;
-                    if (rank == 0) mbarrier_expect_tx(&full_bar[s], 2 * (A_BYTES + half * BK * 2));
+                    if (rank == 0) mbarrier_expect_tx(&full_bar[s], 2 * (A_BYTES + boxes * box_rows * BK * 2));
                     if (GATED) {
-                        tma_load_pair(stage, &map_w, &full_bar[s], k, f0);
-                        tma_load_pair(stage + A_BYTES / 2, &map_w, &full_bar[s], k, p.features + f0);
+                        tma_load_pair(stage, &map_w, &full_bar[s], k, at.w0);
+                        tma_load_pair(stage + A_BYTES / 2, &map_w, &full_bar[s], k, p.features + at.w0);
                     } else {
-                        tma_load_pair(stage, &map_w, &full_bar[s], k, f0);
+                        tma_load_pair(stage, &map_w, &full_bar[s], k, at.w0);
                     }
-                    tma_load_pair(stage + A_BYTES, &map_x, &full_bar[s], k, t0 + rank * half);
+                    for (int box = 0; box < boxes; ++box)
+                        tma_load_pair(stage + A_BYTES + box * GROUP_BOX * BK * 2, &map_x, &full_bar[s], k, at.t0 + rank * half + box * GROUP_BOX);
                 }
                 __syncwarp();
             }
@@ -819,9 +812,9 @@ gemm_tcgen05_pairs_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     } else if (warp == 1) {
         // -------------------------------------------------------------- issuer: the first block's, for both
         const unsigned memory = __shfl_sync(0xffffffffu, tmem_base, 0);
-        const unsigned idesc = make_instr_desc(p.columns) + ((unsigned)(BM >> 4) << 24);           // M = 256
         int consumed = 0, done = 0;
-        for (int tile = pair; rank == 0 && tile < p.tiles && ok; tile += pairs, ++done) {
+        for (int tile = pair; rank == 0 && tile < count && ok; tile += pairs, ++done) {
+            const unsigned idesc = make_instr_desc(locate(tile).columns) + ((unsigned)(BM >> 4) << 24);         // M = 256
             const int buffer = done & 1;
             if (done >= 2) ok = mbarrier_wait_warp(&drained_bar[buffer], ((done >> 1) - 1) & 1, abort_flag);
             if (!ok) {
@@ -858,16 +851,16 @@ gemm_tcgen05_pairs_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
         for (int b = 0; b < 2; ++b)
             asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(drained[b]) : "r"(smem_u32(&drained_bar[b])));
         int done = 0, staged_chunks = 0;
-        for (int tile = pair; tile < p.tiles; tile += pairs, ++done) {
-            int t0, f0;
-            locate(tile, t0, f0);
+        for (int tile = pair; tile < count; tile += pairs, ++done) {
+            const Tile at = locate(tile);
             const int buffer = done & 1;
             const unsigned accumulator = tmem_base + buffer * PAIR_COLUMNS + ((unsigned)(quarter * 32) << 16);
             ok = ok && mbarrier_wait_warp(&ready_bar[buffer], (done >> 1) & 1, abort_flag);
             if (!ok && lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.error, 3); }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // (all four warps take part, whatever they found: they meet at barriers)
-            if (f0 < p.features) store_tile<GATED, epilogue_columns<PAIR_COLUMNS, GATED>(), TY>(p, map_y, accumulator, f0, t0, p.columns, ok, row, exchange, staging, staged_chunks);
+            if (at.f0 < p.features)
+                store_tile<GATED, epilogue_columns<PAIR_COLUMNS, GATED>(), TY>(p, map_y, accumulator, at.f0, at.t0, at.columns, ok, row, exchange, staging, staged_chunks);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(drained[buffer]) : "memory");
@@ -938,9 +931,9 @@ int make_store_map(CUtensorMap* map, void* base, long long tokens, long long fea
 }
 
 // The same with a kilobyte to align the stages.
-template <int BN, int STAGES, bool GROUPED>
+template <int BN, int STAGES>
 constexpr size_t shared_bytes() {
-    return shared_floor<BN, STAGES>() + 1024 + (GROUPED ? sizeof(GroupPieces) : 0);
+    return shared_floor<BN, STAGES>() + 1024;
 }
 
 // Sets the kernel up (once) and returns how many of its blocks the device promises to hold on an SM
@@ -948,9 +941,9 @@ constexpr size_t shared_bytes() {
 // tensor memory the device reports one, whatever its other needs; two such blocks do run on an SM
 // together where shared memory and tensor memory allow (measured), which launches whose blocks do not
 // wait for each other make use of.
-template <int BN, int STAGES, bool GATED, typename TY, bool GROUPED = false>
+template <int BN, int STAGES, bool GATED, typename TY>
 int blocks_per_sm() {
-    constexpr size_t shared = shared_bytes<BN, STAGES, GROUPED>();
+    constexpr size_t shared = shared_bytes<BN, STAGES>();
     static_assert(shared <= (BN <= 64 ? 113 : 227) * 1024, "the stages fit an SM's shared memory (twice for small tiles)");
     static std::atomic<int> known_by_device[64];         // 0: not asked yet; else the answer + 1
     int device = 0;
@@ -958,7 +951,7 @@ int blocks_per_sm() {
     std::atomic<int>& known = known_by_device[device];
     int value = known.load(std::memory_order_acquire) - 1;
     if (value < 0) {
-        auto kernel = gemm_tcgen05_kernel<BN, STAGES, GATED, TY, GROUPED>;
+        auto kernel = gemm_tcgen05_kernel<BN, STAGES, GATED, TY>;
         value = 0;
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) == cudaSuccess &&
             cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) ==
@@ -973,12 +966,12 @@ int blocks_per_sm() {
     return value;
 }
 
-template <int BN, int STAGES, bool GATED, typename TY, bool GROUPED = false>
+template <int BN, int STAGES, bool GATED, typename TY>
 int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const CUtensorMap& map_y, const Params& p, int blocks,
            cudaStream_t stream) {
-    constexpr size_t shared = shared_bytes<BN, STAGES, GROUPED>();
-    auto kernel = gemm_tcgen05_kernel<BN, STAGES, GATED, TY, GROUPED>;
-    const int per_sm = blocks_per_sm<BN, STAGES, GATED, TY, GROUPED>();
+    constexpr size_t shared = shared_bytes<BN, STAGES>();
+    auto kernel = gemm_tcgen05_kernel<BN, STAGES, GATED, TY>;
+    const int per_sm = blocks_per_sm<BN, STAGES, GATED, TY>();
     if (per_sm <= 0) return KIDI_REFUSED_SIZE;
     if (p.rounds > 0) {
         kernel<<<blocks, THREADS, shared, stream>>>(map_w, map_x, map_y, p);
@@ -1032,11 +1025,11 @@ int pair_columns(int tokens, int features, int span) {
     return best;
 }
 
-template <bool GATED, typename TY>
+template <bool GATED, typename TY, bool GROUPED = false>
 int launch_pairs(const CUtensorMap& map_w, const CUtensorMap& map_x, const CUtensorMap& map_y, const Params& p, cudaStream_t stream) {
-    constexpr size_t shared = pair_shared_bytes();
+    constexpr size_t shared = pair_shared_bytes<GROUPED>();
     static_assert(shared <= 226 * 1024, "the stages fit an SM's shared memory");
-    auto kernel = gemm_tcgen05_pairs_kernel<GATED, TY>;
+    auto kernel = gemm_tcgen05_pairs_kernel<GATED, TY, GROUPED>;
     static std::atomic<unsigned long long> allowed{0};
     const cudaError_t status = kidi_allow_shared(kernel, shared, allowed);
     if (status != cudaSuccess) return (int)status;
@@ -1200,7 +1193,6 @@ KIDI_API int kidi_gemm_tcgen05_grouped(const void* x, const void* w, void* y, in
         groups <= 0 || rows > 0x7fffffffLL || tokens % GROUP_TILE || !group_of_tile || !error)
         return KIDI_REFUSED_SIZE;
     const int span = gated ? 64 : BM;
-    const int feature_tiles = (features + span - 1) / span;
     // A launch knows 1,024 tiles; more go in several (tiles of one group that fall into two launches are not paired).
     for (int first = 0; first < tokens / GROUP_TILE; first += MOST_GROUP_TILES) {
         const int count = tokens / GROUP_TILE - first < MOST_GROUP_TILES ? tokens / GROUP_TILE - first : MOST_GROUP_TILES;
@@ -1215,22 +1207,18 @@ KIDI_API int kidi_gemm_tcgen05_grouped(const void* x, const void* w, void* y, in
         p.features = features;
         p.k_blocks = (K + BK - 1) / BK;
         p.token_tiles = count;
-        p.tiles = (long long)feature_tiles * count;
+        p.tiles = (long long)((features + 2 * span - 1) / (2 * span)) * count;      // (at most: the kernel knows its pieces)
         p.group_of_tile = group_of_tile + first;
         p.used_of_tile = used ? used + first : nullptr;
         p.group_rows = features * (gated ? 2 : 1);
-        p.staged = 1;
+        p.staged = !(features & 7);
         if (gate) p.gate = *gate;
-        const long long sms = sm_count_of_current_device();
-        const int blocks = (int)(p.tiles < sms ? p.tiles : sms);
-        p.rounds = 1;                    // (the kernel counts its rounds itself: it knows how many pieces of work there are)
-        p.tail_first = p.tiles;
         CUtensorMap map_w, map_x, map_y;
         int status = make_map(&map_w, w, rows, K, K, gated ? 64 : BM);
         if (!status) status = make_map(&map_x, from, p.tokens, K, ldx, GROUP_BOX);
-        if (!status) status = make_store_map(&map_y, to, p.tokens, features, ldy, span);
-        if (!status) status = gated ? launch<256, 4, true, bf16, true>(map_w, map_x, map_y, p, blocks, stream)
-                                    : launch<256, 4, false, bf16, true>(map_w, map_x, map_y, p, blocks, stream);
+        if (!status && p.staged) status = make_store_map(&map_y, to, p.tokens, features, ldy, span);
+        if (!status) status = gated ? launch_pairs<true, bf16, true>(map_w, map_x, map_y, p, stream)
+                                    : launch_pairs<false, bf16, true>(map_w, map_x, map_y, p, stream);
         if (status) return status;
     }
     return 0;
